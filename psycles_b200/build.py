@@ -83,7 +83,7 @@ def _build(force: bool, verbose_ptxas: bool, defs: list[str]) -> pathlib.Path:
 
 def main(argv: list[str]) -> None:
     """`--force`, `--ptxas`, `-D NAME=VALUE` (repeatable: a kernel tuning
-    macro or the build option PSY_BVH_WIDTH=8) and `--out PATH` (a variant
+    macro) and `--out PATH` (a variant
     library beside the default one; load it with PSYCLES_CUDA_LIB=PATH)."""
     import argparse
     ap = argparse.ArgumentParser(prog="python -m psycles_b200.build")
