@@ -290,6 +290,14 @@ struct Box {
     }
 };
 
+// A node of the binary build.
+struct BinaryNode {
+    float4 x;    // left.lo.x, left.hi.x, right.lo.x, right.hi.x
+    float4 y;    // left.lo.y, left.hi.y, right.lo.y, right.hi.y
+    float4 z;    // left.lo.z, left.hi.z, right.lo.z, right.hi.z
+    int4 child;  // x/y: >= 0 inner node, < 0 leaf ~first; z/w: leaf counts
+};
+
 struct Prim {
     Box box;
     double c[3];
@@ -312,9 +320,6 @@ void padded(const Box &b, float lo[3], float hi[3]) {
     }
 }
 
-#ifndef PSY_LEAF_SIZE
-#define PSY_LEAF_SIZE 1u
-#endif
 #ifndef PSY_SAH_BINS
 #define PSY_SAH_BINS 32
 #endif
@@ -322,10 +327,70 @@ void padded(const Box &b, float lo[3], float hi[3]) {
 #define PSY_SAH_AXES 3
 #endif
 
+// A 4-wide node as built: child boxes in float, links as the traversal takes
+// them (node indices and leaf triangles relative to the tree).
+struct WideNode {
+    float lo[3][4], hi[3][4];
+    uint32_t link[4] = {psy::kInvalidId, psy::kInvalidId, psy::kInvalidId, psy::kInvalidId};
+};
+
+// The device form of a wide node: its children's boxes on the node's byte
+// grid, rounded outward, and its links moved to the scene's node and
+// triangle arrays.  The slab test evaluates a plane as f * (span / d) +
+// (base - o) / d in float; in units of position its rounding stays within a
+// few 2^-24 of the extent, the coordinates and the ray's own origin and
+// reach.  The margin takes 4e-6 (64 such units) of the first two on either
+// side; the last two are covered as they were for float planes, by the boxes' own
+// padding and the widened far bound.  span is at least 128 / 127 of the
+// padded extent, so cell 127's plane lies past every child.  Boxes that are
+// not finite in float (or whose span would not be) give NaN planes, which
+// the test ignores.
+psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offset) {
+    psy::NodeGpu g{};
+    uint32_t *words[6] = {&g.lox, &g.hix, &g.loy, &g.hiy, &g.loz, &g.hiz};
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t v = w.link[k];
+        if (v == psy::kInvalidId || (v & ~psy::kLinkLeaf) >= psy::kLinkInstance) g.link[k] = v;
+        else g.link[k] = v + ((v & psy::kLinkLeaf) ? tri_offset : node_offset);
+    }
+    for (int a = 0; a < 3; ++a) {
+        double lo = 1e300, hi = -1e300;
+        for (int k = 0; k < 4; ++k) {
+            if (w.link[k] == psy::kInvalidId) continue;
+            lo = std::min(lo, double(w.lo[a][k]));
+            hi = std::max(hi, double(w.hi[a][k]));
+        }
+        if (lo > hi) lo = hi = 0.0;
+        const double margin = 4e-6 * (hi - lo) + 4e-6 * std::max(std::fabs(lo), std::fabs(hi)) + 1e-30;
+        lo -= margin;
+        hi += margin;
+        float span = std::nextafter(float((hi - lo) * (128.0 / 127.0)), INFINITY);
+        float base = 0.0f;
+        for (int tries = 0; tries < 64; ++tries) {
+            base = std::nextafter(float(lo - double(span)), -INFINITY);
+            if (double(base) + double(span) * (255.0 / 128.0) >= hi) break;
+            span = std::nextafter(span * 1.000001f, INFINITY);
+        }
+        if (!std::isfinite(base) || !std::isfinite(span)) base = span = NAN;
+        g.base[a] = base;
+        g.span[a] = span;
+        for (int k = 0; k < 4; ++k) {
+            double ql = 127.0, qh = 0.0;  // empty
+            if (w.link[k] != psy::kInvalidId && std::isfinite(base)) {
+                ql = std::floor((double(w.lo[a][k]) - margin - base) / double(span) * 128.0 - 128.0);
+                qh = std::ceil((double(w.hi[a][k]) + margin - base) / double(span) * 128.0 - 128.0);
+            }
+            *words[2 * a] |= (0x80u | uint32_t(std::min(std::max(ql, 0.0), 127.0))) << (8 * k);
+            *words[2 * a + 1] |= (0x80u | uint32_t(std::min(std::max(qh, 0.0), 127.0))) << (8 * k);
+        }
+    }
+    return g;
+}
+
 struct Builder {
-    std::vector<psy::BvhNodeGpu> nodes;
+    std::vector<BinaryNode> nodes;
     std::vector<Prim> prims;
-    uint32_t leaf_size = PSY_LEAF_SIZE;
+    static constexpr uint32_t leaf_size = 1u;
     bool leaf_is_id = false;  // TLAS: leaf link = ~prim id, count 1
     bool parallel = true;     // large subtrees on threads of their own
     // binary depth below which splits are chosen by SAH; deeper ranges split
@@ -369,7 +434,7 @@ struct Builder {
     }
 
     // `box` / `cbox` bound the prims [begin, end) and their centroids.
-    Child build_into(std::vector<psy::BvhNodeGpu> &out, uint32_t begin, uint32_t end, int depth, const Box &box,
+    Child build_into(std::vector<BinaryNode> &out, uint32_t begin, uint32_t end, int depth, const Box &box,
                      const Box &cbox) {
         const uint32_t count = end - begin;
         if (count <= leaf_size) return leaf(begin, end, box);
@@ -507,7 +572,7 @@ struct Builder {
         out.push_back({});
         Child l, r;
         if (parallel && depth < 8 && count >= 2048u) {
-            std::vector<psy::BvhNodeGpu> right_nodes;
+            std::vector<BinaryNode> right_nodes;
             std::exception_ptr error;
             std::thread worker([&]() {
                 try {
@@ -525,7 +590,7 @@ struct Builder {
             worker.join();
             if (error) std::rethrow_exception(error);
             const int offset = int(out.size());
-            for (psy::BvhNodeGpu &n : right_nodes) {
+            for (BinaryNode &n : right_nodes) {
                 if (n.child.x >= 0) n.child.x += offset;
                 if (n.child.y >= 0) n.child.y += offset;
             }
@@ -541,11 +606,11 @@ struct Builder {
 
     void write(int index, const Child &l, const Child &r) { write(nodes, index, l, r); }
 
-    void write(std::vector<psy::BvhNodeGpu> &out, int index, const Child &l, const Child &r) {
+    void write(std::vector<BinaryNode> &out, int index, const Child &l, const Child &r) {
         float llo[3], lhi[3], rlo[3], rhi[3];
         padded(l.box, llo, lhi);
         padded(r.box, rlo, rhi);
-        psy::BvhNodeGpu &n = out[size_t(index)];
+        BinaryNode &n = out[size_t(index)];
         n.x = make_float4(llo[0], lhi[0], rlo[0], rhi[0]);
         n.y = make_float4(llo[1], lhi[1], rlo[1], rhi[1]);
         n.z = make_float4(llo[2], lhi[2], rlo[2], rhi[2]);
@@ -557,10 +622,15 @@ struct Builder {
     // own two children until four children (or only leaves) remain; then
     // every inner child is collapsed the same way.  Child boxes are the
     // binary build's padded boxes, so the slab test stays conservative.
-    std::vector<psy::WideNodeGpu> widen() const {
-        std::vector<psy::WideNodeGpu> wide;
+    // Links are tree-relative; leaf links count along `order`, which
+    // receives the prims (indices into `prims`) a node's leaves follow one
+    // another in.
+    std::vector<WideNode> widen(std::vector<uint32_t> &order) const {
+        std::vector<WideNode> wide;
         wide.reserve(nodes.size() / 2u + 1u);
-        collapse(0, wide);
+        order.clear();
+        order.reserve(prims.size());
+        collapse(0, wide, order);
         return wide;
     }
 
@@ -575,7 +645,7 @@ struct Builder {
     };
 
     WideChild child_of(int node, int side) const {
-        const psy::BvhNodeGpu &n = nodes[size_t(node)];
+        const BinaryNode &n = nodes[size_t(node)];
         WideChild c;
         if (side == 0) {
             c.lo[0] = n.x.x, c.hi[0] = n.x.y, c.lo[1] = n.y.x, c.hi[1] = n.y.y, c.lo[2] = n.z.x, c.hi[2] = n.z.y;
@@ -587,7 +657,7 @@ struct Builder {
         return c;
     }
 
-    int collapse(int node, std::vector<psy::WideNodeGpu> &wide) const {
+    int collapse(int node, std::vector<WideNode> &wide, std::vector<uint32_t> &order) const {
         WideChild kids[4] = {child_of(node, 0), child_of(node, 1), {}, {}};
         int n = 2;
         while (n < 4) {
@@ -605,48 +675,27 @@ struct Builder {
         }
         const int index = int(wide.size());
         wide.push_back({});
-        int links[4], counts[4];
-        float lo[3][4], hi[3][4];
-        // empty slots (and empty leaves) get +inf planes on every axis: the
-        // traversal's slab test then misses them for any ray direction
-        for (int k = 0; k < 4; ++k) {
-            if (k < n && (kids[k].link >= 0 || kids[k].count > 0)) {
-                for (int a = 0; a < 3; ++a) {
-                    lo[a][k] = kids[k].lo[a];
-                    hi[a][k] = kids[k].hi[a];
-                }
-                // the traversal pushes a count-0 slot's link as it is: a
-                // tagged node index (BLAS indices are made global when the
-                // meshes are concatenated) or a tagged instance; a leaf of
-                // triangles keeps its first primitive (made global likewise)
-                if (kids[k].link >= 0) {
-                    links[k] = int((leaf_is_id ? psy::kTagTlas : psy::kTagBlas) | uint32_t(collapse(kids[k].link, wide)));
-                    counts[k] = 0;
-                } else if (leaf_is_id) {
-                    links[k] = int(psy::kTagInstance | uint32_t(~kids[k].link));
-                    counts[k] = 0;
-                } else {
-                    links[k] = ~kids[k].link;
-                    counts[k] = kids[k].count;
-                }
-            } else {
-                for (int a = 0; a < 3; ++a) {
-                    lo[a][k] = INFINITY;
-                    hi[a][k] = INFINITY;
-                }
-                links[k] = int(psy::kInvalidId);
-                counts[k] = 0;
+        WideNode w;
+        // leaves (of triangles) first, then inner children and instances;
+        // empty slots keep kInvalidId
+        int k = 0;
+        auto put = [&](const WideChild &c, uint32_t link) {
+            for (int a = 0; a < 3; ++a) {
+                w.lo[a][k] = c.lo[a];
+                w.hi[a][k] = c.hi[a];
             }
+            w.link[k++] = link;
+        };
+        for (int c = 0; c < n; ++c) {
+            if (leaf_is_id || kids[c].link >= 0 || kids[c].count == 0) continue;
+            put(kids[c], psy::kLinkLeaf | uint32_t(order.size()));
+            order.push_back(uint32_t(~kids[c].link));
         }
-        psy::WideNodeGpu &w = wide[size_t(index)];
-        w.lox = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
-        w.hix = make_float4(hi[0][0], hi[0][1], hi[0][2], hi[0][3]);
-        w.loy = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
-        w.hiy = make_float4(hi[1][0], hi[1][1], hi[1][2], hi[1][3]);
-        w.loz = make_float4(lo[2][0], lo[2][1], lo[2][2], lo[2][3]);
-        w.hiz = make_float4(hi[2][0], hi[2][1], hi[2][2], hi[2][3]);
-        w.link = make_int4(links[0], links[1], links[2], links[3]);
-        w.count = make_int4(counts[0], counts[1], counts[2], counts[3]);
+        for (int c = 0; c < n; ++c) {
+            if (kids[c].link >= 0) put(kids[c], uint32_t(collapse(kids[c].link, wide, order)));
+            else if (leaf_is_id && kids[c].count > 0) put(kids[c], psy::kLinkInstance | uint32_t(~kids[c].link));
+        }
+        wide[size_t(index)] = w;
         return index;
     }
 
@@ -685,25 +734,24 @@ struct Builder {
 // largest stack any ray can build, and the compile step keeps them within
 // the device stack (psy::kTraversalStackSize).
 
-// Pushable children (count-0 slots with a link) of a wide node.
-int wide_pushable(const psy::WideNodeGpu &w, uint32_t links[4]) {
-    const int *lk = &w.link.x;
-    const int *ct = &w.count.x;
+// Pushable children (inner nodes and instances) of a wide node; leaf
+// triangles are tested before anything is pushed above them.
+int wide_pushable(const WideNode &w, uint32_t links[4]) {
     int n = 0;
     for (int k = 0; k < 4; ++k)
-        if (ct[k] == 0 && uint32_t(lk[k]) != psy::kInvalidId) links[n++] = uint32_t(lk[k]);
+        if ((w.link[k] & psy::kLinkLeaf) == 0u) links[n++] = w.link[k];
     return n;
 }
 
 // Entries a BLAS walk adds above those waiting when its root is entered
 // (mesh-local node indices; a parent precedes its children).
-uint32_t blas_stack_need(const std::vector<psy::WideNodeGpu> &w) {
+uint32_t blas_stack_need(const std::vector<WideNode> &w) {
     std::vector<uint32_t> need(w.size(), 0u);
     for (size_t i = w.size(); i-- > 0;) {
         uint32_t links[4];
         const int n = wide_pushable(w[i], links);
         uint32_t deepest = 0u;
-        for (int k = 0; k < n; ++k) deepest = std::max(deepest, need[links[k] & ~psy::kTagMask]);
+        for (int k = 0; k < n; ++k) deepest = std::max(deepest, need[links[k]]);
         need[i] = n > 0 ? uint32_t(n - 1) + deepest : 0u;
     }
     return w.empty() ? 0u : need[0];
@@ -711,18 +759,17 @@ uint32_t blas_stack_need(const std::vector<psy::WideNodeGpu> &w) {
 
 // Entries waiting on the stack when each instance of the TLAS is entered
 // (0 for instances the TLAS does not reference).
-std::vector<uint32_t> tlas_instance_depths(const std::vector<psy::WideNodeGpu> &w, uint32_t instance_count) {
+std::vector<uint32_t> tlas_instance_depths(const std::vector<WideNode> &w, uint32_t instance_count) {
     std::vector<uint32_t> depth(w.size(), 0u), inst(instance_count, 0u);
     for (size_t i = 0; i < w.size(); ++i) {
         uint32_t links[4];
         const int n = wide_pushable(w[i], links);
         for (int k = 0; k < n; ++k) {
             const uint32_t below = depth[i] + uint32_t(n - 1);
-            const uint32_t idx = links[k] & ~psy::kTagMask;
-            if ((links[k] & psy::kTagMask) == psy::kTagInstance) {
-                if (idx < instance_count) inst[idx] = below;
-            } else if (idx < w.size()) {
-                depth[idx] = below;
+            if (links[k] >= psy::kLinkInstance) {
+                if (links[k] - psy::kLinkInstance < instance_count) inst[links[k] - psy::kLinkInstance] = below;
+            } else if (links[k] < w.size()) {
+                depth[links[k]] = below;
             }
         }
     }
@@ -1431,15 +1478,15 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     std::vector<psy::MeshGpu> meshes(d->mesh_count);
     std::vector<float> positions, normals;
     std::vector<uint32_t> indices, tri_materials;
-    std::vector<psy::WideNodeGpu> blas;
-    std::vector<float4> tris;
+    std::vector<psy::NodeGpu> nodes;
+    std::vector<psy::TriGpu> tris;
     std::vector<Box> mesh_boxes(d->mesh_count);
-    std::vector<std::vector<psy::WideNodeGpu>> mesh_wide(d->mesh_count);
+    std::vector<std::vector<WideNode>> mesh_wide(d->mesh_count);
     // triangle records in BVH leaf order, written by each mesh's build at
     // the mesh's offset (meshes in input order)
     std::vector<uint64_t> mesh_tri_first(d->mesh_count + 1u, 0u);
     for (uint32_t i = 0; i < d->mesh_count; ++i) mesh_tri_first[i + 1u] = mesh_tri_first[i] + d->meshes[i].triangle_count;
-    tris.resize(3u * mesh_tri_first[d->mesh_count]);
+    tris.resize(mesh_tri_first[d->mesh_count]);
     // one mesh's BLAS, its triangle records in leaf order and its stack need
     std::vector<uint32_t> mesh_need(d->mesh_count, 0u);
     auto build_mesh = [&](uint32_t i, int sah_depth_limit) {
@@ -1457,18 +1504,20 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
             p.id = k;
         }
         mesh_boxes[i] = bld.build_root();
-        float4 *out = tris.data() + 3u * mesh_tri_first[i];
-        auto put = [&](uint32_t id) {
-            for (int c = 0; c < 3; ++c) {
-                const float *v = m.positions + 3ull * m.indices[3ull * id + c];
-                float w = 0.0f;
-                if (c == 0) std::memcpy(&w, &id, 4);
-                *out++ = make_float4(v[0], v[1], v[2], w);
-            }
-        };
-        mesh_wide[i] = bld.widen();
+        std::vector<uint32_t> order;
+        mesh_wide[i] = bld.widen(order);
         mesh_need[i] = blas_stack_need(mesh_wide[i]);
-        for (const Prim &p : bld.prims) put(p.id);
+        psy::TriGpu *out = tris.data() + mesh_tri_first[i];
+        for (const uint32_t leaf : order) {
+            const uint32_t id = bld.prims[leaf].id;
+            float4 v[3];
+            for (int c = 0; c < 3; ++c) {
+                const float *p = m.positions + 3ull * m.indices[3ull * id + c];
+                v[c] = make_float4(p[0], p[1], p[2], 0.0f);
+            }
+            std::memcpy(&v[0].w, &id, 4);
+            *out++ = psy::TriGpu{v[0], v[1], v[2], make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
+        }
     };
     {
         std::vector<uint32_t> by_size(d->mesh_count);
@@ -1485,7 +1534,6 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // ---- instances + TLAS
     std::vector<psy::InstanceGpu> instances(d->instance_count);
     Builder tl;
-    tl.leaf_size = 1u;
     tl.leaf_is_id = true;
     std::vector<M34> o2w(d->instance_count);
     for (uint32_t i = 0; i < d->instance_count; ++i) {
@@ -1554,9 +1602,10 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // levels); a scene that still exceeds it is rejected, so no traversal
     // ever drops a subtree.
     const uint32_t stack_cap = psy::kTraversalStackSize;
-    std::vector<psy::WideNodeGpu> tl_wide = tl.widen();
+    std::vector<WideNode> tl_wide;
+    std::vector<uint32_t> tl_order;
     auto instance_depths = [&]() {
-        tl_wide = tl.widen();
+        tl_wide = tl.widen(tl_order);
         return tlas_instance_depths(tl_wide, d->instance_count);
     };
     std::vector<uint32_t> inst_depth = instance_depths();
@@ -1598,6 +1647,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         sc->stats.stack_capacity = stack_cap;
     }
 
+    uint32_t node_count = uint32_t(tl_wide.size());
     uint32_t prim_offset = 0;
     for (uint32_t i = 0; i < d->mesh_count; ++i) {
         const psy_mesh_desc &m = d->meshes[i];
@@ -1619,23 +1669,42 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
             g.material_offset = psy::kInvalidId;
         }
         g.tri_offset = uint32_t(mesh_tri_first[i]);
-        g.node_offset = uint32_t(blas.size());
-        // global node and triangle indices of the mesh's links
-        for (psy::WideNodeGpu &w : mesh_wide[i]) {
-            int *lk = &w.link.x;
-            const int *ct = &w.count.x;
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t v = uint32_t(lk[k]);
-                if (ct[k] > 0) lk[k] = int(v + g.tri_offset);
-                else if (v != psy::kInvalidId && (v & psy::kTagMask) == psy::kTagBlas)
-                    lk[k] = int(psy::kTagBlas | ((v & ~psy::kTagMask) + g.node_offset));
-            }
-        }
-        blas.insert(blas.end(), mesh_wide[i].begin(), mesh_wide[i].end());
-        std::vector<psy::WideNodeGpu>().swap(mesh_wide[i]);
+        g.node_offset = node_count;
+        node_count += uint32_t(mesh_wide[i].size());
         sc->triangle_count += m.triangle_count;
     }
-    if (blas.empty()) blas.push_back({});
+    // the device nodes, in parallel over chunks of each tree
+    nodes.resize(node_count);
+    {
+        constexpr size_t kNodeChunk = 1024u;
+        struct NodeJob {
+            const std::vector<WideNode> *wide;
+            size_t first;
+            uint32_t node_offset, tri_offset;
+        };
+        std::vector<NodeJob> node_jobs;
+        for (size_t f = 0; f < tl_wide.size(); f += kNodeChunk) node_jobs.push_back({&tl_wide, f, 0u, 0u});
+        for (uint32_t i = 0; i < d->mesh_count; ++i)
+            for (size_t f = 0; f < mesh_wide[i].size(); f += kNodeChunk)
+                node_jobs.push_back({&mesh_wide[i], f, meshes[i].node_offset, meshes[i].tri_offset});
+        const psy_status quantised = parallel_for(uint32_t(node_jobs.size()), nullptr, [&](uint32_t job) {
+            const NodeJob &j = node_jobs[job];
+            const size_t end = std::min(j.wide->size(), j.first + kNodeChunk);
+            for (size_t k = j.first; k < end; ++k)
+                nodes[j.node_offset + k] = quantise((*j.wide)[k], j.node_offset, j.tri_offset);
+        });
+        if (quantised != PSY_OK) return quantised;
+    }
+    std::vector<psy::EntryGpu> entries(d->instance_count);
+    for (uint32_t i = 0; i < d->instance_count; ++i) {
+        const psy::MeshGpu &mesh = meshes[instances[i].mesh];
+        psy::EntryGpu &e = entries[i];
+        std::copy(std::begin(instances[i].w2o), std::end(instances[i].w2o), e.w2o);
+        e.root = mesh.node_offset;
+        e.prim_offset = mesh.prim_offset;
+        e.visibility = instances[i].visibility;
+        e.pad = 0u;
+    }
 
     // ---- materials and parameter blocks
     std::vector<psy_closure_instruction> code;
@@ -1813,13 +1882,13 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // device pool: a later compile reuses the memory a destroyed scene gave
     // back, and parameter blocks replaced by edits are retired without
     // waiting on the device.
-    for (DeviceBuffer *b : {&sc->tlas, &sc->blas, &sc->tris, &sc->instances, &sc->meshes, &sc->positions, &sc->normals,
+    for (DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions, &sc->normals,
                             &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->code, &sc->value_buf, &sc->scalar_buf,
                             &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights, &sc->lamp_consts,
                             &sc->lamp_bounds, &sc->lamp_ids})
         b->ordered = st;
-    PSY_CUDA_TRY(sc->tlas.upload(tl_wide, st));
-    PSY_CUDA_TRY(sc->blas.upload(blas, st));
+    PSY_CUDA_TRY(sc->nodes.upload(nodes, st));
+    PSY_CUDA_TRY(sc->entries.upload(entries, st));
     PSY_CUDA_TRY(sc->tris.upload(tris, st));
     PSY_CUDA_TRY(sc->instances.upload(instances, st));
     PSY_CUDA_TRY(sc->meshes.upload(meshes, st));
@@ -1867,15 +1936,15 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     PSY_CUDA_TRY(sc->lamp_ids.upload(lamp_ids, st));
     PSY_CUDA_TRY(cudaStreamSynchronize(st));
     sc->stats.upload_bytes = 0u;
-    for (const DeviceBuffer *b : {&sc->tlas, &sc->blas, &sc->tris, &sc->instances, &sc->meshes, &sc->positions,
+    for (const DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions,
                                   &sc->normals, &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->code,
                                   &sc->value_buf, &sc->scalar_buf, &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights,
                                   &sc->lamp_consts, &sc->lamp_bounds, &sc->lamp_ids})
         sc->stats.upload_bytes += b->bytes;
     psy::SceneView &v = sc->view;
-    v.tlas = sc->tlas.as<psy::WideNodeGpu>();
-    v.blas = sc->blas.as<psy::WideNodeGpu>();
-    v.tris = sc->tris.as<float4>();
+    v.nodes = sc->nodes.as<psy::NodeGpu>();
+    v.entries = sc->entries.as<psy::EntryGpu>();
+    v.tris = sc->tris.as<psy::TriGpu>();
     v.instances = sc->instances.as<psy::InstanceGpu>();
     v.meshes = sc->meshes.as<psy::MeshGpu>();
     v.positions = sc->positions.as<float>();
@@ -2091,7 +2160,7 @@ psy_status psy_session_read_trace(psy_session *s, psy_path_trace *out) {
 
 uint64_t psy::host::scene_device_bytes(const psy_scene *s) {
     uint64_t n = 0u;
-    for (const DeviceBuffer *b : {&s->tlas, &s->blas, &s->tris, &s->instances, &s->meshes, &s->positions, &s->normals,
+    for (const DeviceBuffer *b : {&s->nodes, &s->entries, &s->tris, &s->instances, &s->meshes, &s->positions, &s->normals,
                                   &s->indices, &s->tri_materials, &s->material_buf, &s->code, &s->value_buf, &s->scalar_buf,
                                   &s->vector_buf, &s->emitters, &s->distribution, &s->ggx_tables, &s->lights, &s->lamp_consts, &s->lamp_bounds,
                                   &s->lamp_ids, &s->lt_nodes, &s->lt_emitters, &s->lt_mapping, &s->lt_lookup})

@@ -194,22 +194,34 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 }
 
 // Persistent closest-hit kernel: each lane owns one ray at a time and, when
-// it finishes, the warp refills its idle lanes from a global fetch counter
-// (one atomic per warp), so lanes do not wait for the warp's longest ray.
-#ifndef PSY_TRAVERSAL_BUDGET
-#define PSY_TRAVERSAL_BUDGET 24
+// some have finished, the warp refills its idle lanes from a global fetch
+// counter (one atomic per warp), so lanes do not wait for the warp's longest
+// ray.  Refilling at 12 idle lanes measured best (4: 182 ms of closest hits
+// per 1080p procedural frame of 64 spp, 8: 169, 12: 165, 16: 164 with shadow
+// rays slower again).
+//
+// Both traversal kernels were bound by L1 wavefronts (72 % of peak for closest
+// hits: a 128-byte node in eight 16-byte loads, each a wavefront per lane)
+// and by divergence (9 and 7 of 32 lanes).  With 64-byte nodes in two loads
+// and steps taken together (traverse_warp) they are issue-bound; the lower
+// register budgets (64 and 80) give the latency more warps to hide in: 155 and 117 ms at
+// 8 and 5 blocks of 128 an SM, 169 and 134 ms at 6 and 4, 154 at 9 for
+// closest hits.  Together 224 -> 144 ms for closest hits and 185 -> 108 ms for
+// shadow rays.
+#ifndef PSY_REFILL_LANES
+#define PSY_REFILL_LANES 12
 #endif
 #ifndef PSY_INTERSECT_MIN_BLOCKS
-#define PSY_INTERSECT_MIN_BLOCKS 6
+#define PSY_INTERSECT_MIN_BLOCKS 8
 #endif
 #ifndef PSY_SHADE_MIN_BLOCKS
 #define PSY_SHADE_MIN_BLOCKS 3
 #endif
 #ifndef PSY_SHADOW_MIN_BLOCKS
-#define PSY_SHADOW_MIN_BLOCKS 4
+#define PSY_SHADOW_MIN_BLOCKS 6
 #endif
-// Nodes a lane advances between refills of idle lanes.
-constexpr int kTraversalBudget = PSY_TRAVERSAL_BUDGET;
+// Lanes that finish before a warp is refilled.
+constexpr int kRefillLanes = PSY_REFILL_LANES;
 constexpr uint32_t kFullMask = 0xffffffffu;
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
@@ -238,8 +250,11 @@ __global__ void __launch_bounds__(128, PSY_INTERSECT_MIN_BLOCKS)
     const uint32_t count = b.counters[0];
     const bool sorted = sort_threshold != 0u && count >= sort_threshold;
     TraversalState t;
-    Hit best;
-    bool has = false, active = false, exhausted = false;
+    t.node = kLinkDone;
+    t.leaves = 0u;
+    float best_t = 0.0f, best_u = 0.0f, best_v = 0.0f;
+    uint32_t best_instance = kInvalid, best_prim = kInvalid;
+    bool active = false, exhausted = false;
     uint32_t path = 0u, job = 0u;
     for (;;) {
         const uint32_t q = warp_fetch(&b.counters[3], count, !active, exhausted);
@@ -256,34 +271,30 @@ __global__ void __launch_bounds__(128, PSY_INTERSECT_MIN_BLOCKS)
             const uint32_t vis = st.y;
             const Ray ray{mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w};
             traversal_begin(t, s, ray, contract_visibility(vis), st2.y, st2.z, kInvalid, kInvalid);
-            has = false;
-            best.t = ray.tmax;
-            best.u = best.v = 0.0f;
-            best.instance = best.prim = best.object = best.cycles_prim = kInvalid;
+            best_t = ray.tmax;
+            best_u = best_v = 0.0f;
+            best_instance = best_prim = kInvalid;
             active = true;
         }
-        if (!__any_sync(kFullMask, active)) break;
-        if (active) {
-            const bool done = traversal_steps(t, s, kTraversalBudget,
-                                              [&](uint32_t ii, uint32_t local, uint32_t cp, float th, float u, float v) {
-                const bool later = ii > best.object || (ii == best.object && cp > best.cycles_prim);
-                if (has && !(th < best.t || (th == best.t && later))) return false;
-                has = true;
-                best.t = th;
-                best.u = u;
-                best.v = v;
-                best.instance = ii;
-                best.prim = local;
-                best.object = ii;
-                best.cycles_prim = cp;
-                t.tmax = th;
-                return false;
-            });
-            if (done) {
-                store_pair(b.hit, path, make_float4(best.t, best.u, best.v, __uint_as_float(best.instance)),
-                           make_uint4(has ? best.prim : kInvalid, 0u, 0u, 0u));
-                active = false;
-            }
+        const int busy = __popc(__ballot_sync(kFullMask, active));
+        if (busy == 0) break;
+        traverse_warp<true>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
+                            [&](uint32_t ii, uint32_t local, uint32_t, float th, float u, float v) {
+            // equal distances go to the greatest (object, primitive)
+            const bool later = ii > best_instance || (ii == best_instance && local > best_prim);
+            if (best_instance != kInvalid && !(th < best_t || (th == best_t && later))) return false;
+            best_t = th;
+            best_u = u;
+            best_v = v;
+            best_instance = ii;
+            best_prim = local;
+            t.tmax = th;
+            return false;
+        });
+        if (active && t.node == kLinkDone && t.leaves == 0u) {
+            store_pair(b.hit, path, make_float4(best_t, best_u, best_v, __uint_as_float(best_instance)),
+                       make_uint4(best_prim, 0u, 0u, 0u));
+            active = false;
         }
     }
 }
@@ -999,8 +1010,9 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
 // product in distance order (coincident distances count once, the greatest
 // identity standing for them).  The kernel computes it with one any-hit
 // traversal: it stops at the first opaque surface, collects transparent
-// ones, and multiplies them sorted by distance.  A ray whose surface count
-// outgrows the collector falls back to the iterated closest hit.
+// ones, and multiplies them sorted by distance.  A ray with more surfaces
+// than the collector holds keeps the nearest, multiplies them, and is traced
+// again from behind the last of them.
 
 constexpr int kShadowList = 8;
 
@@ -1010,99 +1022,10 @@ __device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_
     return mesh.material_offset == kInvalid ? inst.material : s.tri_materials[mesh.material_offset + local];
 }
 
-__device__ __noinline__ f3 shadow_iterated(const SceneView &s, const RenderParams &p, Ray ray, uint4 ids, uint32_t depth) {
-    f3 transmittance = mk3(1.0f);
-    for (uint32_t guard = 0; guard < 4096u; ++guard) {
-        Hit h;
-        if (!trace_closest(s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w, h)) return transmittance;
-        if (depth >= p.transparent_max) return mk3(0.0f);
-        const f3 t = clamp3(transparent_extinction(s, s.materials[surface_material(s, h.instance, h.prim)]), 0.0f, 1.0f);
-        if (!(max_component(t) > 0.0f)) return mk3(0.0f);
-        transmittance = transmittance * t;
-        depth += 1u;
-        ray.tmin = h.t == 0.0f ? 1.17549435e-38f : __uint_as_float(__float_as_uint(h.t) + 1u);
-    }
-    return mk3(0.0f);
-}
-
-__device__ __forceinline__ f3 shadow_transmittance(const SceneView &s, const RenderParams &p, const Ray &ray,
-                                                   uint4 ids, uint32_t depth) {
-    float tmax = ray.tmax;
-    if (!s.any_transparent) {
-        bool blocked = false;
-        traverse_scene(s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w, tmax,
-                       [&](uint32_t, uint32_t, uint32_t, float, float, float) {
-                           blocked = true;
-                           return true;
-                       });
-        return blocked ? mk3(0.0f) : mk3(1.0f);
-    }
-    float lt[kShadowList];
-    uint32_t lo[kShadowList], lp[kShadowList], lm[kShadowList];
-    int n = 0;
-    bool blocked = false, overflow = false;
-    traverse_scene(s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w, tmax,
-                   [&](uint32_t ii, uint32_t local, uint32_t cp, float t, float, float) {
-                       const uint32_t mi = surface_material(s, ii, local);
-                       const MaterialGpu m = s.materials[mi];
-                       if (!m.has_transparent) {
-                           blocked = true;
-                           return true;
-                       }
-                       for (int k = 0; k < n; ++k) {
-                           if (lt[k] == t) {  // coincident: keep the greatest identity
-                               if (ii > lo[k] || (ii == lo[k] && cp > lp[k])) {
-                                   lo[k] = ii;
-                                   lp[k] = cp;
-                                   lm[k] = mi;
-                               }
-                               return false;
-                           }
-                       }
-                       if (n == kShadowList) {
-                           overflow = true;
-                           return true;
-                       }
-                       lt[n] = t;
-                       lo[n] = ii;
-                       lp[n] = cp;
-                       lm[n] = mi;
-                       ++n;
-                       return false;
-                   });
-    if (blocked) return mk3(0.0f);
-    const uint32_t budget = depth >= p.transparent_max ? 0u : p.transparent_max - depth;
-    if (overflow) {
-        if (uint32_t(kShadowList) > budget) return mk3(0.0f);
-        return shadow_iterated(s, p, ray, ids, depth);
-    }
-    if (uint32_t(n) > budget) return mk3(0.0f);
-    // insertion sort by distance, then multiply in that order
-    for (int i = 1; i < n; ++i) {
-        const float kt = lt[i];
-        const uint32_t km = lm[i];
-        int j = i - 1;
-        while (j >= 0 && lt[j] > kt) {
-            lt[j + 1] = lt[j];
-            lm[j + 1] = lm[j];
-            --j;
-        }
-        lt[j + 1] = kt;
-        lm[j + 1] = km;
-    }
-    f3 transmittance = mk3(1.0f);
-    for (int i = 0; i < n; ++i) {
-        const f3 t = clamp3(transparent_extinction(s, s.materials[lm[i]]), 0.0f, 1.0f);
-        if (!(max_component(t) > 0.0f)) return mk3(0.0f);
-        transmittance = transmittance * t;
-    }
-    return transmittance;
-}
-
 // Persistent any-hit shadow kernel (same refill scheme as k_intersect).
 // Opaque-only scenes stop at the first accepted candidate; otherwise
-// transparent hits are collected per lane and resolved as in
-// shadow_transmittance once the traversal ends.
+// transparent hits are collected per lane and resolved by distance once
+// the traversal ends.
 // kMulti: shadow rays of a batched wavefront, each in its path's job.
 template <bool kMulti>
 __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
@@ -1112,11 +1035,16 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
     const uint32_t count = b.counters[2];
     const bool sorted = sort_threshold != 0u && count >= sort_threshold;
     TraversalState t;
+    t.node = kLinkDone;
+    t.leaves = 0u;
     bool active = false, exhausted = false, blocked = false, overflow = false;
     uint32_t q_cur = 0u, job = 0u;
     float lt[kShadowList];
     uint32_t lo[kShadowList], lp[kShadowList], lm[kShadowList];
     int n = 0;
+    // surfaces and their product before the ray's current start
+    uint32_t passed = 0u;
+    f3 transmittance = mk3(1.0f);
     for (;;) {
         uint32_t q = warp_fetch(&b.counters[4], count, !active, exhausted);
         if (sorted && q != kInvalid) q = b.queue_sorted[q];
@@ -1131,81 +1059,94 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
             traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w);
             blocked = overflow = false;
             n = 0;
+            passed = __float_as_uint(d.w);
+            transmittance = mk3(1.0f);
             active = true;
         }
-        if (!__any_sync(kFullMask, active)) break;
-        if (!active) continue;
-        bool done;
-        if (!s.any_transparent) {
-            done = traversal_steps<false>(t, s, kTraversalBudget, [&](uint32_t, uint32_t, uint32_t, float, float, float) {
+        const int busy = __popc(__ballot_sync(kFullMask, active));
+        if (busy == 0) break;
+        traverse_warp<false>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
+                             [&](uint32_t ii, uint32_t local, uint32_t cp, float th, float, float) {
+            if (!s.any_transparent) {
                 blocked = true;
                 return true;
-            });
-        } else {
-            done = traversal_steps<false>(t, s, kTraversalBudget,
-                                          [&](uint32_t ii, uint32_t local, uint32_t cp, float th, float, float) {
-                const uint32_t mi = surface_material(s, ii, local);
-                if (!s.materials[mi].has_transparent) {
+            }
+            const uint32_t mi = surface_material(s, ii, local);
+            if (!s.materials[mi].has_transparent) {
+                blocked = true;
+                return true;
+            }
+            for (int k = 0; k < n; ++k) {
+                if (lt[k] == th) {
+                    if (ii > lo[k] || (ii == lo[k] && cp > lp[k])) {
+                        lo[k] = ii;
+                        lp[k] = cp;
+                        lm[k] = mi;
+                    }
+                    return false;
+                }
+            }
+            int slot = n;
+            if (n == kShadowList) {
+                // more surfaces than the collector holds: keep the nearest,
+                // unless they exceed the ray's budget already
+                if (passed + uint32_t(kShadowList) >= p.transparent_max) {
                     blocked = true;
                     return true;
                 }
-                for (int k = 0; k < n; ++k) {
-                    if (lt[k] == th) {
-                        if (ii > lo[k] || (ii == lo[k] && cp > lp[k])) {
-                            lo[k] = ii;
-                            lp[k] = cp;
-                            lm[k] = mi;
-                        }
-                        return false;
-                    }
-                }
-                if (n == kShadowList) {
-                    overflow = true;
-                    return true;
-                }
-                lt[n] = th;
-                lo[n] = ii;
-                lp[n] = cp;
-                lm[n] = mi;
+                overflow = true;
+                slot = 0;
+                for (int k = 1; k < kShadowList; ++k)
+                    if (lt[k] > lt[slot]) slot = k;
+                if (th > lt[slot]) return false;
+            } else {
                 ++n;
-                return false;
-            });
-        }
-        if (!done) continue;
-        active = false;
-        const float4 d = b.sh_d[q_cur], c = b.sh_c[q_cur];
-        const uint32_t depth = __float_as_uint(c.w);
-        const uint32_t tdepth = __float_as_uint(d.w);
-        f3 transmittance = mk3(0.0f);
+            }
+            lt[slot] = th;
+            lo[slot] = ii;
+            lp[slot] = cp;
+            lm[slot] = mi;
+            return false;
+        });
+        if (!active || t.node != kLinkDone || t.leaves != 0u) continue;
+        // (transparent_max - passed surfaces may still lie on the ray)
+        if (uint32_t(n) > (passed >= p.transparent_max ? 0u : p.transparent_max - passed)) blocked = true;
         if (!blocked) {
-            const uint32_t budget = tdepth >= p.transparent_max ? 0u : p.transparent_max - tdepth;
-            if (overflow) {
-                if (uint32_t(kShadowList) <= budget)
-                    transmittance = shadow_iterated(s, p, t.ray, b.sh_ids[q_cur], tdepth);
-            } else if (uint32_t(n) <= budget) {
-                for (int i = 1; i < n; ++i) {
-                    const float kt = lt[i];
-                    const uint32_t km = lm[i];
-                    int j = i - 1;
-                    while (j >= 0 && lt[j] > kt) {
-                        lt[j + 1] = lt[j];
-                        lm[j + 1] = lm[j];
-                        --j;
-                    }
-                    lt[j + 1] = kt;
-                    lm[j + 1] = km;
+            for (int i = 1; i < n; ++i) {
+                const float kt = lt[i];
+                const uint32_t km = lm[i];
+                int j = i - 1;
+                while (j >= 0 && lt[j] > kt) {
+                    lt[j + 1] = lt[j];
+                    lm[j + 1] = lm[j];
+                    --j;
                 }
-                transmittance = mk3(1.0f);
-                for (int i = 0; i < n; ++i) {
-                    const f3 e = clamp3(transparent_extinction(s, s.materials[lm[i]]), 0.0f, 1.0f);
-                    if (!(max_component(e) > 0.0f)) {
-                        transmittance = mk3(0.0f);
-                        break;
-                    }
-                    transmittance = transmittance * e;
+                lt[j + 1] = kt;
+                lm[j + 1] = km;
+            }
+            for (int i = 0; i < n; ++i) {
+                const f3 e = clamp3(transparent_extinction(s, s.materials[lm[i]]), 0.0f, 1.0f);
+                if (!(max_component(e) > 0.0f)) {
+                    blocked = true;
+                    break;
                 }
+                transmittance = transmittance * e;
+            }
+            if (!blocked && overflow) {
+                passed += uint32_t(n);
+                const uint4 ids = b.sh_ids[q_cur];
+                Ray ray = t.ray;
+                ray.tmin = next_float_up(lt[n - 1]);
+                traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w);
+                overflow = false;
+                n = 0;
+                continue;
             }
         }
+        if (blocked) transmittance = mk3(0.0f);
+        active = false;
+        const float4 c = b.sh_c[q_cur];
+        const uint32_t depth = __float_as_uint(c.w);
         const uint32_t owner = b.sh_path[q_cur];
         const uint32_t path = owner & ~kShadowFinal;
         f3 contribution = mk3(0.0f);

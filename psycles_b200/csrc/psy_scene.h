@@ -1,12 +1,12 @@
 // Device-resident scene and render parameters of the B200 path tracer.
 //
 // HBM layout (one allocation per array, all 16-byte aligned):
-//   tlas / blas   4-wide BVH nodes, 128 B each (two 64-byte lines): six
-//                 float4 hold the four children's x/y/z slabs lane by
-//                 lane, two int4 the child links and leaf counts
-//   tris          leaf-ordered triangles of all meshes, 3 float4 per
-//                 triangle (48 B): object-space vertices, v0.w = local
-//                 primitive index bits
+//   nodes         4-wide BVH nodes with byte-quantised boxes, 64 B each
+//                 (two 32-byte sectors): the instance tree, then every
+//                 mesh's tree
+//   tris          leaf triangles of all meshes in node order, 64 B each:
+//                 object-space vertices, v0.w = local primitive index bits
+//   entries       per instance, the ray's transform and the mesh's root (64 B)
 //   positions / normals / indices  the meshes' shading data
 //   instances     InstanceGpu (object<->world transforms, mesh, material)
 //   materials / code / scalars / vectors  closure programs and their
@@ -30,23 +30,12 @@ constexpr uint32_t kInvalidId = 0xffffffffu;
 constexpr uint32_t kLightFlagUseMis = 1u << 30;
 constexpr uint32_t kLightFlagForward = 1u << 31;
 
-struct alignas(16) BvhNodeGpu {
-    float4 x;    // left.lo.x, left.hi.x, right.lo.x, right.hi.x
-    float4 y;    // left.lo.y, left.hi.y, right.lo.y, right.hi.y
-    float4 z;    // left.lo.z, left.hi.z, right.lo.z, right.hi.z
-    int4 child;  // x/y: >= 0 inner node, < 0 leaf ~first; z/w: leaf counts
-};
-static_assert(sizeof(BvhNodeGpu) == 64, "BVH node is one 64-byte line");
-
-// 4-wide node, collapsed from the binary build: child k's slabs in lane k.
-// link >= 0: inner node (relative to the BVH's first node); link < 0 with
-// count > 0: a leaf (~first triangle, or ~instance in the TLAS); count 0
-// with link < 0: an empty slot.
-// Traversal stack entries carry a 2-bit tag: a TLAS node, a BLAS node
-// (global index), an instance to enter, or the marker that returns to the
-// world ray.
-constexpr uint32_t kTagTlas = 0u, kTagBlas = 1u << 30, kTagInstance = 2u << 30, kTagLeave = 3u << 30;
-constexpr uint32_t kTagMask = 3u << 30;
+// Child links and traversal-stack entries: an inner node (global index), an
+// instance to enter, the marker that returns to the world ray, the end of
+// the traversal, or -- only as a child link -- a leaf triangle.  An empty
+// child slot holds kInvalidId.
+constexpr uint32_t kLinkInstance = 1u << 30, kLinkLeaf = 1u << 31;
+constexpr uint32_t kLinkLeave = kLinkLeaf - 1u, kLinkDone = kLinkLeaf - 2u;
 // Entries of the per-ray traversal stack.  Scene compile proves, from the
 // built trees, that no ray can push more (see blas_stack_need /
 // tlas_instance_depths in psy_host.cpp), rebuilding a mesh with median
@@ -55,16 +44,35 @@ constexpr uint32_t kTagMask = 3u << 30;
 constexpr uint32_t kTraversalStackSize = 48u;
 constexpr uint32_t kGgxETableSize = 32u * 32u, kGgxEavgTableSize = 32u;
 
-// Four children of a wide BVH node: boxes as six planes of four lanes, and
-// per child either a ready stack entry (count 0: a tagged global node index
-// or, in the TLAS, a tagged instance) or the first of `count` triangles in
-// the global triangle array.  Empty slots have +inf planes and count 0.
-struct alignas(16) WideNodeGpu {
-    float4 lox, hix, loy, hiy, loz, hiz;
-    int4 link;
-    int4 count;
+// Four children of a wide BVH node in two 32-byte sectors, so one ray reads
+// it with two 256-bit loads.  Child k's box is stored as one byte per plane
+// on a grid of 127 cells per axis: byte 0x80 | c stands for the factor
+// f = 1 + c / 128 and the plane base + span * f.  The host rounds the planes
+// outward, with a margin for the rounding of the slab test (see quantise in
+// psy_host.cpp).  Leaf children come first; their triangles follow one
+// another, so slot k's is the first slot's plus k.
+struct alignas(32) NodeGpu {
+    float base[3], span[3];
+    uint32_t lox, hix, loy, hiy, loz, hiz;  // byte k: child k
+    uint32_t link[4];
 };
-static_assert(sizeof(WideNodeGpu) == 128, "wide BVH node is two 64-byte lines");
+static_assert(sizeof(NodeGpu) == 64, "a node is two 32-byte sectors");
+
+// A leaf triangle (object space) in two sectors.
+struct alignas(32) TriGpu {
+    float4 v0;  // w: local primitive index bits
+    float4 v1, v2, pad;
+};
+static_assert(sizeof(TriGpu) == 64, "a triangle is two 32-byte sectors");
+
+// What a ray needs to enter an instance, in two sectors.
+struct alignas(32) EntryGpu {
+    float w2o[12];
+    uint32_t root;         // root node of the mesh
+    uint32_t prim_offset;  // Cycles primitive id of local primitive 0
+    uint32_t visibility, pad;
+};
+static_assert(sizeof(EntryGpu) == 64, "an instance entry is two 32-byte sectors");
 
 struct alignas(16) InstanceGpu {
     float o2w[12];  // column-major c0, c1, c2, c3 (xyz each)
@@ -74,7 +82,7 @@ struct alignas(16) InstanceGpu {
 };
 
 struct alignas(16) MeshGpu {
-    uint32_t node_offset;    // root of the mesh BLAS in `blas`
+    uint32_t node_offset;    // root of the mesh's tree in `nodes`
     uint32_t tri_offset;     // first leaf triangle in `tris`
     uint32_t triangle_count;
     uint32_t prim_offset;    // Cycles primitive id of local primitive 0
@@ -122,9 +130,9 @@ struct alignas(16) LampConstGpu {
 };
 
 struct SceneView {
-    const WideNodeGpu *tlas;
-    const WideNodeGpu *blas;
-    const float4 *tris;
+    const NodeGpu *nodes;  // the instance tree from node 0, then every mesh's tree
+    const TriGpu *tris;
+    const EntryGpu *entries;  // one per instance
     const InstanceGpu *instances;
     const MeshGpu *meshes;
     const float *positions;
