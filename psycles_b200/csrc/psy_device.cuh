@@ -368,8 +368,10 @@ struct ClosurePoint {
 // Shading routines are instantiated with and without glossy closures
 // (kGlossy): a scene without them runs code with no glossy branch, which
 // keeps the shading kernel's register budget where it was before them.
-constexpr uint32_t kLeavesOf(bool glossy) { return glossy ? 15u : 7u; }
 
+// The shading point's closures.  Without glossy closures they are the
+// material's baked list as it is; with them the point keeps a copy whose
+// glossy and dielectric closures carry what the point adds.
 template <bool kGlossy>
 struct SurfaceClosures {
     f3 normal;          // the diffuse closures' normal
@@ -377,6 +379,23 @@ struct SurfaceClosures {
     typename ClosureSlot<kGlossy>::type c[kMaxClosures];
     uint32_t count;
     f3 emission;
+    __device__ __forceinline__ const DielectricClosure &at(uint32_t i) const { return c[i]; }
+    __device__ __forceinline__ uint32_t op(uint32_t i) const { return c[i].op; }
+    __device__ __forceinline__ float sample_weight(uint32_t i) const { return c[i].sample_weight; }
+};
+template <>
+struct SurfaceClosures<false> {
+    f3 normal;
+    bool normal_exact;
+    const BakedClosureGpu *list;
+    uint32_t count;
+    f3 emission;
+    __device__ __forceinline__ PhysicalClosure at(uint32_t i) const {
+        const float4 w = __ldg(&list[i].weight), c = __ldg(&list[i].color);
+        return {ld3(w), w.w, __float_as_uint(c.w), ld3(c), __ldg(&list[i].params.x)};
+    }
+    __device__ __forceinline__ uint32_t op(uint32_t i) const { return __float_as_uint(__ldg(&list[i].color.w)); }
+    __device__ __forceinline__ float sample_weight(uint32_t i) const { return __ldg(&list[i].weight.w); }
 };
 
 __device__ __forceinline__ float closure_sample_weight(f3 w) { return fabsf((w.x + w.y + w.z) / 3.0f); }
@@ -674,101 +693,48 @@ __device__ __forceinline__ float f0_from_ior(float ior) {
 // keeps its signed weight, uses the cutoff on |average|, and every
 // allocated transparent contribution merges into the first one
 // (bsdf_transparent_setup, :483-518: summed weights and sample weights).
+// What does not depend on the shading point is baked (bake_material), the
+// rest is added by collect_surface.
+__device__ __forceinline__ BakedMaterialGpu bake_material(const SceneView &s, const MaterialGpu &m,
+                                                          BakedClosureGpu *closures);
+
 template <bool kGlossy>
-__device__ __forceinline__ void collect_surface(const SceneView &s, const MaterialGpu &m, const ClosurePoint &pt,
-                                    SurfaceClosures<kGlossy> &out) {
-    out.count = 0u;
-    out.emission = mk3(0.0f);
+__device__ __forceinline__ void collect_surface(const SceneView &s, const BakedMaterialGpu &m, const ClosurePoint &pt,
+                                                SurfaceClosures<kGlossy> &out) {
+    out.count = __float_as_uint(m.extinction.w);
+    out.emission = ld3(m.emission);
     out.normal = safe_normalize(pt.shading_normal, pt.shading_normal);
     out.normal_exact = out.normal.x == pt.shading_normal.x && out.normal.y == pt.shading_normal.y &&
                        out.normal.z == pt.shading_normal.z;
-    int transparent_slot = -1;
-    walk_closures<kLeavesOf(kGlossy)>(s, m, [&](uint32_t op, f3 w, f3 color, float roughness, float ior) {
-        if (op == PSY_CLOSURE_EMISSION) {
-            out.emission = out.emission + w;
-            return;
-        }
-        typename ClosureSlot<kGlossy>::type p;
-        p.op = op;
-        p.color = color;
-        p.roughness = roughness;
-        if constexpr (kGlossy) {
-            p.ior = 1.0f;
-            p.f0 = 0.0f;
-        }
-        if (op == PSY_CLOSURE_DIFFUSE) {
-            p.weight = bsdf_allocated_weight(w);
-            p.sample_weight = closure_sample_weight(p.weight);
-            if (!any_nonzero(p.weight)) return;
-        } else if (kGlossy && is_glossy(op)) {
-            const f3 allocated = max3(w, mk3(0.0f));
-            const float allocation = closure_sample_weight(allocated);
-            if (!(allocation >= 1.0e-5f)) return;
-            p.weight = allocated;
-            p.sample_weight = allocation * closure_sample_weight(mk3(1.0f));
-            p.color = specular_normal(pt.bump_correction, pt.geometric_normal, pt.view, out.normal);
-            if constexpr (kGlossy) {
-                if ((op & kGlossyMultiscatter) != 0u) {
-                    // ggx_energy (graph_surface_scattering.cpp:170-198) with the Fresnel
-                    // single-scattering albedo max(colour, 0); the weight takes the
-                    // darkening, evaluations the scale 1 / E
-                    const GgxEnergy e = ggx_energy(s, clampf_(roughness, 0.0f, 1.0f),
-                                                   clampf_(dot(p.color, pt.view), 0.0f, 1.0f), max3(color, mk3(0.0f)));
-                    p.weight = allocated * e.darkening;
-                    p.sample_weight = allocation * closure_sample_weight(e.darkening);
-                    p.f0 = e.energy_scale;
-                }
+    const BakedClosureGpu *list = s.closures + __float_as_uint(m.emission.w);
+    if constexpr (!kGlossy) {
+        out.list = list;
+    } else {
+        for (uint32_t i = 0; i < out.count; ++i) {
+            const float4 w = __ldg(&list[i].weight), c = __ldg(&list[i].color), q = __ldg(&list[i].params);
+            DielectricClosure p;
+            p.weight = ld3(w);
+            p.sample_weight = w.w;
+            p.op = __float_as_uint(c.w);
+            p.color = ld3(c);
+            p.roughness = q.x;
+            p.ior = pt.back_facing ? q.z : q.y;
+            p.f0 = q.w;
+            if (is_glossy(p.op) || is_refraction(p.op))
+                p.color = specular_normal(pt.bump_correction, pt.geometric_normal, pt.view, out.normal);
+            if ((p.op & kGlossyMultiscatter) != 0u) {
+                // ggx_energy (graph_surface_scattering.cpp:170-198) with the Fresnel
+                // single-scattering albedo max(colour, 0); the weight takes the
+                // darkening, evaluations the scale 1 / E
+                const GgxEnergy e = ggx_energy(s, clampf_(p.roughness, 0.0f, 1.0f),
+                                               clampf_(dot(p.color, pt.view), 0.0f, 1.0f), max3(ld3(c), mk3(0.0f)));
+                p.sample_weight = closure_sample_weight(p.weight) * closure_sample_weight(e.darkening);
+                p.weight = p.weight * e.darkening;
+                p.f0 = e.energy_scale;
             }
-        } else if (kGlossy && is_dielectric(op)) {
-            // MicrofacetGlassComponent::setup (microfacet_glass_component.cpp:180-232): the
-            // corrected normal, roughness sqrt(clamp(r^2)), the IOR inverted on a back
-            // face, weight max(weight, 0) (no energy preservation).  A glass closure's
-            // selection weight would also carry Cycles' tabulated Fresnel albedo; it is
-            // the only BSDF closure of its material (compile refuses other mixes), where
-            // that factor only rescales weighted_pdf / total, and is taken as one.
-            const f3 allocated = max3(w, mk3(0.0f));
-            const float allocation = closure_sample_weight(allocated);
-            if (!(allocation >= 1.0e-5f)) return;
-            p.weight = allocated;
-            p.sample_weight = allocation * 1.0f * closure_sample_weight(mk3(1.0f));
-            p.roughness = sqrtf(clampf_(roughness * roughness, 0.0f, 1.0f));
-            if constexpr (kGlossy) {
-                p.ior = pt.back_facing ? 1.0f / ior : ior;
-                p.f0 = clampf_(f0_from_ior(ior), 0.0f, 1.0f);
-            }
-            if (is_refraction(op)) p.color = specular_normal(pt.bump_correction, pt.geometric_normal, pt.view, out.normal);
-        } else {
-            const float sw = closure_sample_weight(w);
-            if (!(sw >= 1.0e-5f)) return;
-            if (transparent_slot >= 0) {
-                out.c[transparent_slot].weight = out.c[transparent_slot].weight + w;
-                out.c[transparent_slot].sample_weight += sw;
-                return;
-            }
-            p.weight = w;
-            p.sample_weight = sw;
+            out.c[i] = p;
         }
-        if (out.count >= kMaxClosures) return;
-        if (op == PSY_CLOSURE_TRANSPARENT) transparent_slot = int(out.count);
-        out.c[out.count++] = p;
-    });
-}
-
-__device__ __forceinline__ f3 material_emission(const SceneView &s, const MaterialGpu &m) {
-    f3 r = mk3(0.0f);
-    walk_closures<kLeafEmission>(s, m, [&](uint32_t op, f3 w, f3, float, float) {
-        if (op == PSY_CLOSURE_EMISSION) r = r + w;
-    });
-    return r;
-}
-
-// transparent_extinction (src/luisa/graph_surface_implementation.cpp:354-372).
-__device__ __forceinline__ f3 transparent_extinction(const SceneView &s, const MaterialGpu &m) {
-    f3 r = mk3(0.0f);
-    walk_closures<kLeafTransparent>(s, m, [&](uint32_t op, f3 w, f3, float, float) {
-        if (op == PSY_CLOSURE_TRANSPARENT && closure_sample_weight(w) >= 1.0e-5f) r = r + w;
-    });
-    return r;
+    }
 }
 
 constexpr uint32_t kEventReflection = 1u, kEventTransmission = 2u, kEventDiffuse = 4u, kEventGlossy = 8u,
@@ -802,19 +768,72 @@ __device__ __forceinline__ bool microfacet_singular(float roughness) {
     return a * a <= kMicrofacetSingularAlphaProduct;
 }
 
-// cycles_runtime_flags (src/luisa/graph_surface_scattering.cpp:292-365).
-template <bool kGlossy>
-__device__ __forceinline__ uint32_t runtime_flags(const SurfaceClosures<kGlossy> &s, bool back_facing) {
-    uint32_t f = back_facing ? kRuntimeBackfacing : 0u;
-    for (uint32_t i = 0; i < s.count; ++i) {
-        const auto &c = s.c[i];
-        if (c.op == PSY_CLOSURE_DIFFUSE) f |= kRuntimeBsdf | kRuntimeBsdfHasEval;
-        else if (is_glossy(c.op)) f |= kRuntimeBsdf | (microfacet_singular(c.roughness) ? 0u : kRuntimeBsdfHasEval);
-        else if (is_dielectric(c.op))
-            f |= kRuntimeBsdf | (microfacet_singular(c.roughness) ? 0u : kRuntimeBsdfHasEval) | kRuntimeBsdfHasTransmission;
-        else f |= kRuntimeBsdf | kRuntimeTransparent;
-    }
-    return f;
+__device__ __forceinline__ BakedMaterialGpu bake_material(const SceneView &s, const MaterialGpu &m,
+                                                          BakedClosureGpu *closures) {
+    f3 emission = mk3(0.0f), extinction = mk3(0.0f);
+    // cycles_runtime_flags (src/luisa/graph_surface_scattering.cpp:292-365)
+    uint32_t count = 0u, runtime = 0u;
+    int transparent_slot = -1;
+    walk_closures<kLeafAll>(s, m, [&](uint32_t op, f3 w, f3 color, float roughness, float ior) {
+        if (op == PSY_CLOSURE_EMISSION) {
+            emission = emission + w;
+            return;
+        }
+        f3 weight = w;
+        float sample_weight, f0 = 0.0f, back_ior = 1.0f;
+        if (op == PSY_CLOSURE_DIFFUSE) {
+            weight = bsdf_allocated_weight(w);
+            sample_weight = closure_sample_weight(weight);
+            if (!any_nonzero(weight)) return;
+        } else if (is_glossy(op)) {
+            weight = max3(w, mk3(0.0f));
+            sample_weight = closure_sample_weight(weight);
+            if (!(sample_weight >= 1.0e-5f)) return;
+            sample_weight = sample_weight * closure_sample_weight(mk3(1.0f));
+        } else if (is_dielectric(op)) {
+            // MicrofacetGlassComponent::setup (microfacet_glass_component.cpp:180-232): the
+            // corrected normal, roughness sqrt(clamp(r^2)), the IOR inverted on a back
+            // face, weight max(weight, 0) (no energy preservation).  A glass closure's
+            // selection weight would also carry Cycles' tabulated Fresnel albedo; it is
+            // the only BSDF closure of its material (compile refuses other mixes), where
+            // that factor only rescales weighted_pdf / total, and is taken as one.
+            weight = max3(w, mk3(0.0f));
+            sample_weight = closure_sample_weight(weight);
+            if (!(sample_weight >= 1.0e-5f)) return;
+            sample_weight = sample_weight * 1.0f * closure_sample_weight(mk3(1.0f));
+            roughness = sqrtf(clampf_(roughness * roughness, 0.0f, 1.0f));
+            back_ior = 1.0f / ior;
+            f0 = clampf_(f0_from_ior(ior), 0.0f, 1.0f);
+        } else {
+            // transparent_extinction (src/luisa/graph_surface_implementation.cpp:354-372)
+            sample_weight = closure_sample_weight(w);
+            if (!(sample_weight >= 1.0e-5f)) return;
+            extinction = extinction + w;
+            if (transparent_slot >= 0) {
+                float4 &t = closures[transparent_slot].weight;
+                t = make_float4(t.x + w.x, t.y + w.y, t.z + w.z, t.w + sample_weight);
+                return;
+            }
+        }
+        if (op == PSY_CLOSURE_DIFFUSE) runtime |= kRuntimeBsdf | kRuntimeBsdfHasEval;
+        else if (is_glossy(op)) runtime |= kRuntimeBsdf | (microfacet_singular(roughness) ? 0u : kRuntimeBsdfHasEval);
+        else if (is_dielectric(op))
+            runtime |= kRuntimeBsdf | (microfacet_singular(roughness) ? 0u : kRuntimeBsdfHasEval) | kRuntimeBsdfHasTransmission;
+        else runtime |= kRuntimeBsdf | kRuntimeTransparent;
+        if (count >= kMaxClosures) return;
+        if (op == PSY_CLOSURE_TRANSPARENT) transparent_slot = int(count);
+        closures[count++] = BakedClosureGpu{make_float4(weight.x, weight.y, weight.z, sample_weight),
+                                            make_float4(color.x, color.y, color.z, __uint_as_float(op)),
+                                            make_float4(roughness, ior, back_ior, f0)};
+    });
+    BakedMaterialGpu b;
+    b.emission = make_float4(emission.x, emission.y, emission.z, __uint_as_float(m.closure_first));
+    b.extinction = make_float4(extinction.x, extinction.y, extinction.z, __uint_as_float(count));
+    b.runtime = runtime;
+    b.emission_sampling = m.emission_sampling;
+    b.has_emission = m.has_emission;
+    b.bump_correction = m.bump_correction;
+    return b;
 }
 
 // bump_shadowing_term (src/luisa/graph_surface_scattering.cpp:219-281) of a
@@ -1089,7 +1108,7 @@ __device__ __noinline__ Evaluation evaluate_mixture(const SurfaceClosures<kGloss
         s.normal_exact ? 1.0f : bump_shadowing_general(pt.shading_normal, n, outgoing, true, true, pt.bump_correction);
     const float lambert = nl * kInvPi;
     for (uint32_t i = 0; i < s.count; ++i) {
-        const auto &c = s.c[i];
+        const auto c = s.at(i);
         if (c.op == PSY_CLOSURE_TRANSPARENT) {
             if (transparent_enabled) total += c.sample_weight;
             continue;
@@ -1209,14 +1228,14 @@ __device__ __forceinline__ SurfaceSample sample_surface(const SurfaceClosures<kG
     out.eval = {mk3(0.0f), 0.0f, 0u};
     out.closure_index = kInvalid;
     float total = 0.0f;
-    for (uint32_t i = 0; i < s.count; ++i) total += closure_eligible(s.c[i].op, lobe_mask) ? s.c[i].sample_weight : 0.0f;
+    for (uint32_t i = 0; i < s.count; ++i) total += closure_eligible(s.op(i), lobe_mask) ? s.sample_weight(i) : 0.0f;
     const float random_lobe = clampf_(u_lobe, 0.0f, 0.99999994f);
     const float target = random_lobe * total;
     float accumulated = 0.0f;
     int chosen = -1;
     float chosen_weight = 0.0f, rescaled = random_lobe;
     for (uint32_t i = 0; i < s.count; ++i) {
-        const float w = closure_eligible(s.c[i].op, lobe_mask) ? s.c[i].sample_weight : 0.0f;
+        const float w = closure_eligible(s.op(i), lobe_mask) ? s.sample_weight(i) : 0.0f;
         const float next = accumulated + w;
         if (chosen < 0 && w > 0.0f && target < next) {
             chosen = int(i);
@@ -1228,7 +1247,7 @@ __device__ __forceinline__ SurfaceSample sample_surface(const SurfaceClosures<kG
         accumulated = next;
     }
     if (chosen < 0) return out;
-    const auto c = s.c[chosen];
+    const auto c = s.at(uint32_t(chosen));
     const bool transparent = c.op == PSY_CLOSURE_TRANSPARENT;
     const bool glossy = kGlossy && is_glossy(c.op);
     const bool dielectric = kGlossy && is_dielectric(c.op);
@@ -1302,7 +1321,7 @@ __device__ __forceinline__ void surface_aov(const SurfaceClosures<kGlossy> &s, c
     f3 n = mk3(0.0f);
     float total = 0.0f;
     for (uint32_t i = 0; i < s.count; ++i) {
-        const auto &c = s.c[i];
+        const auto c = s.at(i);
         if (c.op == PSY_CLOSURE_DIFFUSE) {
             albedo = albedo + c.weight;
             const float w = closure_sample_weight(c.weight);

@@ -888,8 +888,9 @@ psy_status clear_film(psy_session *s, bool sync = true) {
 // Checks a compiled SurfaceProgram against what the kernels interpret: the
 // in-scope closure and value operations, operands that name earlier value
 // instructions of the right type, parameter slots inside the block, and
-// closure inputs of the type their socket takes.
-psy_status validate_material(const psy_material_desc &m) {
+// closure inputs of the type their socket takes.  `closures` receives the most
+// BSDF closures the program can allocate.
+psy_status validate_material(const psy_material_desc &m, uint32_t *closures) {
     if (m.closure_count == 0u || !m.closures || m.root >= m.closure_count)
         return fail(PSY_ERROR_INVALID_ARGUMENT, "material without a valid closure root");
     if (m.value_count > psy::kMaxValues)
@@ -1004,6 +1005,7 @@ psy_status validate_material(const psy_material_desc &m) {
     // tabulated Fresnel albedo, which this build does not carry
     if (glass && leaves + (transparent ? 1u : 0u) > 1u)
         return fail(PSY_ERROR_UNSUPPORTED, "a glass closure must be the only BSDF closure of its material");
+    *closures = leaves + (transparent ? 1u : 0u);
     return PSY_OK;
 }
 
@@ -1152,6 +1154,19 @@ cudaError_t replace_buffer(psy_scene *sc, DeviceBuffer &slot, const std::vector<
     return cudaSuccess;
 }
 
+// Replaces a device buffer by a stream-ordered copy of itself, for an edit
+// of part of it; the old one is retired.
+cudaError_t copy_buffer(psy_scene *sc, DeviceBuffer &slot) {
+    auto fresh = std::make_unique<DeviceBuffer>(sc->context->stream);
+    cudaError_t e = fresh->alloc(slot.bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyAsync(fresh->ptr, slot.ptr, slot.bytes, cudaMemcpyDeviceToDevice, sc->context->stream);
+    if (e != cudaSuccess) return e;
+    slot.swap(*fresh);
+    if (fresh->ptr) sc->retired.push_back(std::move(fresh));
+    return cudaSuccess;
+}
+
 // The many-light tree over the scene's emitter population -- emissive
 // triangles in emitter order, then the analytic lights -- built from the
 // host copies and uploaded (src/luisa/path_tracer_light_sampling_scene.cpp:
@@ -1276,6 +1291,13 @@ psy_status psy::host::rebind_parameters_versioned(psy_scene *s, uint32_t materia
     PSY_CUDA_TRY(replace_buffer(s, s->vector_buf, s->vectors));
     s->view.scalars = s->scalar_buf.as<float>();
     s->view.vectors = s->vector_buf.as<float>();
+    PSY_CUDA_TRY(copy_buffer(s, s->baked));
+    PSY_CUDA_TRY(copy_buffer(s, s->closures));
+    s->view.baked = s->baked.as<psy::BakedMaterialGpu>();
+    s->view.closures = s->closures.as<psy::BakedClosureGpu>();
+    psy::launch_bake_materials(s->context->stream, s->view, s->baked.as<psy::BakedMaterialGpu>(),
+                               s->closures.as<psy::BakedClosureGpu>(), material, 1u);
+    PSY_CUDA_TRY(cudaGetLastError());
     if (m.has_emission) {
         std::lock_guard<std::mutex> lock(s->light_tree_mutex);
         if (s->light_tree_built) {
@@ -1445,8 +1467,9 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
                     return fail(PSY_ERROR_INVALID_ARGUMENT, "triangle material out of range");
         if (m.smooth && !m.normals) return fail(PSY_ERROR_INVALID_ARGUMENT, "smooth mesh without normals");
     }
+    std::vector<uint32_t> closure_capacity(d->material_count);  // the most BSDF closures each material can allocate
     for (uint32_t i = 0; i < d->material_count; ++i) {
-        const psy_status valid = validate_material(d->materials[i]);
+        const psy_status valid = validate_material(d->materials[i], &closure_capacity[i]);
         if (valid != PSY_OK) return valid;
     }
     for (uint32_t i = 0; i < d->light_count; ++i) {
@@ -1710,6 +1733,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     std::vector<psy_closure_instruction> code;
     std::vector<psy_value_instruction> values;
     bool any_transparent = false, any_glossy = false;
+    uint32_t baked_closures = 0u;
     for (uint32_t i = 0; i < d->material_count; ++i) {
         const psy_material_desc &m = d->materials[i];
         psy::MaterialGpu g{};
@@ -1722,6 +1746,8 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         g.scalar_offset = uint32_t(sc->scalars.size());
         g.vector_offset = uint32_t(sc->vectors.size() / 3u);
         g.emission_sampling = m.emission_sampling;
+        g.closure_first = baked_closures;
+        baked_closures += closure_capacity[i];
         g.bump_correction = (m.flags & PSY_MATERIAL_NO_BUMP_MAP_CORRECTION) == 0u ? 1u : 0u;
         for (uint32_t k = 0; k < m.closure_count; ++k) {
             if (m.closures[k].op == PSY_CLOSURE_EMISSION) g.has_emission = 1u;
@@ -1883,7 +1909,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // back, and parameter blocks replaced by edits are retired without
     // waiting on the device.
     for (DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions, &sc->normals,
-                            &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->code, &sc->value_buf, &sc->scalar_buf,
+                            &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->baked, &sc->closures, &sc->code, &sc->value_buf, &sc->scalar_buf,
                             &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights, &sc->lamp_consts,
                             &sc->lamp_bounds, &sc->lamp_ids})
         b->ordered = st;
@@ -1897,6 +1923,8 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     PSY_CUDA_TRY(sc->indices.upload(indices, st));
     PSY_CUDA_TRY(sc->tri_materials.upload(tri_materials, st));
     PSY_CUDA_TRY(sc->material_buf.upload(sc->materials, st));
+    PSY_CUDA_TRY(sc->baked.alloc(sizeof(psy::BakedMaterialGpu) * std::max<size_t>(sc->materials.size(), 1u)));
+    PSY_CUDA_TRY(sc->closures.alloc(sizeof(psy::BakedClosureGpu) * std::max(baked_closures, 1u)));
     PSY_CUDA_TRY(sc->code.upload(code, st));
     PSY_CUDA_TRY(sc->value_buf.upload(values, st));
     PSY_CUDA_TRY(sc->scalar_buf.upload(sc->scalars, st));
@@ -1937,7 +1965,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     PSY_CUDA_TRY(cudaStreamSynchronize(st));
     sc->stats.upload_bytes = 0u;
     for (const DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions,
-                                  &sc->normals, &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->code,
+                                  &sc->normals, &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->baked, &sc->closures, &sc->code,
                                   &sc->value_buf, &sc->scalar_buf, &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights,
                                   &sc->lamp_consts, &sc->lamp_bounds, &sc->lamp_ids})
         sc->stats.upload_bytes += b->bytes;
@@ -1952,6 +1980,8 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     v.indices = sc->indices.as<uint32_t>();
     v.tri_materials = sc->tri_materials.as<uint32_t>();
     v.materials = sc->material_buf.as<psy::MaterialGpu>();
+    v.baked = sc->baked.as<psy::BakedMaterialGpu>();
+    v.closures = sc->closures.as<psy::BakedClosureGpu>();
     v.code = sc->code.as<psy_closure_instruction>();
     v.values = sc->value_buf.as<psy_value_instruction>();
     v.scalars = sc->scalar_buf.as<float>();
@@ -1982,6 +2012,10 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     v.world_visibility = d->world_visibility;
     v.any_transparent = any_transparent ? 1u : 0u;
     v.has_glossy = any_glossy ? 1u : 0u;
+    psy::launch_bake_materials(st, v, sc->baked.as<psy::BakedMaterialGpu>(), sc->closures.as<psy::BakedClosureGpu>(), 0u,
+                               uint32_t(sc->materials.size()));
+    PSY_CUDA_TRY(cudaGetLastError());
+    PSY_CUDA_TRY(cudaStreamSynchronize(st));
     // the light tree is built on first use (ensure_light_tree)
     sc->stats.upload_ms = lap();
     sc->stats.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_begin).count();
@@ -2018,6 +2052,9 @@ psy_status psy_scene_rebind_parameters(psy_scene *s, uint32_t material, const fl
         PSY_CUDA_TRY(cudaMemcpyAsync(s->vector_buf.as<float>() + 3ull * m.vector_offset, vectors,
                                      sizeof(float) * 3u * vector_count, cudaMemcpyHostToDevice, st));
     }
+    psy::launch_bake_materials(st, s->view, s->baked.as<psy::BakedMaterialGpu>(), s->closures.as<psy::BakedClosureGpu>(),
+                               material, 1u);
+    PSY_CUDA_TRY(cudaGetLastError());
     PSY_CUDA_TRY(cudaStreamSynchronize(st));
     // the light tree's energies follow the emission estimates: rebuild a
     // built tree when an emissive material changes, as a recompile would
@@ -2161,7 +2198,7 @@ psy_status psy_session_read_trace(psy_session *s, psy_path_trace *out) {
 uint64_t psy::host::scene_device_bytes(const psy_scene *s) {
     uint64_t n = 0u;
     for (const DeviceBuffer *b : {&s->nodes, &s->entries, &s->tris, &s->instances, &s->meshes, &s->positions, &s->normals,
-                                  &s->indices, &s->tri_materials, &s->material_buf, &s->code, &s->value_buf, &s->scalar_buf,
+                                  &s->indices, &s->tri_materials, &s->material_buf, &s->baked, &s->closures, &s->code, &s->value_buf, &s->scalar_buf,
                                   &s->vector_buf, &s->emitters, &s->distribution, &s->ggx_tables, &s->lights, &s->lamp_consts, &s->lamp_bounds,
                                   &s->lamp_ids, &s->lt_nodes, &s->lt_emitters, &s->lt_mapping, &s->lt_lookup})
         n += b->bytes;

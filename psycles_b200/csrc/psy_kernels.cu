@@ -207,7 +207,7 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 // register budgets (64 and 80) give the latency more warps to hide in: 155 and 117 ms at
 // 8 and 5 blocks of 128 an SM, 169 and 134 ms at 6 and 4, 154 at 9 for
 // closest hits.  Together 224 -> 144 ms for closest hits and 185 -> 108 ms for
-// shadow rays.
+// shadow rays, and 82 ms (8 blocks; 88 at 6) since they read baked materials.
 #ifndef PSY_REFILL_LANES
 #define PSY_REFILL_LANES 12
 #endif
@@ -218,7 +218,7 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 #define PSY_SHADE_MIN_BLOCKS 3
 #endif
 #ifndef PSY_SHADOW_MIN_BLOCKS
-#define PSY_SHADOW_MIN_BLOCKS 6
+#define PSY_SHADOW_MIN_BLOCKS 8
 #endif
 // Lanes that finish before a warp is refilled.
 constexpr int kRefillLanes = PSY_REFILL_LANES;
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                     ev->hit_primitive = h.cycles_prim;
                 }
                 const SurfacePoint sp = surface_point(s, h, ray.d);
-                const MaterialGpu mat = s.materials[sp.material];
+                const BakedMaterialGpu mat = s.baked[sp.material];
                 SurfaceClosures<kGlossy> closures;
                 const ClosurePoint cpt{sp.n, sp.ng, -ray.d, safe_normalize(-ray.d, sp.n), mat.bump_correction != 0u,
                                        sp.back_facing};
@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                             ps.flag |= kFlagSinglePassDone;
                         }
                     }
-                    const uint32_t runtime = runtime_flags(closures, sp.back_facing);
+                    const uint32_t runtime = mat.runtime | (sp.back_facing ? kRuntimeBackfacing : 0u);
                     if (p.use_light_tree) {
                         // light-tree pick after shading (src/luisa/path_kernel_pipeline.cpp:150-159)
                         selected = lt_sample(s, light_sample.z, sp.position, sp.n,
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                                 const bool reject_self = same_primitive && dot(ls.direction, oriented) > 0.0f;
                                 if (!reject_self) {
                                     sampled = true;
-                                    light_radiance = material_emission(s, s.materials[em.material]);
+                                    light_radiance = ld3(__ldg(&s.baked[em.material].emission));
                                     light_pdf = pdf;
                                     pdf_divisor = pdf;
                                     lp = ls.position;
@@ -1000,6 +1000,21 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
     }
 }
 
+// Evaluates the closure programs of materials [first, first + count), one
+// material a thread (microseconds, when a scene is compiled or a material
+// edited).  While shading and shadow rays walked the programs per path, the
+// walk's arrays took 1.6 of the shading kernel's 1.9 KB of local memory and
+// most of the shadow kernel's, whose register budget they also held up: 1080p
+// procedural frame, 64 spp: shading 182 -> 148 ms, shadow rays 108 -> 82 ms (now
+// 8 blocks an SM); value programs, 512x512 at 4 spp: 5.3 -> 2.7 ms.
+__global__ void k_bake_materials(const __grid_constant__ SceneView s, BakedMaterialGpu *baked, BakedClosureGpu *closures,
+                                 uint32_t first, uint32_t count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const MaterialGpu m = s.materials[first + i];
+    baked[first + i] = bake_material(s, m, closures + m.closure_first);
+}
+
 // ------------------------------------------------------------------ shadow
 // make_trace_shadow_callable (src/luisa/path_tracer_geometry.cpp:75-174)
 // iterates closest hits: a transparent surface multiplies its extinction
@@ -1125,7 +1140,7 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
                 lm[j + 1] = km;
             }
             for (int i = 0; i < n; ++i) {
-                const f3 e = clamp3(transparent_extinction(s, s.materials[lm[i]]), 0.0f, 1.0f);
+                const f3 e = clamp3(ld3(__ldg(&s.baked[lm[i]].extinction)), 0.0f, 1.0f);
                 if (!(max_component(e) > 0.0f)) {
                     blocked = true;
                     break;
@@ -1487,6 +1502,11 @@ void launch_debug_light_tree(cudaStream_t st, const SceneView &s, const float4 *
 void launch_debug_light_distribution(cudaStream_t st, const SceneView &s, const float *u, uint32_t count,
                                      uint32_t *out_kind, uint32_t *out_index, float *out_pdf) {
     k_debug_light_distribution<<<(count + 127u) / 128u, 128, 0, st>>>(s, u, count, out_kind, out_index, out_pdf);
+}
+void launch_bake_materials(cudaStream_t st, const SceneView &s, BakedMaterialGpu *baked, BakedClosureGpu *closures,
+                           uint32_t first, uint32_t count) {
+    if (count == 0u) return;
+    k_bake_materials<<<(count + 31u) / 32u, 32, 0, st>>>(s, baked, closures, first, count);
 }
 void launch_debug_sobol(cudaStream_t st, const float4 *table, uint32_t size, const uint32_t *queries, uint32_t count,
                         float4 *out, uint32_t *out_index) {

@@ -40,6 +40,10 @@ void launch_count_rays(cudaStream_t st, const uint32_t *counters, unsigned long 
 void launch_check_counts(cudaStream_t st, const uint32_t *counts, uint32_t n, uint32_t expected, uint32_t *mismatch);
 void launch_resolve_pass(cudaStream_t st, const float4 *film, const uint32_t *counts, uint32_t n, uint32_t kind,
                          float exposure, float *out);
+// Evaluates the closure programs of materials [first, first + count) of `s`
+// from its parameter blocks into the baked tables.
+void launch_bake_materials(cudaStream_t st, const SceneView &s, BakedMaterialGpu *baked, BakedClosureGpu *closures,
+                           uint32_t first, uint32_t count);
 void launch_film(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t pixels, uint32_t samples, float4 *combined,
                  float4 *normal, float4 *albedo, uint32_t *sample_count, uint32_t trace_path, psy_path_trace *trace);
 // Batched wavefront.  round (device memory): paths, film pixels, items.

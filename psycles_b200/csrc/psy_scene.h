@@ -11,6 +11,7 @@
 //   instances     InstanceGpu (object<->world transforms, mesh, material)
 //   materials / code / scalars / vectors  closure programs and their
 //                 parameter blocks (rebinding rewrites scalars/vectors)
+//   baked / closures  the programs evaluated, as the kernels shade with them
 //   emitters / distribution  emissive triangles and the flat light CDF
 //   lights        analytic lights (psy_light_desc)
 #pragma once
@@ -97,7 +98,25 @@ struct alignas(16) MaterialGpu {
     uint32_t vector_offset, emission_sampling, has_emission, has_transparent;
     uint32_t value_offset, value_count;
     uint32_t bump_correction;  // contract::Material::use_bump_map_correction
-    uint32_t pad0;
+    uint32_t closure_first;    // first of the material's baked closures
+};
+
+// A material's closure program evaluated: nothing in it depends on the
+// shading point (no textures or context values), so k_bake_materials walks
+// it once when the scene is compiled or the material's parameters are
+// edited, and shading reads the result.
+struct alignas(16) BakedMaterialGpu {
+    float4 emission;    // xyz: summed emission; w: bits of the first baked closure's index
+    float4 extinction;  // xyz: summed transparent weight (a shadow ray's factor); w: bits of the closure count
+    uint32_t runtime;   // the closures' runtime flags
+    uint32_t emission_sampling, has_emission, bump_correction;
+};
+// A BSDF closure of the shading point's list, up to what its normal and side
+// add (glossy normals, the IOR of a back face, MULTI_GGX's energy factors).
+struct alignas(16) BakedClosureGpu {
+    float4 weight;  // w: sample weight
+    float4 color;   // w: op bits
+    float4 params;  // roughness, IOR, IOR of a back face, F0
 };
 
 // Value instructions a material's program may hold (its stream is
@@ -140,6 +159,8 @@ struct SceneView {
     const uint32_t *indices;
     const uint32_t *tri_materials;
     const MaterialGpu *materials;
+    const BakedMaterialGpu *baked;    // one per material
+    const BakedClosureGpu *closures;
     const psy_closure_instruction *code;
     const psy_value_instruction *values;
     const float *scalars;
