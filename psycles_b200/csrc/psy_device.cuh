@@ -1347,7 +1347,7 @@ struct Ray {
 
 struct Hit {
     float t, u, v;
-    uint32_t instance, prim, object, cycles_prim;
+    uint32_t instance, prim, object;
 };
 
 // clamp_bvh_direction (cycles_triangle_intersection_component.cpp:31-37).
@@ -1385,10 +1385,6 @@ __device__ __forceinline__ bool intersect_triangle(f3 o, f3 d, float tmin, float
     u_out = minf_(u * rs, 1.0f);
     v_out = minf_(v * rs, 1.0f);
     return true;
-}
-
-__device__ __forceinline__ Xform load_xform(const float *m) {
-    return {ld3(m), ld3(m + 3), ld3(m + 6), ld3(m + 9)};
 }
 
 constexpr uint32_t kStackSize = kTraversalStackSize + 1u;  // the end marker lies below the entries
@@ -1692,26 +1688,33 @@ __device__ __forceinline__ f3 tri_interp(float u, float v, f3 a, f3 b, f3 c) {
 // for instanced meshes.
 __device__ __forceinline__ SurfacePoint surface_point(const SceneView &s, const Hit &h, f3 ray_d) {
     SurfacePoint sp;
-    const InstanceGpu &inst = s.instances[h.instance];
-    const MeshGpu mesh = s.meshes[inst.mesh];
-    const uint32_t *idx = s.indices + mesh.index_offset + 3u * h.prim;
-    const uint32_t i0 = idx[0], i1 = idx[1], i2 = idx[2];
-    const float *P = s.positions + 3u * mesh.vertex_offset;
-    sp.p0 = ld3(P + 3u * i0);
-    sp.p1 = ld3(P + 3u * i1);
-    sp.p2 = ld3(P + 3u * i2);
-    const Xform o2w = load_xform(inst.o2w);
-    const Xform nrm = load_xform(inst.nrm);
+    const InstanceGpu *ip = s.instances + h.instance;
+    uint4 i0, i1, i2, i3, i4, i5;
+    load_sector_nc(ip, i0, i1);
+    load_sector_nc(ip->o2w + 8, i2, i3);
+    load_sector_nc(ip->nrm + 4, i4, i5);
+    const float4 m0 = floats4(i0), m1 = floats4(i1), m2 = floats4(i2), m3 = floats4(i3), m4 = floats4(i4);
+    const Xform o2w{mk3(m0.x, m0.y, m0.z), mk3(m0.w, m1.x, m1.y), mk3(m1.z, m1.w, m2.x), mk3(m2.y, m2.z, m2.w)};
+    const Xform nrm{mk3(m3.x, m3.y, m3.z), mk3(m3.w, m4.x, m4.y), mk3(m4.z, m4.w, __uint_as_float(i5.x)), mk3(0.0f)};
+    sp.cycles_prim = i5.y + h.prim;
+    const ShadeTriGpu *tp = s.shade_tris + sp.cycles_prim;
+    uint4 u0, u1, u2, u3, u4, u5;
+    load_sector_nc(tp, u0, u1);
+    load_sector_nc(tp->p2 + 2, u2, u3);
+    load_sector_nc(tp->n2 + 1, u4, u5);
+    const float4 t0 = floats4(u0), t1 = floats4(u1), t2 = floats4(u2), t3 = floats4(u3), t4 = floats4(u4),
+                 t5 = floats4(u5);
+    sp.p0 = mk3(t0.x, t0.y, t0.z);
+    sp.p1 = mk3(t0.w, t1.x, t1.y);
+    sp.p2 = mk3(t1.z, t1.w, t2.x);
     sp.wp0 = xform_point(o2w, sp.p0);
     sp.wp1 = xform_point(o2w, sp.p1);
     sp.wp2 = xform_point(o2w, sp.p2);
-    const f3 ogn = safe_normalize(cross(sp.p1 - sp.p0, sp.p2 - sp.p0), mk3(0.0f, 0.0f, 1.0f));
+    const f3 ogn = mk3(t4.z, t4.w, t5.x);
     f3 ng = safe_normalize(xform_direction(nrm, ogn), -ray_d);
     f3 osn = ogn;
-    if (mesh.smooth) {
-        const float *N = s.normals + 3u * mesh.vertex_offset;
-        osn = tri_interp(h.u, h.v, ld3(N + 3u * i0), ld3(N + 3u * i1), ld3(N + 3u * i2));
-    }
+    if (i5.z != 0u)
+        osn = tri_interp(h.u, h.v, mk3(t2.y, t2.z, t2.w), mk3(t3.x, t3.y, t3.z), mk3(t3.w, t4.x, t4.y));
     f3 n = safe_normalize(xform_direction(nrm, osn), ng);
     sp.back_facing = dot(ng, -ray_d) < 0.0f;
     if (sp.back_facing) {
@@ -1724,10 +1727,32 @@ __device__ __forceinline__ SurfacePoint surface_point(const SceneView &s, const 
     sp.object_position = sp.p0 + (sp.p1 - sp.p0) * h.u + (sp.p2 - sp.p0) * h.v;
     sp.position = xform_point(o2w, sp.object_position);
     sp.instance = h.instance;
-    sp.material = mesh.material_offset == kInvalid ? inst.material : s.tri_materials[mesh.material_offset + h.prim];
+    sp.material = (i5.w != kInvalid ? i5.w : u5.y) & ~kMaterialTransparent;
     sp.object = h.object;
-    sp.cycles_prim = h.cycles_prim;
     return sp;
+}
+
+// An emissive triangle's record in four 16-byte loads and a word.
+struct Emitter {
+    f3 p0, p1, p2, ng;
+    float area;
+    uint32_t material, object, cycles_prim, emission_sampling;
+};
+__device__ __forceinline__ Emitter load_emitter(const EmitterGpu *e) {
+    const float4 *p = reinterpret_cast<const float4 *>(e);
+    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+    return {mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), mk3(b.z, b.w, c.x), mk3(c.y, c.z, c.w), d.x,
+            __float_as_uint(d.y), __float_as_uint(d.z), __float_as_uint(d.w), __ldg(&e->emission_sampling)};
+}
+
+// An instance's world-to-object transform.
+__device__ __forceinline__ Xform world_to_object(const SceneView &s, uint32_t instance) {
+    uint4 w0, w1, w2, w3;
+    const InstanceGpu *ip = s.instances + instance;
+    load_sector_nc(ip->w2o, w0, w1);
+    load_sector_nc(ip->w2o + 8, w2, w3);
+    const float4 a = floats4(w0), b = floats4(w1), c = floats4(w2);
+    return {mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), mk3(b.z, b.w, c.x), mk3(c.y, c.z, c.w)};
 }
 
 // Wachter & Binder robust offset (Ray Tracing Gems ch. 6), the published

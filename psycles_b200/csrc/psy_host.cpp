@@ -1502,15 +1502,15 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     std::vector<float> positions, normals;
     std::vector<uint32_t> indices, tri_materials;
     std::vector<psy::NodeGpu> nodes;
-    std::vector<psy::TriGpu> tris;
+    std::vector<uint32_t> order;  // per leaf slot of all meshes, the mesh's triangle
     std::vector<Box> mesh_boxes(d->mesh_count);
     std::vector<std::vector<WideNode>> mesh_wide(d->mesh_count);
-    // triangle records in BVH leaf order, written by each mesh's build at
-    // the mesh's offset (meshes in input order)
+    // triangles in BVH leaf order, written by each mesh's build at the mesh's
+    // offset (meshes in input order)
     std::vector<uint64_t> mesh_tri_first(d->mesh_count + 1u, 0u);
     for (uint32_t i = 0; i < d->mesh_count; ++i) mesh_tri_first[i + 1u] = mesh_tri_first[i] + d->meshes[i].triangle_count;
-    tris.resize(mesh_tri_first[d->mesh_count]);
-    // one mesh's BLAS, its triangle records in leaf order and its stack need
+    order.resize(mesh_tri_first[d->mesh_count]);
+    // one mesh's BLAS, its triangles in leaf order and its stack need
     std::vector<uint32_t> mesh_need(d->mesh_count, 0u);
     auto build_mesh = [&](uint32_t i, int sah_depth_limit) {
         const psy_mesh_desc &m = d->meshes[i];
@@ -1527,20 +1527,11 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
             p.id = k;
         }
         mesh_boxes[i] = bld.build_root();
-        std::vector<uint32_t> order;
-        mesh_wide[i] = bld.widen(order);
+        std::vector<uint32_t> leaves;
+        mesh_wide[i] = bld.widen(leaves);
         mesh_need[i] = blas_stack_need(mesh_wide[i]);
-        psy::TriGpu *out = tris.data() + mesh_tri_first[i];
-        for (const uint32_t leaf : order) {
-            const uint32_t id = bld.prims[leaf].id;
-            float4 v[3];
-            for (int c = 0; c < 3; ++c) {
-                const float *p = m.positions + 3ull * m.indices[3ull * id + c];
-                v[c] = make_float4(p[0], p[1], p[2], 0.0f);
-            }
-            std::memcpy(&v[0].w, &id, 4);
-            *out++ = psy::TriGpu{v[0], v[1], v[2], make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
-        }
+        uint32_t *out = order.data() + mesh_tri_first[i];
+        for (const uint32_t leaf : leaves) *out++ = bld.prims[leaf].id;
     };
     {
         std::vector<uint32_t> by_size(d->mesh_count);
@@ -1568,13 +1559,17 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         nrm.c0 = {w2o.c0.x, w2o.c1.x, w2o.c2.x};
         nrm.c1 = {w2o.c0.y, w2o.c1.y, w2o.c2.y};
         nrm.c2 = {w2o.c0.z, w2o.c1.z, w2o.c2.z};
-        nrm.c3 = {0.0f, 0.0f, 0.0f};
         store34(g.o2w, o2w[i]);
         store34(g.w2o, w2o);
-        store34(g.nrm, nrm);
+        const V3 columns[3] = {nrm.c0, nrm.c1, nrm.c2};
+        for (int c = 0; c < 3; ++c) {
+            g.nrm[3 * c] = columns[c].x;
+            g.nrm[3 * c + 1] = columns[c].y;
+            g.nrm[3 * c + 2] = columns[c].z;
+        }
         g.mesh = id.mesh;
-        g.material = id.material;
         g.visibility = id.visibility;
+        g.pad[0] = g.pad[1] = 0u;
     }
     // Instance boxes: the world-space bounds of the instance's transformed
     // vertices (the mesh box's transformed corners would be up to about 1.7
@@ -1671,16 +1666,14 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     }
 
     uint32_t node_count = uint32_t(tl_wide.size());
-    uint32_t prim_offset = 0;
+    std::vector<uint32_t> node_offsets(d->mesh_count);
     for (uint32_t i = 0; i < d->mesh_count; ++i) {
         const psy_mesh_desc &m = d->meshes[i];
         psy::MeshGpu &g = meshes[i];
         g.vertex_offset = uint32_t(positions.size() / 3u);
         g.index_offset = uint32_t(indices.size());
         g.triangle_count = m.triangle_count;
-        g.prim_offset = prim_offset;
         g.smooth = m.smooth ? 1u : 0u;
-        prim_offset += m.triangle_count;
         positions.insert(positions.end(), m.positions, m.positions + 3ull * m.vertex_count);
         if (m.smooth) normals.insert(normals.end(), m.normals, m.normals + 3ull * m.vertex_count);
         else normals.resize(positions.size(), 0.0f);
@@ -1692,7 +1685,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
             g.material_offset = psy::kInvalidId;
         }
         g.tri_offset = uint32_t(mesh_tri_first[i]);
-        g.node_offset = node_count;
+        node_offsets[i] = node_count;
         node_count += uint32_t(mesh_wide[i].size());
         sc->triangle_count += m.triangle_count;
     }
@@ -1709,7 +1702,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         for (size_t f = 0; f < tl_wide.size(); f += kNodeChunk) node_jobs.push_back({&tl_wide, f, 0u, 0u});
         for (uint32_t i = 0; i < d->mesh_count; ++i)
             for (size_t f = 0; f < mesh_wide[i].size(); f += kNodeChunk)
-                node_jobs.push_back({&mesh_wide[i], f, meshes[i].node_offset, meshes[i].tri_offset});
+                node_jobs.push_back({&mesh_wide[i], f, node_offsets[i], meshes[i].tri_offset});
         const psy_status quantised = parallel_for(uint32_t(node_jobs.size()), nullptr, [&](uint32_t job) {
             const NodeJob &j = node_jobs[job];
             const size_t end = std::min(j.wide->size(), j.first + kNodeChunk);
@@ -1718,15 +1711,30 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         });
         if (quantised != PSY_OK) return quantised;
     }
+    // a material index with kMaterialTransparent where its program has
+    // transparent closures
+    auto tagged_material = [d](uint32_t material) {
+        const psy_material_desc &m = d->materials[material];
+        for (uint32_t k = 0; k < m.closure_count; ++k)
+            if (m.closures[k].op == PSY_CLOSURE_TRANSPARENT) return material | psy::kMaterialTransparent;
+        return material;
+    };
+    {
+        std::vector<uint32_t> tagged(d->material_count);
+        for (uint32_t i = 0; i < d->material_count; ++i) tagged[i] = tagged_material(i);
+        for (uint32_t &m : tri_materials) m = tagged[m];
+    }
     std::vector<psy::EntryGpu> entries(d->instance_count);
     for (uint32_t i = 0; i < d->instance_count; ++i) {
         const psy::MeshGpu &mesh = meshes[instances[i].mesh];
         psy::EntryGpu &e = entries[i];
         std::copy(std::begin(instances[i].w2o), std::end(instances[i].w2o), e.w2o);
-        e.root = mesh.node_offset;
-        e.prim_offset = mesh.prim_offset;
+        e.root = node_offsets[instances[i].mesh];
+        e.prim_offset = instances[i].prim_offset = mesh.tri_offset;
         e.visibility = instances[i].visibility;
-        e.pad = 0u;
+        e.material = instances[i].material =
+            mesh.material_offset != psy::kInvalidId ? psy::kInvalidId : tagged_material(d->instances[i].material);
+        instances[i].smooth = mesh.smooth;
     }
 
     // ---- materials and parameter blocks
@@ -1832,7 +1840,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
             e.area = 0.5f * std::sqrt(dt(cr, cr));
             e.material = mi;
             e.object = i;
-            e.cycles_prim = meshes[id.mesh].prim_offset + k;
+            e.cycles_prim = meshes[id.mesh].tri_offset + k;
             e.emission_sampling = mat.emission_sampling;
             out_e.push_back(e);
         }
@@ -1908,20 +1916,29 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // device pool: a later compile reuses the memory a destroyed scene gave
     // back, and parameter blocks replaced by edits are retired without
     // waiting on the device.
-    for (DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions, &sc->normals,
-                            &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->baked, &sc->closures, &sc->code, &sc->value_buf, &sc->scalar_buf,
+    for (DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->shade_tris, &sc->instances, &sc->material_buf, &sc->baked, &sc->closures, &sc->code, &sc->value_buf, &sc->scalar_buf,
                             &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights, &sc->lamp_consts,
                             &sc->lamp_bounds, &sc->lamp_ids})
         b->ordered = st;
     PSY_CUDA_TRY(sc->nodes.upload(nodes, st));
     PSY_CUDA_TRY(sc->entries.upload(entries, st));
-    PSY_CUDA_TRY(sc->tris.upload(tris, st));
     PSY_CUDA_TRY(sc->instances.upload(instances, st));
-    PSY_CUDA_TRY(sc->meshes.upload(meshes, st));
-    PSY_CUDA_TRY(sc->positions.upload(positions, st));
-    PSY_CUDA_TRY(sc->normals.upload(normals, st));
-    PSY_CUDA_TRY(sc->indices.upload(indices, st));
-    PSY_CUDA_TRY(sc->tri_materials.upload(tri_materials, st));
+    // the triangle records are packed on the device; the vertex arrays go
+    // back to the pool when the compile ends
+    DeviceBuffer mesh_records(st), positions_buf(st), normals_buf(st), indices_buf(st), tri_materials_buf(st), order_buf(st);
+    PSY_CUDA_TRY(mesh_records.upload(meshes, st));
+    PSY_CUDA_TRY(positions_buf.upload(positions, st));
+    PSY_CUDA_TRY(normals_buf.upload(normals, st));
+    PSY_CUDA_TRY(indices_buf.upload(indices, st));
+    PSY_CUDA_TRY(tri_materials_buf.upload(tri_materials, st));
+    PSY_CUDA_TRY(order_buf.upload(order, st));
+    PSY_CUDA_TRY(sc->tris.alloc(sizeof(psy::TriGpu) * std::max<size_t>(order.size(), 1u)));
+    PSY_CUDA_TRY(sc->shade_tris.alloc(sizeof(psy::ShadeTriGpu) * std::max<size_t>(order.size(), 1u)));
+    psy::launch_pack_triangles(st, mesh_records.as<psy::MeshGpu>(), d->mesh_count, positions_buf.as<float>(),
+                               normals_buf.as<float>(), indices_buf.as<uint32_t>(), tri_materials_buf.as<uint32_t>(),
+                               order_buf.as<uint32_t>(), uint32_t(order.size()), sc->tris.as<psy::TriGpu>(),
+                               sc->shade_tris.as<psy::ShadeTriGpu>());
+    PSY_CUDA_TRY(cudaGetLastError());
     PSY_CUDA_TRY(sc->material_buf.upload(sc->materials, st));
     PSY_CUDA_TRY(sc->baked.alloc(sizeof(psy::BakedMaterialGpu) * std::max<size_t>(sc->materials.size(), 1u)));
     PSY_CUDA_TRY(sc->closures.alloc(sizeof(psy::BakedClosureGpu) * std::max(baked_closures, 1u)));
@@ -1964,8 +1981,8 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     PSY_CUDA_TRY(sc->lamp_ids.upload(lamp_ids, st));
     PSY_CUDA_TRY(cudaStreamSynchronize(st));
     sc->stats.upload_bytes = 0u;
-    for (const DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->instances, &sc->meshes, &sc->positions,
-                                  &sc->normals, &sc->indices, &sc->tri_materials, &sc->material_buf, &sc->baked, &sc->closures, &sc->code,
+    for (const DeviceBuffer *b : {&sc->nodes, &sc->entries, &mesh_records, &positions_buf, &normals_buf, &indices_buf,
+                                  &tri_materials_buf, &order_buf, &sc->instances, &sc->material_buf, &sc->baked, &sc->closures, &sc->code,
                                   &sc->value_buf, &sc->scalar_buf, &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights,
                                   &sc->lamp_consts, &sc->lamp_bounds, &sc->lamp_ids})
         sc->stats.upload_bytes += b->bytes;
@@ -1974,11 +1991,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     v.entries = sc->entries.as<psy::EntryGpu>();
     v.tris = sc->tris.as<psy::TriGpu>();
     v.instances = sc->instances.as<psy::InstanceGpu>();
-    v.meshes = sc->meshes.as<psy::MeshGpu>();
-    v.positions = sc->positions.as<float>();
-    v.normals = sc->normals.as<float>();
-    v.indices = sc->indices.as<uint32_t>();
-    v.tri_materials = sc->tri_materials.as<uint32_t>();
+    v.shade_tris = sc->shade_tris.as<psy::ShadeTriGpu>();
     v.materials = sc->material_buf.as<psy::MaterialGpu>();
     v.baked = sc->baked.as<psy::BakedMaterialGpu>();
     v.closures = sc->closures.as<psy::BakedClosureGpu>();
@@ -2197,8 +2210,7 @@ psy_status psy_session_read_trace(psy_session *s, psy_path_trace *out) {
 
 uint64_t psy::host::scene_device_bytes(const psy_scene *s) {
     uint64_t n = 0u;
-    for (const DeviceBuffer *b : {&s->nodes, &s->entries, &s->tris, &s->instances, &s->meshes, &s->positions, &s->normals,
-                                  &s->indices, &s->tri_materials, &s->material_buf, &s->baked, &s->closures, &s->code, &s->value_buf, &s->scalar_buf,
+    for (const DeviceBuffer *b : {&s->nodes, &s->entries, &s->tris, &s->shade_tris, &s->instances, &s->material_buf, &s->baked, &s->closures, &s->code, &s->value_buf, &s->scalar_buf,
                                   &s->vector_buf, &s->emitters, &s->distribution, &s->ggx_tables, &s->lights, &s->lamp_consts, &s->lamp_bounds,
                                   &s->lamp_ids, &s->lt_nodes, &s->lt_emitters, &s->lt_mapping, &s->lt_lookup})
         n += b->bytes;

@@ -154,7 +154,7 @@ struct psy_scene {
     psy_camera_desc camera{};
     std::vector<psy::MaterialGpu> materials;
     std::vector<float> scalars, vectors;
-    psy::host::DeviceBuffer nodes, entries, tris, instances, meshes, positions, normals, indices, tri_materials, material_buf, baked, closures, code,
+    psy::host::DeviceBuffer nodes, entries, tris, shade_tris, instances, material_buf, baked, closures, code,
         value_buf, scalar_buf, vector_buf, emitters, distribution, ggx_tables, lights, lamp_consts, lamp_bounds, lamp_ids, lt_nodes, lt_emitters,
         lt_mapping, lt_lookup;
     psy::SceneView view{};

@@ -402,7 +402,7 @@ __device__ __forceinline__ float next_float_up(float t) {
 }
 
 // ------------------------------------------------------ sort by material
-__device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_t instance, uint32_t local);
+__device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_t instance, uint32_t cycles_prim);
 
 // The kind of lamp a path's next-event sample will take under the flat
 // light distribution, estimated from the same random number the shading
@@ -457,7 +457,9 @@ __global__ void k_sort_count(const __grid_constant__ SceneView s_arg, const __gr
             const uint32_t job = kMulti ? b.job[i] : 0u;
             const SceneView &s = kMulti ? jobs[job].s : s_arg;
             const RenderParams &p = kMulti ? jobs[job].p : p_arg;
-            const uint32_t mat = surface_material(s, __float_as_uint(h4.w), prim);
+            const uint32_t instance = __float_as_uint(h4.w);
+            const uint32_t mat =
+                surface_material(s, instance, s.entries[instance].prim_offset + prim) & ~kMaterialTransparent;
             key = 1u + (mat * 8u + nee_kind_hint(s, p, b, i) + job * 977u) % (kSortBuckets - 1u);
         }
         b.sort_keys[q] = key;
@@ -744,12 +746,11 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                 h.instance = __float_as_uint(h4.w);
                 h.prim = prim;
                 h.object = h.instance;
-                h.cycles_prim = s.meshes[s.instances[h.instance].mesh].prim_offset + prim;
+                const SurfacePoint sp = surface_point(s, h, ray.d);
                 if (ev) {
                     ev->hit_object = h.object;
-                    ev->hit_primitive = h.cycles_prim;
+                    ev->hit_primitive = sp.cycles_prim;
                 }
-                const SurfacePoint sp = surface_point(s, h, ray.d);
                 const BakedMaterialGpu mat = s.baked[sp.material];
                 SurfaceClosures<kGlossy> closures;
                 const ClosurePoint cpt{sp.n, sp.ng, -ray.d, safe_normalize(-ray.d, sp.n), mat.bump_correction != 0u,
@@ -824,7 +825,6 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                         }
                     }
                     const uint32_t lobe_mask = terminate_after_transparent ? kEventTransparent : 0xffffffffu;
-                    const InstanceGpu &inst = s.instances[sp.instance];
                     // Direct lighting (src/luisa/path_kernel_pipeline.cpp:160-172)
                     if (p.nee && (runtime & kRuntimeBsdfHasEval) != 0u) {
                         f3 lp = mk3(0.0f), ldir = mk3(0.0f);
@@ -842,10 +842,10 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                         float light_pdf = 0.0f, pdf_divisor = 1.0f;
                         if (selected.kind == 0u) {
                             // EmissiveMeshLightingComponent (src/luisa/path_kernel_nee_emissive_mesh.cpp:32-296)
-                            const EmitterGpu &em = s.emitters[selected.index];
-                            const TriSample ls = sample_triangle(sp.position, ld3(em.p0), ld3(em.p1), ld3(em.p2),
+                            const Emitter em = load_emitter(s.emitters + selected.index);
+                            const TriSample ls = sample_triangle(sp.position, em.p0, em.p1, em.p2,
                                                                  mk2(light_sample.x, light_sample.y));
-                            const bool side = sampled_side(em.emission_sampling, ld3(em.ng), ls.direction);
+                            const bool side = sampled_side(em.emission_sampling, em.ng, ls.direction);
                             const float pdf = ls.pdf * selected.selection_pdf;
                             if (ls.valid && side && em.area > 0.0f && pdf > 0.0f) {
                                 const bool is_transmission = dot(ls.direction, sp.n) < 0.0f;
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                         }
                         if (emit) {
                             // make_shadow_origin (src/luisa/path_kernel_surface_geometry.cpp:168-185)
-                            const Xform w2o = xform12(inst.w2o);
+                            const Xform w2o = world_to_object(s, sp.instance);
                             const f3 so = origin_with_self_exclusion(sp, xform_point(w2o, sp.position),
                                                                      xform_direction(w2o, ldir));
                             const f3 off = lp - so;
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
                                 ray.tmin = next_float_up(h.t);
                             } else {
                                 const f3 wi = normalize(ss.wi);
-                                const Xform w2o = xform12(inst.w2o);
+                                const Xform w2o = world_to_object(s, sp.instance);
                                 ray.o = origin_with_self_exclusion(sp, sp.object_position, xform_direction(w2o, wi));
                                 ray.d = wi;
                                 ray.tmin = 0.0f;
@@ -1000,6 +1000,49 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
     }
 }
 
+// Triangle records of all meshes from their vertex arrays: thread i takes
+// leaf slot i, which holds triangle order[i] of its mesh.
+__global__ void k_pack_triangles(const MeshGpu *meshes, uint32_t mesh_count, const float *positions,
+                                 const float *normals, const uint32_t *indices, const uint32_t *tri_materials,
+                                 const uint32_t *order, uint32_t triangles, TriGpu *tris, ShadeTriGpu *shade_tris) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= triangles) return;
+    // the last mesh that begins at or before the slot (meshes without
+    // triangles share their successor's first slot)
+    uint32_t lo = 0u, hi = mesh_count;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (meshes[mid].tri_offset <= i) lo = mid;
+        else hi = mid;
+    }
+    const MeshGpu m = meshes[lo];
+    const uint32_t local = order[i];
+    const uint32_t *idx = indices + m.index_offset + 3u * local;
+    const float *P = positions + 3u * m.vertex_offset, *N = normals + 3u * m.vertex_offset;
+    f3 p[3], n[3];
+    for (int k = 0; k < 3; ++k) {
+        p[k] = ld3(P + 3u * idx[k]);
+        n[k] = m.smooth ? ld3(N + 3u * idx[k]) : mk3(0.0f);
+    }
+    TriGpu t;
+    t.v0 = make_float4(p[0].x, p[0].y, p[0].z, __uint_as_float(local));
+    t.v1 = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
+    t.v2 = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
+    t.pad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    tris[i] = t;
+    const f3 ng = safe_normalize(cross(p[1] - p[0], p[2] - p[0]), mk3(0.0f, 0.0f, 1.0f));
+    ShadeTriGpu o;
+    for (int k = 0; k < 3; ++k) {
+        float *op = k == 0 ? o.p0 : k == 1 ? o.p1 : o.p2, *on = k == 0 ? o.n0 : k == 1 ? o.n1 : o.n2;
+        op[0] = p[k].x, op[1] = p[k].y, op[2] = p[k].z;
+        on[0] = n[k].x, on[1] = n[k].y, on[2] = n[k].z;
+    }
+    o.ng[0] = ng.x, o.ng[1] = ng.y, o.ng[2] = ng.z;
+    o.material = m.material_offset == kInvalid ? kInvalid : tri_materials[m.material_offset + local];
+    o.pad[0] = o.pad[1] = 0u;
+    shade_tris[m.tri_offset + local] = o;
+}
+
 // Evaluates the closure programs of materials [first, first + count), one
 // material a thread (microseconds, when a scene is compiled or a material
 // edited).  While shading and shadow rays walked the programs per path, the
@@ -1031,10 +1074,11 @@ __global__ void k_bake_materials(const __grid_constant__ SceneView s, BakedMater
 
 constexpr int kShadowList = 8;
 
-__device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_t instance, uint32_t local) {
-    const InstanceGpu &inst = s.instances[instance];
-    const MeshGpu mesh = s.meshes[inst.mesh];
-    return mesh.material_offset == kInvalid ? inst.material : s.tri_materials[mesh.material_offset + local];
+// The material of a surface, with kMaterialTransparent where it has
+// transparent closures.
+__device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_t instance, uint32_t cycles_prim) {
+    const uint32_t m = __ldg(&s.entries[instance].material);
+    return m != kInvalid ? m : __ldg(&s.shade_tris[cycles_prim].material);
 }
 
 // Persistent any-hit shadow kernel (same refill scheme as k_intersect).
@@ -1081,16 +1125,17 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
         const int busy = __popc(__ballot_sync(kFullMask, active));
         if (busy == 0) break;
         traverse_warp<false>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
-                             [&](uint32_t ii, uint32_t local, uint32_t cp, float th, float, float) {
+                             [&](uint32_t ii, uint32_t, uint32_t cp, float th, float, float) {
             if (!s.any_transparent) {
                 blocked = true;
                 return true;
             }
-            const uint32_t mi = surface_material(s, ii, local);
-            if (!s.materials[mi].has_transparent) {
+            uint32_t mi = surface_material(s, ii, cp);
+            if ((mi & kMaterialTransparent) == 0u) {
                 blocked = true;
                 return true;
             }
+            mi &= ~kMaterialTransparent;
             for (int k = 0; k < n; ++k) {
                 if (lt[k] == th) {
                     if (ii > lo[k] || (ii == lo[k] && cp > lp[k])) {
@@ -1507,6 +1552,13 @@ void launch_bake_materials(cudaStream_t st, const SceneView &s, BakedMaterialGpu
                            uint32_t first, uint32_t count) {
     if (count == 0u) return;
     k_bake_materials<<<(count + 31u) / 32u, 32, 0, st>>>(s, baked, closures, first, count);
+}
+void launch_pack_triangles(cudaStream_t st, const MeshGpu *meshes, uint32_t mesh_count, const float *positions,
+                           const float *normals, const uint32_t *indices, const uint32_t *tri_materials,
+                           const uint32_t *order, uint32_t triangles, TriGpu *tris, ShadeTriGpu *shade_tris) {
+    if (triangles == 0u) return;
+    k_pack_triangles<<<(triangles + 127u) / 128u, 128, 0, st>>>(meshes, mesh_count, positions, normals, indices,
+                                                                tri_materials, order, triangles, tris, shade_tris);
 }
 void launch_debug_sobol(cudaStream_t st, const float4 *table, uint32_t size, const uint32_t *queries, uint32_t count,
                         float4 *out, uint32_t *out_index) {

@@ -44,6 +44,10 @@ void launch_resolve_pass(cudaStream_t st, const float4 *film, const uint32_t *co
 // from its parameter blocks into the baked tables.
 void launch_bake_materials(cudaStream_t st, const SceneView &s, BakedMaterialGpu *baked, BakedClosureGpu *closures,
                            uint32_t first, uint32_t count);
+// Leaf and shading triangle records from the meshes' vertex arrays.
+void launch_pack_triangles(cudaStream_t st, const MeshGpu *meshes, uint32_t mesh_count, const float *positions,
+                           const float *normals, const uint32_t *indices, const uint32_t *tri_materials,
+                           const uint32_t *order, uint32_t triangles, TriGpu *tris, ShadeTriGpu *shade_tris);
 void launch_film(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t pixels, uint32_t samples, float4 *combined,
                  float4 *normal, float4 *albedo, uint32_t *sample_count, uint32_t trace_path, psy_path_trace *trace);
 // Batched wavefront.  round (device memory): paths, film pixels, items.

@@ -7,8 +7,8 @@
 //   tris          leaf triangles of all meshes in node order, 64 B each:
 //                 object-space vertices, v0.w = local primitive index bits
 //   entries       per instance, the ray's transform and the mesh's root (64 B)
-//   positions / normals / indices  the meshes' shading data
-//   instances     InstanceGpu (object<->world transforms, mesh, material)
+//   shade_tris    the meshes' triangles as shading reads them, 96 B each
+//   instances     InstanceGpu (object<->world transforms, material)
 //   materials / code / scalars / vectors  closure programs and their
 //                 parameter blocks (rebinding rewrites scalars/vectors)
 //   baked / closures  the programs evaluated, as the kernels shade with them
@@ -71,26 +71,45 @@ struct alignas(32) EntryGpu {
     float w2o[12];
     uint32_t root;         // root node of the mesh
     uint32_t prim_offset;  // Cycles primitive id of local primitive 0
-    uint32_t visibility, pad;
+    uint32_t visibility;
+    uint32_t material;  // as InstanceGpu::material
 };
 static_assert(sizeof(EntryGpu) == 64, "an instance entry is two 32-byte sectors");
 
-struct alignas(16) InstanceGpu {
+// An instance as shading reads it: three sectors for the hit point, two for
+// the object-space ray of a new origin.
+struct alignas(32) InstanceGpu {
     float o2w[12];  // column-major c0, c1, c2, c3 (xyz each)
-    float w2o[12];
-    float nrm[12];  // normal-to-world columns (c3 unused)
-    uint32_t mesh, material, visibility, pad;
-};
-
-struct alignas(16) MeshGpu {
-    uint32_t node_offset;    // root of the mesh's tree in `nodes`
-    uint32_t tri_offset;     // first leaf triangle in `tris`
-    uint32_t triangle_count;
-    uint32_t prim_offset;    // Cycles primitive id of local primitive 0
-    uint32_t vertex_offset;  // into positions / normals (vertices)
-    uint32_t index_offset;   // into indices (uint32 elements)
-    uint32_t material_offset;  // into tri_materials, kInvalid = instance material
+    float nrm[9];   // normal-to-world columns
+    uint32_t prim_offset;  // Cycles primitive id of local primitive 0
     uint32_t smooth;
+    uint32_t material;  // of the whole instance, with kMaterialTransparent; kInvalidId: per triangle
+    float w2o[12];
+    uint32_t mesh, visibility, pad[2];
+};
+static_assert(sizeof(InstanceGpu) == 160, "an instance is five 32-byte sectors");
+// Set beside a material index whose program has transparent closures.
+constexpr uint32_t kMaterialTransparent = 1u << 31;
+
+// A triangle as shading reads it, in Cycles primitive order: three sectors
+// instead of a gather through the index, position and normal arrays.
+struct alignas(32) ShadeTriGpu {
+    float p0[3], p1[3], p2[3];  // object space
+    float n0[3], n1[3], n2[3];  // vertex normals (smooth meshes)
+    float ng[3];                // normalised geometric normal
+    uint32_t material;          // with kMaterialTransparent; kInvalidId: the instance's
+    uint32_t pad[2];
+};
+static_assert(sizeof(ShadeTriGpu) == 96, "a shading triangle is three 32-byte sectors");
+
+// A mesh while its triangle records are packed (k_pack_triangles).
+struct alignas(16) MeshGpu {
+    uint32_t tri_offset;  // first leaf triangle in `tris`, also the Cycles primitive id of local primitive 0
+    uint32_t triangle_count;
+    uint32_t vertex_offset;    // into positions / normals (vertices)
+    uint32_t index_offset;     // into indices (uint32 elements)
+    uint32_t material_offset;  // into the triangle materials, kInvalid = instance material
+    uint32_t smooth, pad0, pad1;
 };
 
 struct alignas(16) MaterialGpu {
@@ -153,11 +172,7 @@ struct SceneView {
     const TriGpu *tris;
     const EntryGpu *entries;  // one per instance
     const InstanceGpu *instances;
-    const MeshGpu *meshes;
-    const float *positions;
-    const float *normals;
-    const uint32_t *indices;
-    const uint32_t *tri_materials;
+    const ShadeTriGpu *shade_tris;
     const MaterialGpu *materials;
     const BakedMaterialGpu *baked;    // one per material
     const BakedClosureGpu *closures;
