@@ -84,6 +84,9 @@ struct DeviceBuffer {
         if (n == 0) return cudaSuccess;
         return ordered ? cudaMallocAsync(&ptr, n, ordered) : cudaMalloc(&ptr, n);
     }
+    // As alloc, but memory of that size already held is kept: for buffers
+    // whose earlier content no queued work of another stream still reads.
+    cudaError_t ensure(size_t n) { return ptr && bytes == n ? cudaSuccess : alloc(n); }
     template <typename T>
     cudaError_t upload(const std::vector<T> &v, cudaStream_t st) {
         cudaError_t e = alloc(std::max<size_t>(v.size() * sizeof(T), 16));
