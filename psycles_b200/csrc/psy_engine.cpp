@@ -105,19 +105,19 @@ uint32_t WavefrontEngine::issue(uint32_t steps, bool allow_exit, psy_status &sta
     const uint32_t *rd = round_.as<uint32_t>();
     const uint32_t cap = arena_.capacity;
     PathBuffers b = arena_.view;
+    unsigned long long *stats = arena_.stats.as<unsigned long long>();
     status = PSY_OK;
-    launch_begin_round(st, b.counters, round_.as<uint32_t>(), items_.as<BatchItem>(), plan_rounds_.as<uint32_t>(),
+    launch_begin_round(st, lc, b.counters, round_.as<uint32_t>(), items_.as<BatchItem>(), plan_rounds_.as<uint32_t>(),
                        plan_items_.as<BatchItem>(), cursor_.as<uint32_t>(), max_jobs_);
     launch_raygen_batch(st, lc, jt, it, rd, b, cap);
     uint32_t launches = 2u;
     for (uint32_t step = 0; step < steps; ++step) {
         launch_intersect_batch(st, lc, jt, b, cap);
         launch_shade_batch(st, lc, jt, b, cap, step);
-        launch_count_rays(st, b.counters, arena_.stats.as<unsigned long long>());
         launch_shadow_batch(st, lc, jt, b, cap, step);
-        launch_swap(st, b.counters);
+        launch_end_step(st, lc, b.counters, stats, step);
         std::swap(b.queue_in, b.queue_out);
-        launches += 5u;
+        launches += 4u;
         if (allow_exit && (step + 1u) % check_interval_ == 0u) {
             uint32_t left = 0u;
             if (cudaMemcpyAsync(&left, b.counters, sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -125,11 +125,12 @@ uint32_t WavefrontEngine::issue(uint32_t steps, bool allow_exit, psy_status &sta
                 status = fail(PSY_ERROR_CUDA, "wavefront: reading the live path count failed");
                 return launches;
             }
-            if (left == 0u) break;
+            if (left < std::max(lc.tail_paths, 1u)) break;
         }
     }
+    launch_tail_batch(st, lc, jt, arena_.view, cap, stats);
     launch_film_batch(st, lc, jt, it, rd, b, cap);
-    return launches + 1u;
+    return launches + 2u;
 }
 
 psy_status WavefrontEngine::ensure_graph(uint32_t steps) {
@@ -191,7 +192,7 @@ psy_status WavefrontEngine::run(const EnginePlan &plan, uint32_t steps, EngineRu
         if (use_graph_) {
             PSY_CUDA_TRY(cudaGraphLaunch(graph_, st));
             out.graph_launches += 1u;
-            out.kernel_launches += 3u + 5u * steps;
+            out.kernel_launches += 4u + 4u * steps;
         } else {
             psy_status s = PSY_OK;
             out.kernel_launches += issue(steps, true, s);

@@ -217,6 +217,9 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 #ifndef PSY_SHADE_MIN_BLOCKS
 #define PSY_SHADE_MIN_BLOCKS 4
 #endif
+#ifndef PSY_TAIL_MIN_BLOCKS
+#define PSY_TAIL_MIN_BLOCKS 3
+#endif
 #ifndef PSY_MISS_MIN_BLOCKS
 #define PSY_MISS_MIN_BLOCKS 8
 #endif
@@ -245,18 +248,52 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *fetch_counter, uint32_t
     return q < count ? q : kInvalid;
 }
 
+// A path's closest hit so far.
+struct ClosestHit {
+    float t, u, v;
+    uint32_t instance, prim;  // kInvalid: none yet
+};
+
+__device__ __forceinline__ void closest_begin(ClosestHit &best, TraversalState &t, const SceneView &s,
+                                              const PathBuffers &b, uint32_t path) {
+    float4 o, d;
+    uint4 st, st2;
+    load_pair(b.ray_o, path, o, d);
+    load_pair(b.st, path, st, st2);
+    const Ray ray{mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w};
+    traversal_begin(t, s, ray, contract_visibility(st.y), st2.y, st2.z, kInvalid, kInvalid);
+    best.t = ray.tmax;
+    best.u = best.v = 0.0f;
+    best.instance = best.prim = kInvalid;
+}
+
+__device__ __forceinline__ bool closest_hit(ClosestHit &best, TraversalState &t, uint32_t instance, uint32_t prim,
+                                            float th, float u, float v) {
+    // equal distances go to the greatest (object, primitive)
+    const bool later = instance > best.instance || (instance == best.instance && prim > best.prim);
+    if (best.instance != kInvalid && !(th < best.t || (th == best.t && later))) return false;
+    best = {th, u, v, instance, prim};
+    t.tmax = th;
+    return false;
+}
+
+__device__ __forceinline__ void closest_store(const ClosestHit &best, const PathBuffers &b, uint32_t path) {
+    store_pair(b.hit, path, make_float4(best.t, best.u, best.v, __uint_as_float(best.instance)),
+               make_uint4(best.prim, 0u, 0u, 0u));
+}
+
 // kMulti: paths of a batched wavefront, each traced in its job's scene.
 template <bool kMulti>
 __global__ void __launch_bounds__(128, PSY_INTERSECT_MIN_BLOCKS)
     k_intersect(const __grid_constant__ SceneView s_arg, const __grid_constant__ PathBuffers b, const JobGpu *jobs,
                 uint32_t sort_threshold) {
     const uint32_t count = b.counters[0];
+    if (b.counters[kCounterTail] != 0u) return;
     const bool sorted = sort_threshold != 0u && count >= sort_threshold;
     TraversalState t;
     t.node = kLinkDone;
     t.leaves = 0u;
-    float best_t = 0.0f, best_u = 0.0f, best_v = 0.0f;
-    uint32_t best_instance = kInvalid, best_prim = kInvalid;
+    ClosestHit best;
     bool active = false, exhausted = false;
     uint32_t path = 0u, job = 0u;
     for (;;) {
@@ -267,36 +304,17 @@ __global__ void __launch_bounds__(128, PSY_INTERSECT_MIN_BLOCKS)
         }
         const SceneView &s = kMulti ? jobs[job].s : s_arg;
         if (q != kInvalid) {
-            float4 o, d;
-            uint4 st, st2;
-            load_pair(b.ray_o, path, o, d);
-            load_pair(b.st, path, st, st2);
-            const uint32_t vis = st.y;
-            const Ray ray{mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w};
-            traversal_begin(t, s, ray, contract_visibility(vis), st2.y, st2.z, kInvalid, kInvalid);
-            best_t = ray.tmax;
-            best_u = best_v = 0.0f;
-            best_instance = best_prim = kInvalid;
+            closest_begin(best, t, s, b, path);
             active = true;
         }
         const int busy = __popc(__ballot_sync(kFullMask, active));
         if (busy == 0) break;
         traverse_warp<true>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
                             [&](uint32_t ii, uint32_t local, uint32_t, float th, float u, float v) {
-            // equal distances go to the greatest (object, primitive)
-            const bool later = ii > best_instance || (ii == best_instance && local > best_prim);
-            if (best_instance != kInvalid && !(th < best_t || (th == best_t && later))) return false;
-            best_t = th;
-            best_u = u;
-            best_v = v;
-            best_instance = ii;
-            best_prim = local;
-            t.tmax = th;
-            return false;
+            return closest_hit(best, t, ii, local, th, u, v);
         });
         if (active && t.node == kLinkDone && t.leaves == 0u) {
-            store_pair(b.hit, path, make_float4(best_t, best_u, best_v, __uint_as_float(best_instance)),
-                       make_uint4(best_prim, 0u, 0u, 0u));
+            closest_store(best, b, path);
             active = false;
         }
     }
@@ -446,7 +464,7 @@ __global__ void k_sort_count(const __grid_constant__ SceneView s_arg, const __gr
                              const __grid_constant__ PathBuffers b, const JobGpu *jobs, uint32_t threshold) {
     __shared__ uint32_t local[kSortBuckets];
     const uint32_t count = b.counters[0];
-    if (count < threshold) return;
+    if (count < threshold || b.counters[kCounterTail] != 0u) return;
     for (uint32_t k = threadIdx.x; k < kSortBuckets; k += blockDim.x) local[k] = 0u;
     __syncthreads();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
@@ -479,7 +497,7 @@ __global__ void k_sort_count(const __grid_constant__ SceneView s_arg, const __gr
 // queue is the shading queue, whose bucket 0 holds the misses.
 __global__ void k_sort_scan(const __grid_constant__ PathBuffers b, uint32_t threshold, uint32_t counter, bool misses) {
     __shared__ uint32_t part[1024];
-    if (b.counters[counter] < threshold) return;
+    if (b.counters[counter] < threshold || b.counters[kCounterTail] != 0u) return;
     constexpr uint32_t kPer = kSortBuckets / 1024u;
     const uint32_t t = threadIdx.x;
     uint32_t v[kPer], sum = 0u;
@@ -515,7 +533,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(const __grid_constant__ Pa
                                                       uint32_t counter) {
     __shared__ uint32_t hist[kSortBuckets];
     const uint32_t count = b.counters[counter];
-    if (count < threshold) return;
+    if (count < threshold || b.counters[kCounterTail] != 0u) return;
     const uint32_t chunk = (count + gridDim.x - 1u) / gridDim.x;
     const uint32_t begin = blockIdx.x * chunk;
     const uint32_t end = min(count, begin + chunk);
@@ -553,7 +571,7 @@ __global__ void k_sort_count_rays(const __grid_constant__ SceneView s_arg, const
                                   const JobGpu *jobs, uint32_t threshold) {
     __shared__ uint32_t local[kSortBuckets];
     const uint32_t count = b.counters[0];
-    if (count < threshold) return;
+    if (count < threshold || b.counters[kCounterTail] != 0u) return;
     for (uint32_t k = threadIdx.x; k < kSortBuckets; k += blockDim.x) local[k] = 0u;
     __syncthreads();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
@@ -585,7 +603,7 @@ __global__ void k_sort_count_rays(const __grid_constant__ SceneView s_arg, const
 __global__ void k_sort_count_shadow(const __grid_constant__ PathBuffers b, uint32_t threshold) {
     __shared__ uint32_t local[kSortBuckets];
     const uint32_t count = b.counters[2];
-    if (count < threshold) return;
+    if (count < threshold || b.counters[kCounterTail] != 0u) return;
     for (uint32_t k = threadIdx.x; k < kSortBuckets; k += blockDim.x) local[k] = 0u;
     __syncthreads();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
@@ -672,7 +690,7 @@ template <bool kMulti>
 __global__ void __launch_bounds__(128, PSY_MISS_MIN_BLOCKS)
     k_shade_miss(const __grid_constant__ SceneView s_arg, const __grid_constant__ RenderParams p_arg,
                  const __grid_constant__ PathBuffers b, const JobGpu *jobs, uint32_t sort_threshold) {
-    if (b.counters[0] < sort_threshold) return;
+    if (b.counters[0] < sort_threshold || b.counters[kCounterTail] != 0u) return;
     const uint32_t count = b.counters[kCounterMisses];
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
         const uint32_t i = b.queue_sorted[q];
@@ -699,8 +717,342 @@ __global__ void __launch_bounds__(128, PSY_MISS_MIN_BLOCKS)
     }
 }
 
+// What shading a path leaves for its queues.
+struct ShadeResult {
+    bool keep;    // the path goes on
+    bool shadow;  // and / or sends the shadow ray below
+    bool final;   // it ends here: its radiance and shadow contribution go to rad_final
+    float4 sh_o, sh_d, sh_c;
+    uint4 sh_ids;
+};
+
+// One path step after its closest hit: background / emission + forward MIS,
+// roulette, AOV, NEE sample, closure sample and path-state transition.  Reads
+// and writes path i's record.
 // kTrace selects the variant that records the per-path trace; the render
 // variant carries no trace code.
+template <bool kTrace, bool kGlossy>
+__device__ __forceinline__ ShadeResult shade_path(const SceneView &s, const RenderParams &p, const PathBuffers &b,
+                                                  uint32_t i, uint32_t step, uint32_t trace_path,
+                                                  psy_path_trace *trace) {
+    ShadeResult out;
+    out.keep = out.shadow = out.final = false;
+    psy_path_event *ev = nullptr;
+    if (kTrace && trace && i == trace_path && step < PSY_TRACE_MAX_EVENTS) {
+        ev = &trace->events[step];
+        trace->event_count = step + 1u;
+    }
+    float4 ro, rd, tp4, rad4, h4;
+    uint4 st, st2, hp4;
+    load_pair(b.ray_o, i, ro, rd);
+    load_pair(b.tp, i, tp4, rad4);
+    load_pair(b.st, i, st, st2);
+    load_pair(b.hit, i, h4, hp4);
+    Ray ray{mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), ro.w, rd.w};
+    f3 throughput = mk3(tp4.x, tp4.y, tp4.z);
+    float previous_bsdf_pdf = tp4.w;
+    f3 radiance = mk3(rad4.x, rad4.y, rad4.z);
+    float transparency = rad4.w;
+    PathState ps = unpack_state(st, st2);
+    bool previous_delta = (st2.x & kSt2Delta) != 0u;
+    bool primary_recorded = (st2.x & kSt2Primary) != 0u;
+    const bool terminate_on_next_surface = (st2.x & kSt2TermNext) != 0u;
+    const bool terminate_after_transparent = (st2.x & kSt2TermAfter) != 0u;
+    const uint32_t ray_visibility = contract_visibility(ps.visibility);
+    const uint32_t sample = b.sample[i];
+    const uint32_t local = st2.w;
+    const uint32_t x = p.win_x + local % p.win_w;
+    const uint32_t y = p.win_y + local / p.win_w;
+    const uint32_t rng_hash = pixel_hash(x, p.full_h - 1u - y, p.seed);
+    const float terminate_sample = sample_4d(p, sample, rng_hash, ps.rng_offset + 0u).x;
+    const float4 ls4 = sample_4d(p, sample, rng_hash, ps.rng_offset + 1u);
+    const f3 light_sample = mk3(ls4.x, ls4.y, ls4.z);
+    const float light_terminate = sample_4d(p, sample, rng_hash, ps.rng_offset + 2u).x;
+    const float4 bs4 = sample_4d(p, sample, rng_hash, ps.rng_offset + 3u);
+    // the flat distribution's pick; without a trace to record it, only
+    // paths that take a light sample search for theirs
+    DistEntryGpu selected{0.0f, 0.0f, 3u, 0u};
+    if (kTrace && !p.use_light_tree) selected = distribution_sample(s, light_sample.z);
+    const uint32_t prim = hp4.x;
+    if (ev) {
+        ev->rng_offset = ps.rng_offset;
+        ev->random_terminate = terminate_sample;
+        set3(ev->random_light, light_sample);
+        ev->random_light_terminate = light_terminate;
+        set3(ev->random_bsdf, mk3(bs4.x, bs4.y, bs4.z));
+        ev->light_kind = selected.kind;
+        ev->light_index = selected.index;
+        const bool missed = prim == kInvalid;
+        ev->hit_t = missed ? 0.0f : h4.x;
+        ev->hit_u = missed ? 0.0f : h4.y;
+        ev->hit_v = missed ? 0.0f : h4.z;
+        ev->closure_index = kInvalid;
+        ev->hit_object = kInvalid;
+        ev->hit_primitive = kInvalid;
+    }
+    const uint32_t depth = ps.bounce;
+    bool alive = true;
+    if (s.lamp_count > 0u)
+        alive = lamp_events(s, p, b, i, ray, prim == kInvalid ? ray.tmax : h4.x, ray_visibility, throughput,
+                            previous_bsdf_pdf, previous_delta, ps, radiance, ev);
+    if (!alive) {
+        // a lamp event used up the transparent budget
+    } else if (prim == kInvalid) {
+        background_event(s, p, ray_visibility, throughput, ps, radiance, transparency, ev);
+        if (ev) ev->terminated = 1u;
+        alive = false;
+    } else {
+        Hit h;
+        h.t = h4.x;
+        h.u = h4.y;
+        h.v = h4.z;
+        h.instance = __float_as_uint(h4.w);
+        h.prim = prim;
+        h.object = h.instance;
+        const SurfacePoint sp = surface_point(s, h, ray.d);
+        if (ev) {
+            ev->hit_object = h.object;
+            ev->hit_primitive = sp.cycles_prim;
+        }
+        const BakedMaterialGpu mat = s.baked[sp.material];
+        SurfaceClosures<kGlossy> closures;
+        const ClosurePoint cpt{sp.n, sp.ng, -ray.d, safe_normalize(-ray.d, sp.n), mat.bump_correction != 0u,
+                               sp.back_facing};
+        collect_surface<kGlossy>(s, mat, cpt, closures);
+        // SurfaceShadingStageImpl::emit (src/luisa/path_kernel_surface_shading.cpp:117-250)
+        float emission_weight = 1.0f;
+        if (p.nee && s.triangle_emitters > 0u && mat.emission_sampling != 0u && mat.has_emission) {
+            const bool competing = depth > 0u && !previous_delta;
+            float selection_pdf =
+                0.5f * length(cross(sp.wp1 - sp.wp0, sp.wp2 - sp.wp0)) * s.triangle_area_pdf;
+            if (p.use_light_tree) {
+                // light_tree.forward_pdf (src/luisa/path_tracer_light_tree.cpp:799-838)
+                const float4 mn = b.mis_n[i];
+                selection_pdf = lt_pdf(s, lt_triangle_emitter(s, sp.object, sp.cycles_prim), ray.o,
+                                       mk3(mn.x, mn.y, mn.z), (ps.flag & kFlagMisHadTransmission) != 0u);
+            }
+            const float light_pdf = emissive_forward_pdf(selection_pdf, mat.emission_sampling, ray.o,
+                                                         sp.position, sp.wp0, sp.wp1, sp.wp2,
+                                                         // the geometric normal before the back-face
+                                                         // flip (path_kernel_surface_shading.cpp:130-134)
+                                                         sp.back_facing ? -sp.ng : sp.ng);
+            const bool available = light_pdf > 0.0f;
+            emission_weight = forward_light_weight(p.direct_mode, previous_bsdf_pdf, light_pdf, competing, available);
+        }
+        const f3 ec = clamp_contribution(throughput * closures.emission * emission_weight, depth, p);
+        radiance = radiance + ec;
+        if (ev) add3(ev->emission, ec);
+        if (terminate_on_next_surface) {
+            alive = false;
+            if (ev) ev->terminated = 1u;
+        }
+        if (alive) {
+            // continuation_probability (cycles_path_state.h:413-447)
+            const bool tr_state = (ps.flag & kFlagTransparent) != 0u;
+            const bool before_min = tr_state ? ps.transparent_bounce <= p.transparent_min : ps.bounce <= p.minimum;
+            const float cp = before_min ? 1.0f : minf_(sqrtf(max_abs_component(throughput)), 1.0f);
+            if (ev) ev->continuation_probability = cp;
+            if (cp <= 0.0f) {
+                alive = false;
+            } else if (cp != 1.0f) {
+                if (terminate_sample >= cp) alive = false;
+                else throughput = throughput / cp;
+            }
+            if (!alive && ev) ev->terminated = 1u;
+        }
+        if (alive) {
+            if (depth == 0u) {
+                f3 aov_albedo, aov_normal, aov_transparency;
+                surface_aov<kGlossy>(closures, cpt, aov_albedo, aov_normal, aov_transparency);
+                const float4 a4 = b.aov_a[i];
+                const f3 acc = mk3(a4.x, a4.y, a4.z) + throughput * aov_albedo;
+                b.aov_a[i] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+                const f3 alpha = clamp3(mk3(1.0f) - aov_transparency, 0.0f, 1.0f);
+                const float average_alpha = (alpha.x + alpha.y + alpha.z) * (1.0f / 3.0f);
+                const bool writes_normal = !primary_recorded && (p.pass_alpha_threshold == 0.0f ||
+                                                                 average_alpha >= p.pass_alpha_threshold);
+                if (writes_normal) {
+                    b.aov_n[i] = make_float4(aov_normal.x, aov_normal.y, aov_normal.z, 0.0f);
+                    primary_recorded = true;
+                    ps.flag |= kFlagSinglePassDone;
+                }
+            }
+            const uint32_t runtime = mat.runtime | (sp.back_facing ? kRuntimeBackfacing : 0u);
+            if (p.use_light_tree) {
+                // light-tree pick after shading (src/luisa/path_kernel_pipeline.cpp:150-159)
+                selected = lt_sample(s, light_sample.z, sp.position, sp.n,
+                                     (runtime & kRuntimeBsdfHasTransmission) != 0u);
+                if (ev) {
+                    ev->light_kind = selected.kind;
+                    ev->light_index = selected.index;
+                }
+            }
+            const uint32_t lobe_mask = terminate_after_transparent ? kEventTransparent : 0xffffffffu;
+            // Direct lighting (src/luisa/path_kernel_pipeline.cpp:160-172)
+            if (p.nee && (runtime & kRuntimeBsdfHasEval) != 0u) {
+                if (!kTrace && !p.use_light_tree) selected = distribution_sample(s, light_sample.z);
+                f3 lp = mk3(0.0f), ldir = mk3(0.0f);
+                float ldist = 0.0f;
+                bool distant = false;
+                f3 surviving = mk3(0.0f);
+                uint32_t light_obj = kInvalid, light_prim = kInvalid;
+                bool emit = false;
+                // The light sample of either kind, then one BSDF
+                // evaluation, MIS weight and light roulette shared by
+                // both (a warp's lanes that picked triangles and lamps
+                // evaluate together).
+                bool sampled = false, weigh_mis = true;
+                f3 light_radiance = mk3(0.0f);
+                float light_pdf = 0.0f, pdf_divisor = 1.0f;
+                if (selected.kind == 0u) {
+                    // EmissiveMeshLightingComponent (src/luisa/path_kernel_nee_emissive_mesh.cpp:32-296)
+                    const Emitter em = load_emitter(s.emitters + selected.index);
+                    const TriSample ls = sample_triangle(sp.position, em.p0, em.p1, em.p2,
+                                                         mk2(light_sample.x, light_sample.y));
+                    const bool side = sampled_side(em.emission_sampling, em.ng, ls.direction);
+                    const float pdf = ls.pdf * selected.selection_pdf;
+                    if (ls.valid && side && em.area > 0.0f && pdf > 0.0f) {
+                        const bool is_transmission = dot(ls.direction, sp.n) < 0.0f;
+                        const bool same_primitive = em.cycles_prim == sp.cycles_prim && em.object == sp.object;
+                        const f3 oriented = is_transmission ? -sp.ng : sp.ng;
+                        const bool reject_self = same_primitive && dot(ls.direction, oriented) > 0.0f;
+                        if (!reject_self) {
+                            sampled = true;
+                            light_radiance = ld3(__ldg(&s.baked[em.material].emission));
+                            light_pdf = pdf;
+                            pdf_divisor = pdf;
+                            lp = ls.position;
+                            light_obj = em.object;
+                            light_prim = em.cycles_prim;
+                            ldir = ls.direction;
+                        }
+                    }
+                } else if (selected.kind == 1u) {
+                    // AnalyticLightingComponent (src/luisa/path_kernel_nee_analytic.cpp:98-428)
+                    const psy_light_desc &l = s.lights[selected.index];
+                    if (!(depth > l.max_bounces)) {
+                        const AnalyticSample a =
+                            sample_analytic(l, s.lamp_consts[selected.index], sp.position, sp.n,
+                                            (runtime & kRuntimeBsdfHasTransmission) != 0u,
+                                            mk2(light_sample.x, light_sample.y));
+                        const float pdf = a.pdf * selected.selection_pdf;
+                        if (a.valid && pdf > 0.0f) {
+                            sampled = true;
+                            light_radiance = ld3(l.color) * (l.power * a.eval_factor);
+                            light_pdf = pdf;
+                            pdf_divisor = maxf_(pdf, 1.0e-20f);
+                            // MIS only for lamps a BSDF ray can also hit
+                            // (path_kernel_nee_analytic.cpp:286-292)
+                            weigh_mis = (l.flags & kLightFlagForward) != 0u;
+                            lp = a.position;
+                            ldir = a.direction;
+                            distant = l.type == PSY_LIGHT_DISTANT;
+                        }
+                    }
+                }
+                if (sampled) {
+                    const Evaluation e = evaluate_mixture<kGlossy>(closures, cpt, ldir, lobe_mask, -1);
+                    const float mis = weigh_mis ? nee_light_weight(p.direct_mode, light_pdf, e.pdf) : 1.0f;
+                    const f3 weighted = e.f * light_radiance * (mis / pdf_divisor);
+                    if (any_nonzero(weighted)) {
+                        const f3 unshadowed = weighted * mk3(1.0f);
+                        surviving =
+                            unshadowed * light_roulette_weight(unshadowed, light_terminate, p.inv_rr_threshold);
+                        emit = any_nonzero(surviving);
+                    }
+                }
+                if (emit) {
+                    // make_shadow_origin (src/luisa/path_kernel_surface_geometry.cpp:168-185)
+                    const Xform w2o = world_to_object(s, sp.instance);
+                    const f3 so = origin_with_self_exclusion(sp, xform_point(w2o, sp.position),
+                                                             xform_direction(w2o, ldir));
+                    const f3 off = lp - so;
+                    const float fd = sqrtf(maxf_(dot(off, off), 1.0e-20f));
+                    const f3 sdir = distant ? ldir : off / fd;
+                    ldist = distant ? 1.0e30f : fd;
+                    const f3 c = throughput * surviving;
+                    out.sh_o = make_float4(so.x, so.y, so.z, ldist);
+                    out.sh_d = make_float4(sdir.x, sdir.y, sdir.z, __uint_as_float(ps.transparent_bounce));
+                    out.sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(depth));
+                    out.sh_ids = make_uint4(sp.object, sp.cycles_prim, light_obj, light_prim);
+                    out.shadow = true;
+                }
+            }
+            // SurfaceScatterStageImpl::emit (src/luisa/path_kernel_surface_scatter.cpp:136-291)
+            const SurfaceSample ss = sample_surface<kGlossy>(closures, cpt, bs4.z, mk2(bs4.x, bs4.y), lobe_mask);
+            if (ev) {
+                ev->closure_index = ss.closure_index;
+                ev->bsdf_pdf = ss.eval.pdf;
+                set3(ev->wi, ss.wi);
+            }
+            if (!ss.valid || ss.eval.pdf <= 0.0f) {
+                alive = false;
+            } else {
+                const bool transparent = (ss.eval.events & kEventTransparent) != 0u;
+                const bool singular = (ss.eval.events & kEventSingular) != 0u;
+                const uint32_t label = label_from_events(ss.eval.events);
+                throughput = throughput * (ss.eval.f / ss.eval.pdf);
+                if (ev) {
+                    ev->label = label;
+                    set3(ev->throughput, throughput);
+                }
+                if (any_nan(throughput) || throughput.x < 0.0f || throughput.y < 0.0f || throughput.z < 0.0f) {
+                    alive = false;
+                } else {
+                    ps = next_surface(ps, label, runtime, p);
+                    if (!transparent) {
+                        previous_bsdf_pdf = ss.eval.pdf;
+                        previous_delta = singular;
+                        b.mis_n[i] = make_float4(sp.n.x, sp.n.y, sp.n.z, 0.0f);
+                    }
+                    if (ev) {
+                        ev->bounce = ps.bounce;
+                        ev->transparent_bounce = ps.transparent_bounce;
+                        ev->flag = ps.flag;
+                        ev->visibility = ps.visibility;
+                    }
+                    if (transparent) {
+                        ray.tmin = next_float_up(h.t);
+                    } else {
+                        const f3 wi = normalize(ss.wi);
+                        const Xform w2o = world_to_object(s, sp.instance);
+                        ray.o = origin_with_self_exclusion(sp, sp.object_position, xform_direction(w2o, wi));
+                        ray.d = wi;
+                        ray.tmin = 0.0f;
+                        ray.tmax = 1.0e30f;
+                    }
+                    out.keep = true;
+                    st2.y = sp.object;
+                    st2.z = sp.cycles_prim;
+                }
+            }
+            if (!out.keep && ev) ev->terminated = 1u;
+        }
+    }
+    const float4 rad_out = make_float4(radiance.x, radiance.y, radiance.z, transparency);
+    // an ended path's radiance goes to the film's array; a path still
+    // alive after the last step (none, by the step bound) is written
+    // there as well
+    out.final = !out.keep || step + 1u >= p.steps;
+    if (out.final) b.rad_final[i] = rad_out;
+    if (out.keep) {
+        store_pair(b.ray_o, i, make_float4(ray.o.x, ray.o.y, ray.o.z, ray.tmin),
+                   make_float4(ray.d.x, ray.d.y, ray.d.z, ray.tmax));
+        store_pair(b.tp, i, make_float4(throughput.x, throughput.y, throughput.z, previous_bsdf_pdf), rad_out);
+        const uint4 st_out = make_uint4(ps.flag, ps.visibility, ps.rng_offset,
+                                        ps.bounce | (ps.diffuse_bounce << 8) | (ps.glossy_bounce << 16) |
+                                            (ps.transmission_bounce << 24));
+        uint32_t bits = ps.transparent_bounce & 0xffu;
+        if (previous_delta) bits |= kSt2Delta;
+        if (primary_recorded) bits |= kSt2Primary;
+        if ((ps.flag & kFlagTerminateOnNextSurface) != 0u) bits |= kSt2TermNext;
+        if ((ps.flag & kFlagTerminateAfterTransparent) != 0u) bits |= kSt2TermAfter;
+        st2.x = bits;
+        store_pair(b.st, i, st_out, st2);
+    }
+    return out;
+}
+
 // kMulti: paths of a batched wavefront, each shaded with its job's scene and
 // parameters.
 template <bool kTrace, bool kMulti, bool kGlossy>
@@ -712,6 +1064,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
     // match the wavefront's glossy flag (set by k_begin_round) returns
     if (kMulti && (b.counters[kCounterWaveGlossy] != 0u) != kGlossy) return;
     const uint32_t count = b.counters[0];
+    if (b.counters[kCounterTail] != 0u) return;
     const bool sorted = sort_threshold != 0u && count >= sort_threshold;
     const uint32_t *queue = sorted ? b.queue_sorted : b.queue_in;
     // a sorted queue's misses are k_shade_miss's (a traced launch takes all)
@@ -719,343 +1072,27 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
     const uint32_t rounds = (count - begin + gridDim.x * blockDim.x - 1u) / (gridDim.x * blockDim.x);
     // Every lane runs the same number of rounds so the warp-aggregated queue
     // pushes see the whole warp.
-    for (uint32_t r = 0; r < rounds; ++r) {
-        const uint32_t q = begin + r * gridDim.x * blockDim.x + blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t round = 0; round < rounds; ++round) {
+        const uint32_t q = begin + round * gridDim.x * blockDim.x + blockIdx.x * blockDim.x + threadIdx.x;
         const bool active = q < count;
-        bool keep = false;
-        bool shadow = false;
-        bool final = false;  // the path ends here (its radiance and shadow contribution go to rad_final)
+        ShadeResult r{};
         uint32_t i = 0u;
-        float4 sh_o, sh_d, sh_c;
-        uint4 sh_ids;
         if (active) {
             i = queue[q];
             const uint32_t job = kMulti ? b.job[i] : 0u;
             const SceneView &s = kMulti ? jobs[job].s : s_arg;
             const RenderParams &p = kMulti ? jobs[job].p : p_arg;
-            psy_path_event *ev = nullptr;
-            if (kTrace && trace && i == trace_path && step < PSY_TRACE_MAX_EVENTS) {
-                ev = &trace->events[step];
-                trace->event_count = step + 1u;
-            }
-            float4 ro, rd, tp4, rad4, h4;
-            uint4 st, st2, hp4;
-            load_pair(b.ray_o, i, ro, rd);
-            load_pair(b.tp, i, tp4, rad4);
-            load_pair(b.st, i, st, st2);
-            load_pair(b.hit, i, h4, hp4);
-            Ray ray{mk3(ro.x, ro.y, ro.z), mk3(rd.x, rd.y, rd.z), ro.w, rd.w};
-            f3 throughput = mk3(tp4.x, tp4.y, tp4.z);
-            float previous_bsdf_pdf = tp4.w;
-            f3 radiance = mk3(rad4.x, rad4.y, rad4.z);
-            float transparency = rad4.w;
-            PathState ps = unpack_state(st, st2);
-            bool previous_delta = (st2.x & kSt2Delta) != 0u;
-            bool primary_recorded = (st2.x & kSt2Primary) != 0u;
-            const bool terminate_on_next_surface = (st2.x & kSt2TermNext) != 0u;
-            const bool terminate_after_transparent = (st2.x & kSt2TermAfter) != 0u;
-            const uint32_t ray_visibility = contract_visibility(ps.visibility);
-            const uint32_t sample = b.sample[i];
-            const uint32_t local = st2.w;
-            const uint32_t x = p.win_x + local % p.win_w;
-            const uint32_t y = p.win_y + local / p.win_w;
-            const uint32_t rng_hash = pixel_hash(x, p.full_h - 1u - y, p.seed);
-            const float terminate_sample = sample_4d(p, sample, rng_hash, ps.rng_offset + 0u).x;
-            const float4 ls4 = sample_4d(p, sample, rng_hash, ps.rng_offset + 1u);
-            const f3 light_sample = mk3(ls4.x, ls4.y, ls4.z);
-            const float light_terminate = sample_4d(p, sample, rng_hash, ps.rng_offset + 2u).x;
-            const float4 bs4 = sample_4d(p, sample, rng_hash, ps.rng_offset + 3u);
-            // the flat distribution's pick; without a trace to record it, only
-            // paths that take a light sample search for theirs
-            DistEntryGpu selected{0.0f, 0.0f, 3u, 0u};
-            if (kTrace && !p.use_light_tree) selected = distribution_sample(s, light_sample.z);
-            const uint32_t prim = hp4.x;
-            if (ev) {
-                ev->rng_offset = ps.rng_offset;
-                ev->random_terminate = terminate_sample;
-                set3(ev->random_light, light_sample);
-                ev->random_light_terminate = light_terminate;
-                set3(ev->random_bsdf, mk3(bs4.x, bs4.y, bs4.z));
-                ev->light_kind = selected.kind;
-                ev->light_index = selected.index;
-                const bool missed = prim == kInvalid;
-                ev->hit_t = missed ? 0.0f : h4.x;
-                ev->hit_u = missed ? 0.0f : h4.y;
-                ev->hit_v = missed ? 0.0f : h4.z;
-                ev->closure_index = kInvalid;
-                ev->hit_object = kInvalid;
-                ev->hit_primitive = kInvalid;
-            }
-            const uint32_t depth = ps.bounce;
-            bool alive = true;
-            if (s.lamp_count > 0u)
-                alive = lamp_events(s, p, b, i, ray, prim == kInvalid ? ray.tmax : h4.x, ray_visibility, throughput,
-                                    previous_bsdf_pdf, previous_delta, ps, radiance, ev);
-            if (!alive) {
-                // a lamp event used up the transparent budget
-            } else if (prim == kInvalid) {
-                background_event(s, p, ray_visibility, throughput, ps, radiance, transparency, ev);
-                if (ev) ev->terminated = 1u;
-                alive = false;
-            } else {
-                Hit h;
-                h.t = h4.x;
-                h.u = h4.y;
-                h.v = h4.z;
-                h.instance = __float_as_uint(h4.w);
-                h.prim = prim;
-                h.object = h.instance;
-                const SurfacePoint sp = surface_point(s, h, ray.d);
-                if (ev) {
-                    ev->hit_object = h.object;
-                    ev->hit_primitive = sp.cycles_prim;
-                }
-                const BakedMaterialGpu mat = s.baked[sp.material];
-                SurfaceClosures<kGlossy> closures;
-                const ClosurePoint cpt{sp.n, sp.ng, -ray.d, safe_normalize(-ray.d, sp.n), mat.bump_correction != 0u,
-                                       sp.back_facing};
-                collect_surface<kGlossy>(s, mat, cpt, closures);
-                // SurfaceShadingStageImpl::emit (src/luisa/path_kernel_surface_shading.cpp:117-250)
-                float emission_weight = 1.0f;
-                if (p.nee && s.triangle_emitters > 0u && mat.emission_sampling != 0u && mat.has_emission) {
-                    const bool competing = depth > 0u && !previous_delta;
-                    float selection_pdf =
-                        0.5f * length(cross(sp.wp1 - sp.wp0, sp.wp2 - sp.wp0)) * s.triangle_area_pdf;
-                    if (p.use_light_tree) {
-                        // light_tree.forward_pdf (src/luisa/path_tracer_light_tree.cpp:799-838)
-                        const float4 mn = b.mis_n[i];
-                        selection_pdf = lt_pdf(s, lt_triangle_emitter(s, sp.object, sp.cycles_prim), ray.o,
-                                               mk3(mn.x, mn.y, mn.z), (ps.flag & kFlagMisHadTransmission) != 0u);
-                    }
-                    const float light_pdf = emissive_forward_pdf(selection_pdf, mat.emission_sampling, ray.o,
-                                                                 sp.position, sp.wp0, sp.wp1, sp.wp2,
-                                                                 // the geometric normal before the back-face
-                                                                 // flip (path_kernel_surface_shading.cpp:130-134)
-                                                                 sp.back_facing ? -sp.ng : sp.ng);
-                    const bool available = light_pdf > 0.0f;
-                    emission_weight = forward_light_weight(p.direct_mode, previous_bsdf_pdf, light_pdf, competing, available);
-                }
-                const f3 ec = clamp_contribution(throughput * closures.emission * emission_weight, depth, p);
-                radiance = radiance + ec;
-                if (ev) add3(ev->emission, ec);
-                if (terminate_on_next_surface) {
-                    alive = false;
-                    if (ev) ev->terminated = 1u;
-                }
-                if (alive) {
-                    // continuation_probability (cycles_path_state.h:413-447)
-                    const bool tr_state = (ps.flag & kFlagTransparent) != 0u;
-                    const bool before_min = tr_state ? ps.transparent_bounce <= p.transparent_min : ps.bounce <= p.minimum;
-                    const float cp = before_min ? 1.0f : minf_(sqrtf(max_abs_component(throughput)), 1.0f);
-                    if (ev) ev->continuation_probability = cp;
-                    if (cp <= 0.0f) {
-                        alive = false;
-                    } else if (cp != 1.0f) {
-                        if (terminate_sample >= cp) alive = false;
-                        else throughput = throughput / cp;
-                    }
-                    if (!alive && ev) ev->terminated = 1u;
-                }
-                if (alive) {
-                    if (depth == 0u) {
-                        f3 aov_albedo, aov_normal, aov_transparency;
-                        surface_aov<kGlossy>(closures, cpt, aov_albedo, aov_normal, aov_transparency);
-                        const float4 a4 = b.aov_a[i];
-                        const f3 acc = mk3(a4.x, a4.y, a4.z) + throughput * aov_albedo;
-                        b.aov_a[i] = make_float4(acc.x, acc.y, acc.z, 0.0f);
-                        const f3 alpha = clamp3(mk3(1.0f) - aov_transparency, 0.0f, 1.0f);
-                        const float average_alpha = (alpha.x + alpha.y + alpha.z) * (1.0f / 3.0f);
-                        const bool writes_normal = !primary_recorded && (p.pass_alpha_threshold == 0.0f ||
-                                                                         average_alpha >= p.pass_alpha_threshold);
-                        if (writes_normal) {
-                            b.aov_n[i] = make_float4(aov_normal.x, aov_normal.y, aov_normal.z, 0.0f);
-                            primary_recorded = true;
-                            ps.flag |= kFlagSinglePassDone;
-                        }
-                    }
-                    const uint32_t runtime = mat.runtime | (sp.back_facing ? kRuntimeBackfacing : 0u);
-                    if (p.use_light_tree) {
-                        // light-tree pick after shading (src/luisa/path_kernel_pipeline.cpp:150-159)
-                        selected = lt_sample(s, light_sample.z, sp.position, sp.n,
-                                             (runtime & kRuntimeBsdfHasTransmission) != 0u);
-                        if (ev) {
-                            ev->light_kind = selected.kind;
-                            ev->light_index = selected.index;
-                        }
-                    }
-                    const uint32_t lobe_mask = terminate_after_transparent ? kEventTransparent : 0xffffffffu;
-                    // Direct lighting (src/luisa/path_kernel_pipeline.cpp:160-172)
-                    if (p.nee && (runtime & kRuntimeBsdfHasEval) != 0u) {
-                        if (!kTrace && !p.use_light_tree) selected = distribution_sample(s, light_sample.z);
-                        f3 lp = mk3(0.0f), ldir = mk3(0.0f);
-                        float ldist = 0.0f;
-                        bool distant = false;
-                        f3 surviving = mk3(0.0f);
-                        uint32_t light_obj = kInvalid, light_prim = kInvalid;
-                        bool emit = false;
-                        // The light sample of either kind, then one BSDF
-                        // evaluation, MIS weight and light roulette shared by
-                        // both (a warp's lanes that picked triangles and lamps
-                        // evaluate together).
-                        bool sampled = false, weigh_mis = true;
-                        f3 light_radiance = mk3(0.0f);
-                        float light_pdf = 0.0f, pdf_divisor = 1.0f;
-                        if (selected.kind == 0u) {
-                            // EmissiveMeshLightingComponent (src/luisa/path_kernel_nee_emissive_mesh.cpp:32-296)
-                            const Emitter em = load_emitter(s.emitters + selected.index);
-                            const TriSample ls = sample_triangle(sp.position, em.p0, em.p1, em.p2,
-                                                                 mk2(light_sample.x, light_sample.y));
-                            const bool side = sampled_side(em.emission_sampling, em.ng, ls.direction);
-                            const float pdf = ls.pdf * selected.selection_pdf;
-                            if (ls.valid && side && em.area > 0.0f && pdf > 0.0f) {
-                                const bool is_transmission = dot(ls.direction, sp.n) < 0.0f;
-                                const bool same_primitive = em.cycles_prim == sp.cycles_prim && em.object == sp.object;
-                                const f3 oriented = is_transmission ? -sp.ng : sp.ng;
-                                const bool reject_self = same_primitive && dot(ls.direction, oriented) > 0.0f;
-                                if (!reject_self) {
-                                    sampled = true;
-                                    light_radiance = ld3(__ldg(&s.baked[em.material].emission));
-                                    light_pdf = pdf;
-                                    pdf_divisor = pdf;
-                                    lp = ls.position;
-                                    light_obj = em.object;
-                                    light_prim = em.cycles_prim;
-                                    ldir = ls.direction;
-                                }
-                            }
-                        } else if (selected.kind == 1u) {
-                            // AnalyticLightingComponent (src/luisa/path_kernel_nee_analytic.cpp:98-428)
-                            const psy_light_desc &l = s.lights[selected.index];
-                            if (!(depth > l.max_bounces)) {
-                                const AnalyticSample a =
-                                    sample_analytic(l, s.lamp_consts[selected.index], sp.position, sp.n,
-                                                    (runtime & kRuntimeBsdfHasTransmission) != 0u,
-                                                    mk2(light_sample.x, light_sample.y));
-                                const float pdf = a.pdf * selected.selection_pdf;
-                                if (a.valid && pdf > 0.0f) {
-                                    sampled = true;
-                                    light_radiance = ld3(l.color) * (l.power * a.eval_factor);
-                                    light_pdf = pdf;
-                                    pdf_divisor = maxf_(pdf, 1.0e-20f);
-                                    // MIS only for lamps a BSDF ray can also hit
-                                    // (path_kernel_nee_analytic.cpp:286-292)
-                                    weigh_mis = (l.flags & kLightFlagForward) != 0u;
-                                    lp = a.position;
-                                    ldir = a.direction;
-                                    distant = l.type == PSY_LIGHT_DISTANT;
-                                }
-                            }
-                        }
-                        if (sampled) {
-                            const Evaluation e = evaluate_mixture<kGlossy>(closures, cpt, ldir, lobe_mask, -1);
-                            const float mis = weigh_mis ? nee_light_weight(p.direct_mode, light_pdf, e.pdf) : 1.0f;
-                            const f3 weighted = e.f * light_radiance * (mis / pdf_divisor);
-                            if (any_nonzero(weighted)) {
-                                const f3 unshadowed = weighted * mk3(1.0f);
-                                surviving =
-                                    unshadowed * light_roulette_weight(unshadowed, light_terminate, p.inv_rr_threshold);
-                                emit = any_nonzero(surviving);
-                            }
-                        }
-                        if (emit) {
-                            // make_shadow_origin (src/luisa/path_kernel_surface_geometry.cpp:168-185)
-                            const Xform w2o = world_to_object(s, sp.instance);
-                            const f3 so = origin_with_self_exclusion(sp, xform_point(w2o, sp.position),
-                                                                     xform_direction(w2o, ldir));
-                            const f3 off = lp - so;
-                            const float fd = sqrtf(maxf_(dot(off, off), 1.0e-20f));
-                            const f3 sdir = distant ? ldir : off / fd;
-                            ldist = distant ? 1.0e30f : fd;
-                            const f3 c = throughput * surviving;
-                            sh_o = make_float4(so.x, so.y, so.z, ldist);
-                            sh_d = make_float4(sdir.x, sdir.y, sdir.z, __uint_as_float(ps.transparent_bounce));
-                            sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(depth));
-                            sh_ids = make_uint4(sp.object, sp.cycles_prim, light_obj, light_prim);
-                            shadow = true;
-                        }
-                    }
-                    // SurfaceScatterStageImpl::emit (src/luisa/path_kernel_surface_scatter.cpp:136-291)
-                    const SurfaceSample ss = sample_surface<kGlossy>(closures, cpt, bs4.z, mk2(bs4.x, bs4.y), lobe_mask);
-                    if (ev) {
-                        ev->closure_index = ss.closure_index;
-                        ev->bsdf_pdf = ss.eval.pdf;
-                        set3(ev->wi, ss.wi);
-                    }
-                    if (!ss.valid || ss.eval.pdf <= 0.0f) {
-                        alive = false;
-                    } else {
-                        const bool transparent = (ss.eval.events & kEventTransparent) != 0u;
-                        const bool singular = (ss.eval.events & kEventSingular) != 0u;
-                        const uint32_t label = label_from_events(ss.eval.events);
-                        throughput = throughput * (ss.eval.f / ss.eval.pdf);
-                        if (ev) {
-                            ev->label = label;
-                            set3(ev->throughput, throughput);
-                        }
-                        if (any_nan(throughput) || throughput.x < 0.0f || throughput.y < 0.0f || throughput.z < 0.0f) {
-                            alive = false;
-                        } else {
-                            ps = next_surface(ps, label, runtime, p);
-                            if (!transparent) {
-                                previous_bsdf_pdf = ss.eval.pdf;
-                                previous_delta = singular;
-                                b.mis_n[i] = make_float4(sp.n.x, sp.n.y, sp.n.z, 0.0f);
-                            }
-                            if (ev) {
-                                ev->bounce = ps.bounce;
-                                ev->transparent_bounce = ps.transparent_bounce;
-                                ev->flag = ps.flag;
-                                ev->visibility = ps.visibility;
-                            }
-                            if (transparent) {
-                                ray.tmin = next_float_up(h.t);
-                            } else {
-                                const f3 wi = normalize(ss.wi);
-                                const Xform w2o = world_to_object(s, sp.instance);
-                                ray.o = origin_with_self_exclusion(sp, sp.object_position, xform_direction(w2o, wi));
-                                ray.d = wi;
-                                ray.tmin = 0.0f;
-                                ray.tmax = 1.0e30f;
-                            }
-                            keep = true;
-                            st2.y = sp.object;
-                            st2.z = sp.cycles_prim;
-                        }
-                    }
-                    if (!keep && ev) ev->terminated = 1u;
-                }
-            }
-            const float4 rad_out = make_float4(radiance.x, radiance.y, radiance.z, transparency);
-            // an ended path's radiance goes to the film's array; a path still
-            // alive after the last step (none, by the step bound) is written
-            // there as well
-            final = !keep || step + 1u >= p.steps;
-            if (final) b.rad_final[i] = rad_out;
-            if (keep) {
-                store_pair(b.ray_o, i, make_float4(ray.o.x, ray.o.y, ray.o.z, ray.tmin),
-                           make_float4(ray.d.x, ray.d.y, ray.d.z, ray.tmax));
-                store_pair(b.tp, i, make_float4(throughput.x, throughput.y, throughput.z, previous_bsdf_pdf), rad_out);
-                const uint4 st_out = make_uint4(ps.flag, ps.visibility, ps.rng_offset,
-                                                ps.bounce | (ps.diffuse_bounce << 8) | (ps.glossy_bounce << 16) |
-                                                    (ps.transmission_bounce << 24));
-                uint32_t bits = ps.transparent_bounce & 0xffu;
-                if (previous_delta) bits |= kSt2Delta;
-                if (primary_recorded) bits |= kSt2Primary;
-                if ((ps.flag & kFlagTerminateOnNextSurface) != 0u) bits |= kSt2TermNext;
-                if ((ps.flag & kFlagTerminateAfterTransparent) != 0u) bits |= kSt2TermAfter;
-                st2.x = bits;
-                store_pair(b.st, i, st_out, st2);
-            }
+            r = shade_path<kTrace, kGlossy>(s, p, b, i, step, trace_path, trace);
         }
-        const uint32_t slot = warp_push(&b.counters[1], active && keep);
-        if (active && keep) b.queue_out[slot] = i;
-        const uint32_t sslot = warp_push(&b.counters[2], active && shadow);
-        if (active && shadow) {
-            b.sh_o[sslot] = sh_o;
-            b.sh_d[sslot] = sh_d;
-            b.sh_c[sslot] = sh_c;
-            b.sh_ids[sslot] = sh_ids;
-            b.sh_path[sslot] = i | (final ? kShadowFinal : 0u);
+        const uint32_t slot = warp_push(&b.counters[1], r.keep);
+        if (r.keep) b.queue_out[slot] = i;
+        const uint32_t sslot = warp_push(&b.counters[2], r.shadow);
+        if (r.shadow) {
+            b.sh_o[sslot] = r.sh_o;
+            b.sh_d[sslot] = r.sh_d;
+            b.sh_c[sslot] = r.sh_c;
+            b.sh_ids[sslot] = r.sh_ids;
+            b.sh_path[sslot] = i | (r.final ? kShadowFinal : 0u);
         }
     }
 }
@@ -1141,10 +1178,126 @@ __device__ __forceinline__ uint32_t surface_material(const SceneView &s, uint32_
     return m != kInvalid ? m : __ldg(&s.shade_tris[cycles_prim].material);
 }
 
-// Persistent any-hit shadow kernel (same refill scheme as k_intersect).
-// Opaque-only scenes stop at the first accepted candidate; otherwise
-// transparent hits are collected per lane and resolved by distance once
-// the traversal ends.
+// The transparent surfaces a shadow ray has met, and their product so far.
+struct ShadowHits {
+    float t[kShadowList];
+    uint32_t object[kShadowList], prim[kShadowList], material[kShadowList];
+    int n;
+    uint32_t passed;  // surfaces before the ray's current start
+    f3 transmittance;  // and their product
+    bool blocked, overflow;
+};
+
+__device__ __forceinline__ void shadow_begin(ShadowHits &h, uint32_t transparent_depth) {
+    h.blocked = h.overflow = false;
+    h.n = 0;
+    h.passed = transparent_depth;
+    h.transmittance = mk3(1.0f);
+}
+
+// A surface on the ray; true once it is known to be blocked.
+__device__ __forceinline__ bool shadow_hit(ShadowHits &h, const SceneView &s, const RenderParams &p, uint32_t instance,
+                                           uint32_t cycles_prim, float t) {
+    // opaque-only scenes stop at the first accepted candidate
+    const uint32_t tagged = s.any_transparent ? surface_material(s, instance, cycles_prim) : 0u;
+    if ((tagged & kMaterialTransparent) == 0u) {
+        h.blocked = true;
+        return true;
+    }
+    const uint32_t material = tagged & ~kMaterialTransparent;
+    for (int k = 0; k < h.n; ++k) {
+        if (h.t[k] == t) {  // coincident: keep the greatest identity
+            if (instance > h.object[k] || (instance == h.object[k] && cycles_prim > h.prim[k])) {
+                h.object[k] = instance;
+                h.prim[k] = cycles_prim;
+                h.material[k] = material;
+            }
+            return false;
+        }
+    }
+    int slot = h.n;
+    if (h.n == kShadowList) {
+        // more surfaces than the collector holds: keep the nearest, unless
+        // they exceed the ray's budget already
+        if (h.passed + uint32_t(kShadowList) >= p.transparent_max) {
+            h.blocked = true;
+            return true;
+        }
+        h.overflow = true;
+        slot = 0;
+        for (int k = 1; k < kShadowList; ++k)
+            if (h.t[k] > h.t[slot]) slot = k;
+        if (t > h.t[slot]) return false;
+    } else {
+        ++h.n;
+    }
+    h.t[slot] = t;
+    h.object[slot] = instance;
+    h.prim[slot] = cycles_prim;
+    h.material[slot] = material;
+    return false;
+}
+
+// Multiplies the surfaces met in distance order.  False if the ray has to go
+// on from behind them: `t` has been restarted there.
+__device__ __forceinline__ bool shadow_resolve(ShadowHits &h, TraversalState &t, const SceneView &s,
+                                               const RenderParams &p) {
+    // (transparent_max - passed surfaces may still lie on the ray)
+    if (uint32_t(h.n) > (h.passed >= p.transparent_max ? 0u : p.transparent_max - h.passed)) h.blocked = true;
+    if (!h.blocked) {
+        for (int i = 1; i < h.n; ++i) {
+            const float kt = h.t[i];
+            const uint32_t km = h.material[i];
+            int j = i - 1;
+            while (j >= 0 && h.t[j] > kt) {
+                h.t[j + 1] = h.t[j];
+                h.material[j + 1] = h.material[j];
+                --j;
+            }
+            h.t[j + 1] = kt;
+            h.material[j + 1] = km;
+        }
+        for (int i = 0; i < h.n; ++i) {
+            const f3 e = clamp3(ld3(__ldg(&s.baked[h.material[i]].extinction)), 0.0f, 1.0f);
+            if (!(max_component(e) > 0.0f)) {
+                h.blocked = true;
+                break;
+            }
+            h.transmittance = h.transmittance * e;
+        }
+        if (!h.blocked && h.overflow) {
+            h.passed += uint32_t(h.n);
+            Ray ray = t.ray;
+            ray.tmin = next_float_up(h.t[h.n - 1]);
+            traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, t.src_obj, t.src_prim, t.light_obj, t.light_prim);
+            h.overflow = false;
+            h.n = 0;
+            return false;
+        }
+    }
+    if (h.blocked) h.transmittance = mk3(0.0f);
+    return true;
+}
+
+// The NEE contribution of a resolved shadow ray, added to its path's radiance.
+__device__ __forceinline__ f3 shadow_contribute(const PathBuffers &b, const RenderParams &p, f3 transmittance, float4 c,
+                                                uint32_t path, bool final) {
+    f3 contribution = mk3(0.0f);
+    if (transmittance.x > 0.0f || transmittance.y > 0.0f || transmittance.z > 0.0f) {
+        contribution = clamp_contribution(mk3(c.x, c.y, c.z) * transmittance, __float_as_uint(c.w), p);
+        float4 &dst = final ? b.rad_final[path] : b.rad[path];
+        float4 r = dst;
+        r.x += contribution.x;
+        r.y += contribution.y;
+        r.z += contribution.z;
+        dst = r;
+    }
+    return contribution;
+}
+
+// Persistent any-hit shadow kernel (same refill scheme as k_intersect):
+// transparent hits are collected per lane and resolved by distance once the
+// traversal ends.
 // kMulti: shadow rays of a batched wavefront, each in its path's job.
 template <bool kMulti>
 __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
@@ -1152,18 +1305,15 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
              const __grid_constant__ PathBuffers b, uint32_t step, uint32_t trace_path, psy_path_trace *trace,
              const JobGpu *jobs, uint32_t sort_threshold) {
     const uint32_t count = b.counters[2];
+    if (b.counters[kCounterTail] != 0u) return;
     const bool sorted = sort_threshold != 0u && count >= sort_threshold;
     TraversalState t;
     t.node = kLinkDone;
     t.leaves = 0u;
-    bool active = false, exhausted = false, blocked = false, overflow = false;
+    bool active = false, exhausted = false;
     uint32_t q_cur = 0u, job = 0u;
-    float lt[kShadowList];
-    uint32_t lo[kShadowList], lp[kShadowList], lm[kShadowList];
-    int n = 0;
-    // surfaces and their product before the ray's current start
-    uint32_t passed = 0u;
-    f3 transmittance = mk3(1.0f);
+    ShadowHits h;
+    shadow_begin(h, 0u);
     for (;;) {
         uint32_t q = warp_fetch(&b.counters[4], count, !active, exhausted);
         if (sorted && q != kInvalid) q = b.queue_sorted[q];
@@ -1176,110 +1326,103 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
             const uint4 ids = b.sh_ids[q];
             const Ray ray{mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w};
             traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w);
-            blocked = overflow = false;
-            n = 0;
-            passed = __float_as_uint(d.w);
-            transmittance = mk3(1.0f);
+            shadow_begin(h, __float_as_uint(d.w));
             active = true;
         }
         const int busy = __popc(__ballot_sync(kFullMask, active));
         if (busy == 0) break;
         traverse_warp<false>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
                              [&](uint32_t ii, uint32_t, uint32_t cp, float th, float, float) {
-            if (!s.any_transparent) {
-                blocked = true;
-                return true;
-            }
-            uint32_t mi = surface_material(s, ii, cp);
-            if ((mi & kMaterialTransparent) == 0u) {
-                blocked = true;
-                return true;
-            }
-            mi &= ~kMaterialTransparent;
-            for (int k = 0; k < n; ++k) {
-                if (lt[k] == th) {
-                    if (ii > lo[k] || (ii == lo[k] && cp > lp[k])) {
-                        lo[k] = ii;
-                        lp[k] = cp;
-                        lm[k] = mi;
-                    }
-                    return false;
-                }
-            }
-            int slot = n;
-            if (n == kShadowList) {
-                // more surfaces than the collector holds: keep the nearest,
-                // unless they exceed the ray's budget already
-                if (passed + uint32_t(kShadowList) >= p.transparent_max) {
-                    blocked = true;
-                    return true;
-                }
-                overflow = true;
-                slot = 0;
-                for (int k = 1; k < kShadowList; ++k)
-                    if (lt[k] > lt[slot]) slot = k;
-                if (th > lt[slot]) return false;
-            } else {
-                ++n;
-            }
-            lt[slot] = th;
-            lo[slot] = ii;
-            lp[slot] = cp;
-            lm[slot] = mi;
-            return false;
+            return shadow_hit(h, s, p, ii, cp, th);
         });
         if (!active || t.node != kLinkDone || t.leaves != 0u) continue;
-        // (transparent_max - passed surfaces may still lie on the ray)
-        if (uint32_t(n) > (passed >= p.transparent_max ? 0u : p.transparent_max - passed)) blocked = true;
-        if (!blocked) {
-            for (int i = 1; i < n; ++i) {
-                const float kt = lt[i];
-                const uint32_t km = lm[i];
-                int j = i - 1;
-                while (j >= 0 && lt[j] > kt) {
-                    lt[j + 1] = lt[j];
-                    lm[j + 1] = lm[j];
-                    --j;
-                }
-                lt[j + 1] = kt;
-                lm[j + 1] = km;
-            }
-            for (int i = 0; i < n; ++i) {
-                const f3 e = clamp3(ld3(__ldg(&s.baked[lm[i]].extinction)), 0.0f, 1.0f);
-                if (!(max_component(e) > 0.0f)) {
-                    blocked = true;
-                    break;
-                }
-                transmittance = transmittance * e;
-            }
-            if (!blocked && overflow) {
-                passed += uint32_t(n);
-                const uint4 ids = b.sh_ids[q_cur];
-                Ray ray = t.ray;
-                ray.tmin = next_float_up(lt[n - 1]);
-                traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, ids.x, ids.y, ids.z, ids.w);
-                overflow = false;
-                n = 0;
-                continue;
-            }
-        }
-        if (blocked) transmittance = mk3(0.0f);
+        if (!shadow_resolve(h, t, s, p)) continue;
         active = false;
-        const float4 c = b.sh_c[q_cur];
-        const uint32_t depth = __float_as_uint(c.w);
-        const uint32_t owner = b.sh_path[q_cur];
-        const uint32_t path = owner & ~kShadowFinal;
-        f3 contribution = mk3(0.0f);
-        if (transmittance.x > 0.0f || transmittance.y > 0.0f || transmittance.z > 0.0f) {
-            contribution = clamp_contribution(mk3(c.x, c.y, c.z) * transmittance, depth, p);
-            float4 &dst = (owner & kShadowFinal) != 0u ? b.rad_final[path] : b.rad[path];
-            float4 r = dst;
-            r.x += contribution.x;
-            r.y += contribution.y;
-            r.z += contribution.z;
-            dst = r;
-        }
+        const uint32_t owner = b.sh_path[q_cur], path = owner & ~kShadowFinal;
+        const f3 contribution =
+            shadow_contribute(b, p, h.transmittance, b.sh_c[q_cur], path, (owner & kShadowFinal) != 0u);
         if (trace && path == trace_path && step < PSY_TRACE_MAX_EVENTS) set3(trace->events[step].nee, contribution);
+    }
+}
+
+// -------------------------------------------------------------------- tail
+// All remaining steps of a queue that has become short (k_end_step marks the
+// step from which counters[0] is below the limit), one path a lane: closest
+// hit, shading and shadow ray follow one another without a launch between.
+// In a short queue a step's three launches each wait for their longest ray
+// while the GPU idles, so a path that still bounces pays that wait for
+// every step; here it pays only for the paths of its own warp, and a warp
+// takes few of them (as many as spread the queue over all resident warps).
+// 128x128 procedural viewport at 1 spp: 3.12 -> 1.15 ms; value materials at
+// 512x512, 4 spp: 2.68 -> 2.00 ms; 1080p frame, 64 spp: 340.5 -> 338.8 ms.  The
+// limit of 64 Ki paths lies where these turn: 16 Ki 1.32 / 2.11 / 340.2 ms, 32 Ki
+// 1.21 / 2.16 / 339.5, 64 Ki 1.21 / 2.06 / 339.1 (4 blocks an SM; 3 as above), 128 Ki
+// 1.22 / 2.76 / 341.3.
+template <bool kMulti, bool kGlossy>
+__global__ void __launch_bounds__(128, PSY_TAIL_MIN_BLOCKS)
+    k_tail(const __grid_constant__ SceneView s_arg, const __grid_constant__ RenderParams p_arg,
+           const __grid_constant__ PathBuffers b, const uint32_t *odd_queue, const JobGpu *jobs,
+           unsigned long long *stats) {
+    if (kMulti && (b.counters[kCounterWaveGlossy] != 0u) != kGlossy) return;
+    if (b.counters[kCounterTail] == 0u) return;
+    const uint32_t start = b.counters[kCounterTail] - 1u, count = b.counters[0];
+    const uint32_t *queue = (start & 1u) != 0u ? odd_queue : b.queue_in;
+    const uint32_t warps = gridDim.x * 4u, warp = blockIdx.x * 4u + (threadIdx.x >> 5);
+    const uint32_t share = min(32u, (count + warps - 1u) / warps);
+    uint32_t closest_rays = 0u, shadow_rays = 0u;
+    for (uint32_t base = warp * share; base < count; base += warps * share) {
+        const uint32_t q = base + lane_id();
+        bool active = lane_id() < share && q < count;
+        const uint32_t i = active ? queue[q] : 0u;
+        const uint32_t job = kMulti && active ? b.job[i] : 0u;
+        const SceneView &s = kMulti ? jobs[job].s : s_arg;
+        const RenderParams &p = kMulti ? jobs[job].p : p_arg;
+        for (uint32_t step = start; __any_sync(kFullMask, active); ++step) {
+            TraversalState t;
+            t.node = kLinkDone;
+            t.leaves = 0u;
+            ClosestHit best;
+            if (active) {
+                closest_begin(best, t, s, b, i);
+                closest_rays += 1u;
+            }
+            traverse_warp<true>(t, s, 32, [&](uint32_t ii, uint32_t local, uint32_t, float th, float u, float v) {
+                return closest_hit(best, t, ii, local, th, u, v);
+            });
+            ShadeResult r{};
+            if (active) {
+                closest_store(best, b, i);
+                r = shade_path<false, kGlossy>(s, p, b, i, step, kInvalid, nullptr);
+            }
+            if (__any_sync(kFullMask, r.shadow)) {
+                ShadowHits h;
+                shadow_begin(h, __float_as_uint(r.sh_d.w));
+                t.node = kLinkDone;
+                t.leaves = 0u;
+                bool pending = r.shadow;
+                if (pending) {
+                    const Ray ray{ld3(r.sh_o), ld3(r.sh_d), 0.0f, r.sh_o.w};
+                    traversal_begin(t, s, ray, PSY_VISIBILITY_SHADOW, r.sh_ids.x, r.sh_ids.y, r.sh_ids.z, r.sh_ids.w);
+                    shadow_rays += 1u;
+                }
+                while (__any_sync(kFullMask, pending)) {
+                    traverse_warp<false>(t, s, 32, [&](uint32_t ii, uint32_t, uint32_t cp, float th, float, float) {
+                        return shadow_hit(h, s, p, ii, cp, th);
+                    });
+                    if (pending && shadow_resolve(h, t, s, p)) {
+                        shadow_contribute(b, p, h.transmittance, r.sh_c, i, r.final);
+                        pending = false;
+                    }
+                }
+            }
+            active = r.keep && step + 1u < p.steps;
+        }
+    }
+    closest_rays = __reduce_add_sync(kFullMask, closest_rays);
+    shadow_rays = __reduce_add_sync(kFullMask, shadow_rays);
+    if (lane_id() == 0u && closest_rays != 0u) {
+        atomicAdd(&stats[0], (unsigned long long)closest_rays);
+        atomicAdd(&stats[1], (unsigned long long)shadow_rays);
     }
 }
 
@@ -1360,7 +1503,8 @@ __global__ void k_film_batch(const JobGpu *jobs, const BatchItem *items, const u
 // later kernel reads), the queue counters are set, and the cursor advances.
 // One block.
 __global__ void k_begin_round(uint32_t *counters, uint32_t *round, BatchItem *items, const uint32_t *plan_rounds,
-                              const BatchItem *plan_items, uint32_t *cursor, uint32_t max_items) {
+                              const BatchItem *plan_items, uint32_t *cursor, uint32_t max_items,
+                              uint32_t tail_paths) {
     const uint32_t w = *cursor;
     const uint32_t n = plan_rounds[4u * w + 2u];
     for (uint32_t k = threadIdx.x; k < n && k < max_items; k += blockDim.x)
@@ -1373,30 +1517,33 @@ __global__ void k_begin_round(uint32_t *counters, uint32_t *round, BatchItem *it
         counters[kCounterWaveGlossy] = plan_rounds[4u * w + 3u];
         counters[0] = round[0];
         counters[1] = counters[2] = counters[3] = counters[4] = 0u;
+        counters[kCounterTail] = round[0] < tail_paths ? 1u : 0u;
         *cursor = w + 1u;
     }
 }
 
-__global__ void k_swap_counters(uint32_t *counters) {
+// End of step `step`: its rays are counted, the survivors become the next
+// step's queue, and a queue shorter than `tail_paths` is marked for k_tail --
+// the launches of later steps find the mark and return.
+__global__ void k_end_step(uint32_t *counters, unsigned long long *stats, uint32_t step, uint32_t tail_paths) {
+    if (counters[kCounterTail] != 0u) return;
+    stats[0] += counters[0];
+    stats[1] += counters[2];
     counters[0] = counters[1];
     counters[1] = 0u;
     counters[2] = 0u;
     counters[3] = 0u;
     counters[4] = 0u;
+    if (counters[0] < tail_paths) counters[kCounterTail] = step + 2u;
 }
 
-__global__ void k_set_counters(uint32_t *counters, uint32_t n) {
+__global__ void k_set_counters(uint32_t *counters, uint32_t n, uint32_t tail_paths) {
     counters[0] = n;
     counters[1] = 0u;
     counters[2] = 0u;
     counters[3] = 0u;
     counters[4] = 0u;
-}
-
-// Accumulates the number of rays traced by the queues of one step.
-__global__ void k_count_rays(const uint32_t *counters, unsigned long long *stats) {
-    stats[0] += counters[0];
-    stats[1] += counters[2];
+    counters[kCounterTail] = n < tail_paths ? 1u : 0u;
 }
 
 __global__ void k_check_counts(const uint32_t *counts, uint32_t n, uint32_t expected, uint32_t *mismatch) {
@@ -1484,7 +1631,9 @@ void launch_raygen(cudaStream_t st, const LaunchConfig &lc, const RenderParams &
     k_raygen<<<launch_grid(paths, int(lc.stream_block), lc), lc.stream_block, 0, st>>>(p, b, pixels, paths, sample_base,
                                                                                     trace_path, trace);
 }
-void launch_set_counters(cudaStream_t st, uint32_t *counters, uint32_t n) { k_set_counters<<<1, 1, 0, st>>>(counters, n); }
+void launch_set_counters(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t n) {
+    k_set_counters<<<1, 1, 0, st>>>(counters, n, lc.tail_paths);
+}
 // Persistent kernels: enough resident warps to fill every SM (bounded by the
 // work so small queues launch few blocks).
 int shade_grid(uint32_t work, const LaunchConfig &lc) {
@@ -1553,13 +1702,32 @@ void launch_shadow(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, 
     k_shadow<false><<<persistent_grid(max_work, lc), 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr,
                                                                    lc.shadow_sort_threshold);
 }
-void launch_begin_round(cudaStream_t st, uint32_t *counters, uint32_t *round, BatchItem *items,
+void launch_begin_round(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t *round, BatchItem *items,
                         const uint32_t *plan_rounds, const BatchItem *plan_items, uint32_t *cursor, uint32_t max_items) {
-    k_begin_round<<<1, 256, 0, st>>>(counters, round, items, plan_rounds, plan_items, cursor, max_items);
+    k_begin_round<<<1, 256, 0, st>>>(counters, round, items, plan_rounds, plan_items, cursor, max_items, lc.tail_paths);
 }
-void launch_swap(cudaStream_t st, uint32_t *counters) { k_swap_counters<<<1, 1, 0, st>>>(counters); }
-void launch_count_rays(cudaStream_t st, const uint32_t *counters, unsigned long long *stats) {
-    k_count_rays<<<1, 1, 0, st>>>(counters, stats);
+void launch_end_step(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, unsigned long long *stats,
+                     uint32_t step) {
+    k_end_step<<<1, 1, 0, st>>>(counters, stats, step, lc.tail_paths);
+}
+// Blocks of the tail kernel: all that are resident, but no more than give
+// each warp a path.
+int tail_grid(const LaunchConfig &lc, uint32_t max_work) {
+    return int(std::min(uint32_t(lc.sms) * PSY_TAIL_MIN_BLOCKS, (std::min(max_work, lc.tail_paths) + 3u) / 4u));
+}
+void launch_tail(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+                 uint32_t max_work, unsigned long long *stats) {
+    if (lc.tail_paths == 0u) return;
+    const int grid = tail_grid(lc, max_work);
+    if (s.has_glossy) k_tail<false, true><<<grid, 128, 0, st>>>(s, p, b, b.queue_out, nullptr, stats);
+    else k_tail<false, false><<<grid, 128, 0, st>>>(s, p, b, b.queue_out, nullptr, stats);
+}
+void launch_tail_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b,
+                       uint32_t max_work, unsigned long long *stats) {
+    if (lc.tail_paths == 0u) return;
+    const int grid = tail_grid(lc, max_work);
+    k_tail<true, false><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, b.queue_out, jobs, stats);
+    k_tail<true, true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, b.queue_out, jobs, stats);
 }
 void launch_check_counts(cudaStream_t st, const uint32_t *counts, uint32_t n, uint32_t expected, uint32_t *mismatch) {
     cudaMemsetAsync(mismatch, 0, sizeof(uint32_t), st);

@@ -18,21 +18,27 @@ struct LaunchConfig {
     uint32_t shadow_sort_threshold = 0;     // shadow queue by direction (off: it measured slower); 0: never
     uint32_t ray_sort_threshold = 0;        // closest-hit queue by origin cell and octant (off: it measured slower)
     uint32_t stream_block = 256;            // threads per block of raygen and film
+    uint32_t tail_paths = 1u << 16;         // queues shorter than this finish in k_tail; 0: none
 };
 
 int launch_grid(uint32_t work, int block, const LaunchConfig &lc);
 void launch_raygen(cudaStream_t st, const LaunchConfig &lc, const RenderParams &p, const PathBuffers &b, uint32_t pixels,
                    uint32_t paths, uint32_t sample_base, uint32_t trace_path, psy_path_trace *trace);
-void launch_set_counters(cudaStream_t st, uint32_t *counters, uint32_t n);
+void launch_set_counters(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t n);
 void launch_intersect(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, uint32_t max_work);
 void launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                   uint32_t max_work, uint32_t step, uint32_t trace_path, psy_path_trace *trace);
 void launch_shadow(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                    uint32_t max_work, uint32_t step, uint32_t trace_path, psy_path_trace *trace);
-void launch_swap(cudaStream_t st, uint32_t *counters);
-void launch_begin_round(cudaStream_t st, uint32_t *counters, uint32_t *round, BatchItem *items,
+void launch_end_step(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, unsigned long long *stats,
+                     uint32_t step);
+// The remaining steps of a queue below lc.tail_paths.  `b` as step 0 had it.
+void launch_tail(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+                 uint32_t max_work, unsigned long long *stats);
+void launch_tail_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b,
+                       uint32_t max_work, unsigned long long *stats);
+void launch_begin_round(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t *round, BatchItem *items,
                         const uint32_t *plan_rounds, const BatchItem *plan_items, uint32_t *cursor, uint32_t max_items);
-void launch_count_rays(cudaStream_t st, const uint32_t *counters, unsigned long long *stats);
 // Pass readback: `mismatch` (one word, cleared first) is set when a pixel's
 // sample count differs from `expected`; the resolve writes a pass as the
 // film's consumer sees it (kind: 0 Combined, 1 Normal / Albedo, 2 Sample

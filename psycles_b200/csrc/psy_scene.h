@@ -273,6 +273,7 @@ struct PathBuffers {
     uint32_t *queue_out;
     uint32_t *shadow_queue;
     uint32_t *counters;  // [0] in count, [1] out count, [2] shadow count, [3..4] fetch cursors, [kCounterMisses],
+                         // [kCounterTail],
                          // [kCounterWaveGlossy] a batched wavefront's glossy flag
     uint32_t *job;       // batched wavefronts: the job of each path
     // shading-queue sort by material: per-queue-entry bucket, the sorted
@@ -282,6 +283,8 @@ struct PathBuffers {
 
 constexpr uint32_t kSortBuckets = 2048u;
 constexpr uint32_t kCounterMisses = 5u;  // misses at the front of a sorted shading queue
+// 1 + the step from which the queue is k_tail's; 0 before that
+constexpr uint32_t kCounterTail = 6u;
 constexpr uint32_t kCounterWaveGlossy = 8u;
 // sh_path top bit: the shadow ray's path has ended, its contribution goes to rad_final
 constexpr uint32_t kShadowFinal = 0x80000000u;
