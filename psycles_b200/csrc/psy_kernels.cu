@@ -220,6 +220,9 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 #ifndef PSY_TAIL_MIN_BLOCKS
 #define PSY_TAIL_MIN_BLOCKS 3
 #endif
+#ifndef PSY_PICK_MIN_BLOCKS
+#define PSY_PICK_MIN_BLOCKS 8
+#endif
 #ifndef PSY_MISS_MIN_BLOCKS
 #define PSY_MISS_MIN_BLOCKS 8
 #endif
@@ -717,6 +720,78 @@ __global__ void __launch_bounds__(128, PSY_MISS_MIN_BLOCKS)
     }
 }
 
+// continuation_probability (cycles_path_state.h:413-447).
+__device__ __forceinline__ float continuation_probability(const PathState &ps, const RenderParams &p, f3 throughput) {
+    const bool tr_state = (ps.flag & kFlagTransparent) != 0u;
+    const bool before_min = tr_state ? ps.transparent_bounce <= p.transparent_min : ps.bounce <= p.minimum;
+    return before_min ? 1.0f : minf_(sqrtf(max_abs_component(throughput)), 1.0f);
+}
+
+// light_tree.forward_pdf (src/luisa/path_tracer_light_tree.cpp:799-838) of a hit
+// emissive triangle, seen from the previous scatter (its normal `mn`).
+__device__ __forceinline__ float tree_forward_pdf(const SceneView &s, const SurfacePoint &sp, f3 origin, float4 mn,
+                                                  uint32_t flag) {
+    return lt_pdf(s, lt_triangle_emitter(s, sp.object, sp.cycles_prim), origin, mk3(mn.x, mn.y, mn.z),
+                  (flag & kFlagMisHadTransmission) != 0u);
+}
+
+// The light tree's work of a shading step, ahead of k_shade: each hit path's
+// pick and, where it hit an emitter, the forward pdf, left in the unused words
+// of its hit sector.  A descent evaluates about thirty importances; inside
+// k_shade it ran at that kernel's 4 blocks an SM and evicted its code.
+template <bool kMulti>
+__global__ void __launch_bounds__(128, PSY_PICK_MIN_BLOCKS)
+    k_light_pick(const __grid_constant__ SceneView s_arg, const __grid_constant__ RenderParams p_arg,
+                 const __grid_constant__ PathBuffers b, const JobGpu *jobs, uint32_t sort_threshold) {
+    if (b.counters[kCounterTail] != 0u || (kMulti && b.counters[kCounterWaveTree] == 0u)) return;
+    const uint32_t count = b.counters[0];
+    const bool sorted = sort_threshold != 0u && count >= sort_threshold;
+    const uint32_t *queue = sorted ? b.queue_sorted : b.queue_in;
+    const uint32_t begin = sorted ? b.counters[kCounterMisses] : 0u;
+    for (uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        const uint32_t i = queue[q];
+        const uint32_t job = kMulti ? b.job[i] : 0u;
+        const SceneView &s = kMulti ? jobs[job].s : s_arg;
+        const RenderParams &p = kMulti ? jobs[job].p : p_arg;
+        float4 h4, ro, rd;
+        uint4 hp4, st, st2;
+        load_pair(b.hit, i, h4, hp4);
+        if (hp4.x == kInvalid || !p.use_light_tree || !p.nee) continue;
+        load_pair(b.ray_o, i, ro, rd);
+        load_pair(b.st, i, st, st2);
+        const PathState ps = unpack_state(st, st2);
+        const Hit h{h4.x, h4.y, h4.z, __float_as_uint(h4.w), hp4.x, __float_as_uint(h4.w)};
+        const SurfacePoint sp = surface_point(s, h, mk3(rd.x, rd.y, rd.z));
+        const BakedMaterialGpu mat = s.baked[sp.material];
+        float forward = 0.0f;
+        if (s.triangle_emitters > 0u && mat.emission_sampling != 0u && mat.has_emission)
+            forward = tree_forward_pdf(s, sp, mk3(ro.x, ro.y, ro.z), b.mis_n[i], ps.flag);
+        // paths that end here, or have nothing to evaluate a light with, pick
+        // none (a lamp event on the way may still change a transparent
+        // path's continuation)
+        bool pick = (mat.runtime & kRuntimeBsdfHasEval) != 0u && (st2.x & kSt2TermNext) == 0u;
+        const uint32_t x = p.win_x + st2.w % p.win_w, y = p.win_y + st2.w / p.win_w;
+        const uint32_t rng_hash = pixel_hash(x, p.full_h - 1u - y, p.seed);
+        const uint32_t sample = b.sample[i];
+        if (pick && (s.lamp_count == 0u || (ps.flag & kFlagTransparent) == 0u)) {
+            const float4 tp = b.tp[i];
+            const float cp = continuation_probability(ps, p, mk3(tp.x, tp.y, tp.z));
+            pick = !(cp <= 0.0f) && (cp == 1.0f || !(sample_4d(p, sample, rng_hash, ps.rng_offset).x >= cp));
+        }
+        uint32_t entry = kInvalid;
+        float pdf = 0.0f;
+        if (pick) {
+            const DistEntryGpu e = lt_sample(s, sample_4d(p, sample, rng_hash, ps.rng_offset + 1u).z, sp.position, sp.n,
+                                             (mat.runtime & kRuntimeBsdfHasTransmission) != 0u);
+            if (e.kind <= 1u) {
+                entry = e.kind == 0u ? e.index : s.triangle_emitters + e.index;
+                pdf = e.selection_pdf;
+            }
+        }
+        b.hit_prim[i] = make_uint4(hp4.x, entry, __float_as_uint(pdf), __float_as_uint(forward));
+    }
+}
+
 // What shading a path leaves for its queues.
 struct ShadeResult {
     bool keep;    // the path goes on
@@ -731,7 +806,9 @@ struct ShadeResult {
 // and writes path i's record.
 // kTrace selects the variant that records the per-path trace; the render
 // variant carries no trace code.
-template <bool kTrace, bool kGlossy>
+// kPicked: k_light_pick has left the light tree's pick and forward pdf in the
+// path's record.
+template <bool kTrace, bool kGlossy, bool kPicked>
 __device__ __forceinline__ ShadeResult shade_path(const SceneView &s, const RenderParams &p, const PathBuffers &b,
                                                   uint32_t i, uint32_t step, uint32_t trace_path,
                                                   psy_path_trace *trace) {
@@ -826,10 +903,8 @@ __device__ __forceinline__ ShadeResult shade_path(const SceneView &s, const Rend
             float selection_pdf =
                 0.5f * length(cross(sp.wp1 - sp.wp0, sp.wp2 - sp.wp0)) * s.triangle_area_pdf;
             if (p.use_light_tree) {
-                // light_tree.forward_pdf (src/luisa/path_tracer_light_tree.cpp:799-838)
-                const float4 mn = b.mis_n[i];
-                selection_pdf = lt_pdf(s, lt_triangle_emitter(s, sp.object, sp.cycles_prim), ray.o,
-                                       mk3(mn.x, mn.y, mn.z), (ps.flag & kFlagMisHadTransmission) != 0u);
+                if constexpr (kPicked) selection_pdf = __uint_as_float(hp4.w);
+                else selection_pdf = tree_forward_pdf(s, sp, ray.o, b.mis_n[i], ps.flag);
             }
             const float light_pdf = emissive_forward_pdf(selection_pdf, mat.emission_sampling, ray.o,
                                                          sp.position, sp.wp0, sp.wp1, sp.wp2,
@@ -847,10 +922,7 @@ __device__ __forceinline__ ShadeResult shade_path(const SceneView &s, const Rend
             if (ev) ev->terminated = 1u;
         }
         if (alive) {
-            // continuation_probability (cycles_path_state.h:413-447)
-            const bool tr_state = (ps.flag & kFlagTransparent) != 0u;
-            const bool before_min = tr_state ? ps.transparent_bounce <= p.transparent_min : ps.bounce <= p.minimum;
-            const float cp = before_min ? 1.0f : minf_(sqrtf(max_abs_component(throughput)), 1.0f);
+            const float cp = continuation_probability(ps, p, throughput);
             if (ev) ev->continuation_probability = cp;
             if (cp <= 0.0f) {
                 alive = false;
@@ -880,8 +952,14 @@ __device__ __forceinline__ ShadeResult shade_path(const SceneView &s, const Rend
             const uint32_t runtime = mat.runtime | (sp.back_facing ? kRuntimeBackfacing : 0u);
             if (p.use_light_tree) {
                 // light-tree pick after shading (src/luisa/path_kernel_pipeline.cpp:150-159)
-                selected = lt_sample(s, light_sample.z, sp.position, sp.n,
-                                     (runtime & kRuntimeBsdfHasTransmission) != 0u);
+                if constexpr (kPicked) {
+                    if (hp4.y != kInvalid)
+                        selected = {0.0f, __uint_as_float(hp4.z), hp4.y < s.triangle_emitters ? 0u : 1u,
+                                    hp4.y < s.triangle_emitters ? hp4.y : hp4.y - s.triangle_emitters};
+                } else {
+                    selected = lt_sample(s, light_sample.z, sp.position, sp.n,
+                                         (runtime & kRuntimeBsdfHasTransmission) != 0u);
+                }
                 if (ev) {
                     ev->light_kind = selected.kind;
                     ev->light_index = selected.index;
@@ -1082,7 +1160,7 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
             const uint32_t job = kMulti ? b.job[i] : 0u;
             const SceneView &s = kMulti ? jobs[job].s : s_arg;
             const RenderParams &p = kMulti ? jobs[job].p : p_arg;
-            r = shade_path<kTrace, kGlossy>(s, p, b, i, step, trace_path, trace);
+            r = shade_path<kTrace, kGlossy, !kTrace>(s, p, b, i, step, trace_path, trace);
         }
         const uint32_t slot = warp_push(&b.counters[1], r.keep);
         if (r.keep) b.queue_out[slot] = i;
@@ -1392,7 +1470,7 @@ __global__ void __launch_bounds__(128, PSY_TAIL_MIN_BLOCKS)
             ShadeResult r{};
             if (active) {
                 closest_store(best, b, i);
-                r = shade_path<false, kGlossy>(s, p, b, i, step, kInvalid, nullptr);
+                r = shade_path<false, kGlossy, false>(s, p, b, i, step, kInvalid, nullptr);
             }
             if (__any_sync(kFullMask, r.shadow)) {
                 ShadowHits h;
@@ -1514,7 +1592,8 @@ __global__ void k_begin_round(uint32_t *counters, uint32_t *round, BatchItem *it
         round[0] = plan_rounds[4u * w];
         round[1] = plan_rounds[4u * w + 1u];
         round[2] = n;
-        counters[kCounterWaveGlossy] = plan_rounds[4u * w + 3u];
+        counters[kCounterWaveGlossy] = plan_rounds[4u * w + 3u] & 1u;
+        counters[kCounterWaveTree] = plan_rounds[4u * w + 3u] >> 1;
         counters[0] = round[0];
         counters[1] = counters[2] = counters[3] = counters[4] = 0u;
         counters[kCounterTail] = round[0] < tail_paths ? 1u : 0u;
@@ -1687,6 +1766,7 @@ void launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, c
     if (sorts) launch_sort<false>(st, lc, s, p, b, nullptr, max_work);
     const int grid = shade_grid(max_work, lc);
     if (sorts && !trace) k_shade_miss<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
+    if (p.use_light_tree && !trace) k_light_pick<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
     if (trace && s.has_glossy)
         k_shade<true, false, true><<<grid, 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr, lc.sort_threshold);
     else if (trace)
@@ -1760,6 +1840,7 @@ void launch_shade_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *j
     if (sorts) launch_sort<true>(st, lc, SceneView{}, RenderParams{}, b, jobs, max_work);
     const int grid = shade_grid(max_work, lc);
     if (sorts) k_shade_miss<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, jobs, lc.sort_threshold);
+    k_light_pick<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, jobs, lc.sort_threshold);
     k_shade<false, true, false><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, step, kInvalid, nullptr, jobs,
                                                       lc.sort_threshold);
     k_shade<false, true, true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, step, kInvalid, nullptr, jobs,

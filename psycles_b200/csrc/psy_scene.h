@@ -234,8 +234,8 @@ struct RenderParams {
 // The per-path fields every bounce reads and writes share one 128-byte
 // record per path, in four 32-byte sectors: ray origin and direction; the
 // two state words; throughput and radiance; the hit and its primitive
-// (whose sector's other 12 bytes are written as zeros, so the closest-hit
-// kernel writes whole sectors).  The shading kernel takes its paths in
+// (whose sector's other 12 bytes the closest-hit kernel writes as zeros, so
+// that it writes whole sectors, and the light tree's picks use).  The shading kernel takes its paths in
 // material order, and one cache line per path then replaces a sector in
 // each of eight arrays.
 constexpr size_t kPathRecordBytes = 128u;
@@ -261,7 +261,8 @@ struct PathBuffers {
     float4 *aov_a;              // albedo
     float4 *mis_n;              // shading normal of the last non-transparent scatter (light-tree MIS)
     PathField<float4> hit;      // t, u, v, instance bits
-    PathField<uint4> hit_prim;  // x: primitive (kInvalid on a miss); y, z, w: 0
+    PathField<uint4> hit_prim;  // x: primitive (kInvalid on a miss); y, z, w: the light tree's pick (entry of the
+                                // distribution or kInvalid), its pdf, the forward pdf
     float4 *rad_final;          // radiance and transparency of an ended path (the film reads these
                                 // coalesced instead of a 16-byte field of each 128-byte record)
     float4 *sh_o;     // shadow origin, tmax
@@ -286,6 +287,7 @@ constexpr uint32_t kCounterMisses = 5u;  // misses at the front of a sorted shad
 // 1 + the step from which the queue is k_tail's; 0 before that
 constexpr uint32_t kCounterTail = 6u;
 constexpr uint32_t kCounterWaveGlossy = 8u;
+constexpr uint32_t kCounterWaveTree = 9u;  // a job of the batched wavefront uses its light tree
 // sh_path top bit: the shadow ray's path has ended, its contribution goes to rad_final
 constexpr uint32_t kShadowFinal = 0x80000000u;
 

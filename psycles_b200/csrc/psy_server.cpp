@@ -274,9 +274,12 @@ struct psy_server {
                 // oldest job first, the others backfill the capacity it leaves
                 const uint32_t paths = plan_wavefront(plan, 0u, engine.capacity(), items, film);
                 EnginePlan ep;
-                bool glossy = false;
-                for (const Job *j : planned) glossy = glossy || j->scene->view.has_glossy != 0u;
-                ep.add(items, paths, film, engine.max_jobs(), glossy);
+                bool glossy = false, tree = false;
+                for (const Job *j : planned) {
+                    glossy = glossy || j->scene->view.has_glossy != 0u;
+                    tree = tree || j->settings.use_light_tree != 0u;
+                }
+                ep.add(items, paths, film, engine.max_jobs(), glossy, tree);
                 EngineRun run;
                 psy_status r = cudaEventRecord(slot.begin, engine.stream()) == cudaSuccess ? PSY_OK : PSY_ERROR_CUDA;
                 if (r == PSY_OK) r = engine.run(ep, steps, run);

@@ -37,12 +37,12 @@ def test_tail_equals_wavefronts(backend, name, width, height, spp, tree):
     assert (sa.closest_rays, sa.shadow_rays) == (sb.closest_rays, sb.shadow_rays)
 
 
-@pytest.mark.parametrize("capacity", [4000, 70000])
+@pytest.mark.parametrize("capacity", [4000, 100000])
 def test_batched_tail_equals_wavefronts(backend, capacity):
     compiled = [backend.compile_scene(SCENES[n](seed=2)).scene for n in ("small", "glass")]
     work, references = [], []
     for k in range(4):
-        st = scenes.render_settings(61 + 9 * k, 47, max_bounces=4 + k, seed=k)
+        st = scenes.render_settings(61 + 9 * k, 47, max_bounces=4 + k, seed=k, use_light_tree=k // 2)
         ref = backend.create_session(compiled[k % 2], st)
         _abi.check(ref.lib.psy_session_set_profiling(ref.handle, 1))
         assert ref.render_samples(SampleRange(0, 5, 0, 5))
