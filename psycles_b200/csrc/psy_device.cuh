@@ -1061,15 +1061,14 @@ __device__ __noinline__ float oren_nayar_g(float cosine) {
 // `incoming` points to the viewer, `outgoing` to the light, nl = max(n.outgoing, 0).
 // Below the cutoff the intensity is Lambert's nl / pi, which the callers
 // evaluate inline.
-__device__ __noinline__ f3 oren_nayar_intensity(const PhysicalClosure &c, float sigma, f3 n, f3 incoming,
-                                                f3 outgoing, float nl) {
+__device__ __noinline__ f3 oren_nayar_intensity(f3 color, float sigma, f3 n, f3 incoming, f3 outgoing, float nl) {
     const float a = 1.0f / (kPi + sigma * (kPi * 0.5f - 2.0f / 3.0f));
     const float b = sigma * a;
     const float nv = maxf_(dot(n, incoming), 0.0f);
     float t = dot(outgoing, incoming) - nl * nv;
     if (t > 0.0f) t = t / (maxf_(nl, nv) + 1.17549435e-38f);
     const float single_scatter = a + b * t;
-    const f3 albedo = clamp3(c.color, 0.0f, 1.0f);
+    const f3 albedo = clamp3(color, 0.0f, 1.0f);
     const float e_average = a * kPi + ((2.0f * kPi - 5.6f) / 3.0f) * b;
     const float ratio = e_average / (1.0f - e_average);
     const float keep = 1.0f - e_average;
@@ -1087,12 +1086,15 @@ __device__ __noinline__ f3 oren_nayar_intensity(const PhysicalClosure &c, float 
 // shares the closure normal, so the cosine, pdf and bump term are taken
 // once; a glossy closure is evaluated in its corrected normal, and its bump
 // term (which rejects a direction on the wrong side of the smooth surface
-// unless the closure produced it) is its own.  Out of line: the shading
-// kernel calls it for the light sample and for the BSDF sample, and a
-// single copy keeps the kernel's code within the instruction cache.
+// unless the closure produced it) is its own.  The shading kernel evaluates
+// the light sample and the BSDF sample.  With glossy closures it calls one
+// copy for both, which keeps its code within the instruction cache; without
+// them the function is short, and inlined it needs no copies of its
+// arguments in local memory (1080p procedural frame, 64 spp: shading 108.9 ->
+// 101.6 ms).
 template <bool kGlossy>
-__device__ __noinline__ Evaluation evaluate_mixture(const SurfaceClosures<kGlossy> &s, const ClosurePoint &pt,
-                                                    f3 outgoing_raw, uint32_t lobe_mask, int selected) {
+__device__ __forceinline__ Evaluation evaluate_closures(const SurfaceClosures<kGlossy> &s, const ClosurePoint &pt,
+                                                        f3 outgoing_raw, uint32_t lobe_mask, int selected) {
     const f3 outgoing = safe_normalize(outgoing_raw, pt.shading_normal);
     // make_surface_closure_evaluation_directions (surface_closure_evaluation.cpp:61-70)
     const f3 incoming = pt.view;
@@ -1160,7 +1162,7 @@ __device__ __noinline__ Evaluation evaluate_mixture(const SurfaceClosures<kGloss
         const float pdf = pdf_valid ? lambert : 0.0f;
         if (!diffuse_enabled) continue;
         const float sigma = clampf_(c.roughness, 0.0f, 1.0f);
-        const f3 intensity = sigma < 1.0e-5f ? mk3(lambert) : oren_nayar_intensity(c, sigma, n, incoming, outgoing, nl);
+        const f3 intensity = sigma < 1.0e-5f ? mk3(lambert) : oren_nayar_intensity(c.color, sigma, n, incoming, outgoing, nl);
         const f3 value = c.weight * intensity * bump;
         e.f = e.f + value;
         total += c.sample_weight;
@@ -1170,6 +1172,17 @@ __device__ __noinline__ Evaluation evaluate_mixture(const SurfaceClosures<kGloss
     e.pdf = total > 0.0f ? weighted_pdf / maxf_(total, 1.0e-20f) : 0.0f;
     if (!(weighted_pdf > 0.0f)) e.events = 0u;
     return e;
+}
+
+__device__ __noinline__ Evaluation evaluate_glossy(const SurfaceClosures<true> &s, const ClosurePoint &pt, f3 outgoing,
+                                                   uint32_t lobe_mask, int selected) {
+    return evaluate_closures<true>(s, pt, outgoing, lobe_mask, selected);
+}
+template <bool kGlossy>
+__device__ __forceinline__ Evaluation evaluate_mixture(const SurfaceClosures<kGlossy> &s, const ClosurePoint &pt,
+                                                       f3 outgoing, uint32_t lobe_mask, int selected) {
+    if constexpr (kGlossy) return evaluate_glossy(s, pt, outgoing, lobe_mask, selected);
+    else return evaluate_closures<false>(s, pt, outgoing, lobe_mask, selected);
 }
 
 struct SurfaceSample {
