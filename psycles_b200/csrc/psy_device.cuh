@@ -1485,8 +1485,8 @@ __device__ __forceinline__ void traversal_begin(TraversalState &t, const SceneVi
     t.light_prim = light_prim;
 }
 
-// The plane factors of a node axis: byte k of a plane word (0x80 | c) becomes
-// the float 1 + c / 128 with one byte permutation (0x3f, byte, 0, 0).
+// The plane factor of byte k of a plane word: one byte permutation gives the
+// float of bytes (0x3f, byte, 0, 0).
 __device__ __forceinline__ float plane_factor(uint32_t word, int k) {
     return __uint_as_float(__byte_perm(word, 0x3f000000u, 0x7044u | (uint32_t(k) << 8)));
 }

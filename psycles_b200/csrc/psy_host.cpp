@@ -341,10 +341,9 @@ struct WideNode {
 // few 2^-24 of the extent, the coordinates and the ray's own origin and
 // reach.  The margin takes 4e-6 (64 such units) of the first two on either
 // side; the last two are covered as they were for float planes, by the boxes' own
-// padding and the widened far bound.  span is at least 128 / 127 of the
-// padded extent, so cell 127's plane lies past every child.  Boxes that are
-// not finite in float (or whose span would not be) give NaN planes, which
-// the test ignores.
+// padding and the widened far bound.  span is chosen so that the planes of
+// bytes 0 and 255 enclose the padded extent.  Boxes that are not finite in
+// float (or whose span would not be) give NaN planes, which the test ignores.
 psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offset) {
     psy::NodeGpu g{};
     uint32_t *words[6] = {&g.lox, &g.hix, &g.loy, &g.hiy, &g.loz, &g.hiz};
@@ -364,10 +363,10 @@ psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offs
         const double margin = 4e-6 * (hi - lo) + 4e-6 * std::max(std::fabs(lo), std::fabs(hi)) + 1e-30;
         lo -= margin;
         hi += margin;
-        float span = std::nextafter(float((hi - lo) * (128.0 / 127.0)), INFINITY);
+        float span = std::nextafter(float((hi - lo) / (255.0 / 128.0 - 0.5)), INFINITY);
         float base = 0.0f;
         for (int tries = 0; tries < 64; ++tries) {
-            base = std::nextafter(float(lo - double(span)), -INFINITY);
+            base = std::nextafter(float(lo - 0.5 * double(span)), -INFINITY);
             if (double(base) + double(span) * (255.0 / 128.0) >= hi) break;
             span = std::nextafter(span * 1.000001f, INFINITY);
         }
@@ -375,13 +374,16 @@ psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offs
         g.base[a] = base;
         g.span[a] = span;
         for (int k = 0; k < 4; ++k) {
-            double ql = 127.0, qh = 0.0;  // empty
+            double ql = 255.0, qh = 0.0;  // empty
             if (w.link[k] != psy::kInvalidId && std::isfinite(base)) {
-                ql = std::floor((double(w.lo[a][k]) - margin - base) / double(span) * 128.0 - 128.0);
-                qh = std::ceil((double(w.hi[a][k]) + margin - base) / double(span) * 128.0 - 128.0);
+                // the factor f of a plane, and its place among the bytes'
+                // factors (0.5 + b / 256 up to 1, then 1 + (b - 128) / 128)
+                auto place = [](double f) { return f < 1.0 ? f * 256.0 - 128.0 : f * 128.0; };
+                ql = std::floor(place((double(w.lo[a][k]) - margin - base) / double(span)));
+                qh = std::ceil(place((double(w.hi[a][k]) + margin - base) / double(span)));
             }
-            *words[2 * a] |= (0x80u | uint32_t(std::min(std::max(ql, 0.0), 127.0))) << (8 * k);
-            *words[2 * a + 1] |= (0x80u | uint32_t(std::min(std::max(qh, 0.0), 127.0))) << (8 * k);
+            *words[2 * a] |= uint32_t(std::min(std::max(ql, 0.0), 255.0)) << (8 * k);
+            *words[2 * a + 1] |= uint32_t(std::min(std::max(qh, 0.0), 255.0)) << (8 * k);
         }
     }
     return g;

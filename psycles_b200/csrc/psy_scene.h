@@ -46,9 +46,10 @@ constexpr uint32_t kTraversalStackSize = 48u;
 constexpr uint32_t kGgxETableSize = 32u * 32u, kGgxEavgTableSize = 32u;
 
 // Four children of a wide BVH node in two 32-byte sectors, so one ray reads
-// it with two 256-bit loads.  Child k's box is stored as one byte per plane
-// on a grid of 127 cells per axis: byte 0x80 | c stands for the factor
-// f = 1 + c / 128 and the plane base + span * f.  The host rounds the planes
+// it with two 256-bit loads.  Child k's box is stored as one byte per plane:
+// byte b stands for the float of bits 0x3f000000 | b << 16, a factor f of
+// 0.5 + b / 256 below 1 and 1 + (b - 128) / 128 from there on, and for the
+// plane base + span * f.  The host rounds the planes
 // outward, with a margin for the rounding of the slab test (see quantise in
 // psy_host.cpp).  Leaf children come first; their triangles follow one
 // another, so slot k's is the first slot's plus k.
