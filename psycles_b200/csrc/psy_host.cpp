@@ -1220,10 +1220,30 @@ psy_status build_light_tree(psy_scene *sc, bool sync = true) {
                 return (!m.bounds.empty ? psy::kLtFlagBounds : 0u) | (!m.orientation.empty ? psy::kLtFlagOrientation : 0u) |
                        (distant ? psy::kLtFlagDistant : 0u);
             };
+            // returns the bits of half the half extent's length
             auto pack = [](const psy::LtMeasure &m, float4 &a, float4 &b, float4 &c) {
-                a = make_float4(m.bounds.lo[0], m.bounds.lo[1], m.bounds.lo[2], m.energy);
-                b = make_float4(m.bounds.hi[0], m.bounds.hi[1], m.bounds.hi[2], m.orientation.theta_o);
-                c = make_float4(m.orientation.axis[0], m.orientation.axis[1], m.orientation.axis[2], m.orientation.theta_e);
+                float centre[3], extent[3], axis[3];
+                for (int k = 0; k < 3; ++k) {
+                    centre[k] = (m.bounds.lo[k] + m.bounds.hi[k]) * 0.5f;
+                    extent[k] = m.bounds.hi[k] - centre[k];
+                    axis[k] = m.orientation.axis[k];
+                }
+                const float l2 = axis[0] * axis[0] + axis[1] * axis[1] + axis[2] * axis[2];
+                if (l2 > 1.0e-20f) {
+                    const float inverse = 1.0f / std::sqrt(l2);
+                    for (float &v : axis) v = v * inverse;
+                } else {
+                    axis[0] = axis[1] = 0.0f;
+                    axis[2] = 1.0f;
+                }
+                a = make_float4(centre[0], centre[1], centre[2], m.energy);
+                b = make_float4(extent[0], extent[1], extent[2], m.orientation.theta_o);
+                c = make_float4(axis[0], axis[1], axis[2], m.orientation.theta_e);
+                const float r2 = extent[0] * extent[0] + extent[1] * extent[1] + extent[2] * extent[2];
+                const float radius = 0.5f * std::sqrt(r2);
+                uint32_t bits;
+                std::memcpy(&bits, &radius, 4);
+                return bits;
             };
             // the cone's trigonometry, double-rounded as the kernels' own
             auto cone = [](const psy::LtMeasure &m) {
@@ -1235,18 +1255,18 @@ psy_status build_light_tree(psy_scene *sc, bool sync = true) {
             lt_nodes.reserve(tree.nodes.size());
             for (const psy::LtNode &n : tree.nodes) {
                 psy::LtNodeGpu g{};
-                pack(n.measure, g.min_energy, g.max_theta_o, g.axis_theta_e);
+                const uint32_t radius = pack(n.measure, g.centre_energy, g.extent_theta_o, g.axis_theta_e);
                 g.cone = cone(n.measure);
                 g.topology = make_uint4(n.parent, n.left, n.right, n.kind);
-                g.emitters = make_uint4(n.first, n.count, flags(n.measure, n.kind == psy::kLtDistant), 0u);
+                g.emitters = make_uint4(n.first, n.count, flags(n.measure, n.kind == psy::kLtDistant), radius);
                 lt_nodes.push_back(g);
             }
             lt_emitters.reserve(tree.emitters.size());
             for (const psy::LtEmitter &e : tree.emitters) {
                 psy::LtEmitterGpu g{};
-                pack(e.measure, g.min_energy, g.max_theta_o, g.axis_theta_e);
+                const uint32_t radius = pack(e.measure, g.centre_energy, g.extent_theta_o, g.axis_theta_e);
                 g.cone = cone(e.measure);
-                g.identity = make_uint4(e.emitter_id, flags(e.measure, e.distant), 0u, 0u);
+                g.identity = make_uint4(e.emitter_id, flags(e.measure, e.distant), 0u, radius);
                 lt_emitters.push_back(g);
             }
             for (size_t id = 0; id < tree.emitters.size(); ++id)

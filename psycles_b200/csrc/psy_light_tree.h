@@ -70,27 +70,31 @@ LtEmitter lt_triangle_emitter(uint32_t id, const float p0[3], const float p1[3],
 LtEmitter lt_analytic_emitter(uint32_t id, const void *light_desc);
 
 // Device records: 16-byte lanes as the reference packs them
-// (src/luisa/path_tracer_light_tree_scene.cpp:102-128).
+// (src/luisa/path_tracer_light_tree_scene.cpp:102-128), with what the
+// importance bounds derive from the cluster alone computed on the host in
+// the kernels' float expressions: the bounds as centre and half extent, the
+// normalised cone axis, half the half extent's length (`emitters.w` /
+// `identity.w`, float bits).
 constexpr uint32_t kLtFlagOrientation = 1u, kLtFlagBounds = 2u, kLtFlagDistant = 4u;
 
 // `cone` holds the orientation cone's cosines and sine the importance
 // bounds use, computed on the host in double and rounded once:
 // cos(theta_o), sin(theta_o), cos(theta_o + theta_e), cos(theta_e - theta_o).
 struct alignas(16) LtNodeGpu {
-    float4 min_energy;      // bounds min, energy
-    float4 max_theta_o;     // bounds max, theta_o
+    float4 centre_energy;   // bounds centre, energy
+    float4 extent_theta_o;  // bounds half extent, theta_o
     float4 axis_theta_e;    // cone axis, theta_e
     float4 cone;
     uint4 topology;         // parent, left, right, kind
-    uint4 emitters;         // first, count, flags, pad
+    uint4 emitters;         // first, count, flags, radius term
 };
 
 struct alignas(16) LtEmitterGpu {
-    float4 min_energy;
-    float4 max_theta_o;
+    float4 centre_energy;
+    float4 extent_theta_o;
     float4 axis_theta_e;
     float4 cone;
-    uint4 identity;         // distribution index, flags, emitter id, pad
+    uint4 identity;         // distribution index, flags, emitter id, radius term
 };
 
 }  // namespace psy
