@@ -700,12 +700,12 @@ def run_viewports(backend, compiled, count: int = 64, sweep: str = "descent") ->
 
 
 # DRAM bytes per second of device time of the traversal and shading kernels,
-# from one `ncu --set full` capture of each (the third launch of the 4-spp
+# from one ncu capture of each (the third launch of the 4-spp
 # procedural render: DRAM read + write of the launch over its duration).
 # The traffic of a bench launch is this rate times the launch's mean
 # event-timed duration (the procedural workload only).
-NCU_DRAM_GBS = {"intersect": (319.3 + 65.7) / 2.150, "shadow": (109.0 + 13.2) / 1.775,
-                "shade": (713.4 + 424.1) / 1.202}
+NCU_DRAM_GBS = {"intersect": (323.5 + 66.3) / 1.283, "shadow": (111.7 + 13.4) / 0.758,
+                "shade": (424.0 + 231.5) / 0.537}
 
 
 def kernel_profile(args, backend, compiled, settings) -> dict:
