@@ -3,11 +3,15 @@
 // One render batch holds P window pixels x S samples = N paths whose state
 // lives in HBM as structure-of-arrays (PathBuffers).  Per path step:
 //   k_intersect  closest hit of every queued path (two-level BVH)
-//   k_shade      background / emission + forward MIS / roulette / AOV /
-//                NEE sample + BSDF evaluation (writes one shadow ray) /
-//                closure sample + path-state transition; survivors are
-//                compacted into the next queue with warp-aggregated atomics
+//   k_sort_*     long queues grouped by material and lamp kind, misses first
+//   k_shade_miss the sorted queue's misses: lamps, background
+//   k_light_pick light tree: the paths' picks and forward pdfs
+//   k_shade      emission + forward MIS / roulette / AOV / NEE sample + BSDF
+//                evaluation (writes one shadow ray) / closure sample +
+//                path-state transition; survivors are compacted into the
+//                next queue with warp-aggregated atomics
 //   k_shadow     transmittance of the queued shadow rays, adds NEE radiance
+// k_tail takes a queue that has become short through its remaining steps,
 // and after the last step k_film adds each path's sample into the film in
 // sample order.  The kernels reproduce the Psycles Luisa megakernel
 // (src/luisa/path_kernel_pipeline.cpp:73-183) path by path: the queue order
@@ -205,8 +209,8 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 // and by divergence (9 and 7 of 32 lanes).  With 64-byte nodes in two loads
 // and steps taken together (traverse_warp) they are issue-bound; the lower
 // register budgets (64 and 80) give the latency more warps to hide in: 155 and 117 ms at
-// 8 and 5 blocks of 128 an SM, 169 and 134 ms at 6 and 4, 154 at 9 for
-// closest hits.  Together 224 -> 144 ms for closest hits and 185 -> 108 ms for
+// 8 and 5 blocks of 128 an SM, 169 and 134 ms at 6 and 4 (with the refill at 12,
+// closest hits 146 ms at 8, 153 at 7, 155 at 9).  Together 224 -> 144 ms for closest hits and 185 -> 108 ms for
 // shadow rays, and 82 ms (8 blocks; 88 at 6) since they read baked materials.
 #ifndef PSY_REFILL_LANES
 #define PSY_REFILL_LANES 12
