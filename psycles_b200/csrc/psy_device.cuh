@@ -1445,13 +1445,39 @@ __device__ __forceinline__ SlabRay make_slab_ray(f3 o, f3 raw) {
     return r;
 }
 
+constexpr float kInf = __builtin_huge_valf();
+
+// Whether a ray's slabs meet a padded float box within [tmin, tmax], from
+// `near` on.  This test of a triangle's own box, and of its instance's in the
+// world, is part of what a hit is: where the rounding of the Pluecker test
+// exceeds the padding (rays along shared edges, cameras thousands of object sizes
+// away), a triangle whose box the ray misses is not hit.  The boxes of the
+// nodes above it only have to contain it.  The far bound is widened by a
+// relative 2^-20.
+__device__ __forceinline__ bool box_admits(const SlabRay &r, f3 lo, f3 hi, float tmin, float tmax, float &near) {
+    const bool nx = r.d.x < 0.0f, ny = r.d.y < 0.0f, nz = r.d.z < 0.0f;
+    const float x0 = fmaf(nx ? hi.x : lo.x, r.inv.x, -r.oinv.x), x1 = fmaf(nx ? lo.x : hi.x, r.inv.x, -r.oinv.x);
+    const float y0 = fmaf(ny ? hi.y : lo.y, r.inv.y, -r.oinv.y), y1 = fmaf(ny ? lo.y : hi.y, r.inv.y, -r.oinv.y);
+    const float z0 = fmaf(nz ? hi.z : lo.z, r.inv.z, -r.oinv.z), z1 = fmaf(nz ? lo.z : hi.z, r.inv.z, -r.oinv.z);
+    near = fmaxf(fmaxf(x0, y0), fmaxf(z0, tmin));
+    const float far = fminf(fminf(x1, y1), fminf(z1, tmax));
+    return near <= fmaxf(fmaf(far, 1.00000095367431640625f, 1.0e-30f), far);
+}
+
+// A ray's slabs in an instance's object space, from the transform in its entry.
+__device__ __forceinline__ SlabRay entry_slabs(const uint4 &w0, const uint4 &w1, const uint4 &w2, const Ray &ray) {
+    const float4 a = floats4(w0), b = floats4(w1), c = floats4(w2);
+    const Xform w2o{mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), mk3(b.z, b.w, c.x), mk3(c.y, c.z, c.w)};
+    return make_slab_ray(xform_point(w2o, ray.o), xform_direction(w2o, ray.d));
+}
+
 // Two-level traversal of one ray as three steps -- visit a node, test a leaf
 // triangle, enter or leave an instance -- between which the ray's state
 // lives in registers (stack in local memory), so a warp can take the step
 // most of its lanes wait for (traverse_warp).  Every triangle accepted by
 // the Pluecker predicate in [tmin, tmax] (`tmax` shrinks as the visitor
 // requests) that is neither the source nor the light identity is handed to
-// `on_hit(instance, local, cycles_prim, t, u, v)`; a true return ends the
+// `on_hit(instance, local, cycles_prim, slot, t, u, v)`; a true return ends the
 // traversal.
 struct TraversalState {
     Ray ray;      // world ray
@@ -1462,8 +1488,9 @@ struct TraversalState {
     uint32_t leaf_first;
     uint32_t sp, inst, prim_offset;
     uint32_t visibility, src_obj, src_prim, light_obj, light_prim;
-    uint32_t stack[kStackSize];
+    uint32_t stack[kStackSize + 1u];  // the last for the visitor: used too rarely for a register
 };
+constexpr uint32_t kStackVisitor = kStackSize;
 
 __device__ __forceinline__ void traversal_begin(TraversalState &t, const SceneView &s, const Ray &ray,
                                                 uint32_t visibility, uint32_t src_obj, uint32_t src_prim,
@@ -1503,6 +1530,25 @@ __device__ __forceinline__ void fma2(float a, float b, uint64_t m, uint64_t c, f
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
 }
 
+// Sorts four (distance, link) pairs by distance.
+__device__ __forceinline__ void sort_children(float key[4], uint32_t val[4]) {
+#define PSY_CSWAP(i, j)                 \
+    if (key[j] < key[i]) {              \
+        const float tk = key[i];        \
+        key[i] = key[j];                \
+        key[j] = tk;                    \
+        const uint32_t tv = val[i];     \
+        val[i] = val[j];                \
+        val[j] = tv;                    \
+    }
+    PSY_CSWAP(0, 1)
+    PSY_CSWAP(2, 3)
+    PSY_CSWAP(0, 2)
+    PSY_CSWAP(1, 3)
+    PSY_CSWAP(1, 2)
+#undef PSY_CSWAP
+}
+
 // Visits node t.node: tests its four children's boxes, notes the hit leaf
 // triangles in t.leaves and continues with a hit inner child (or instance),
 // pushing the others.  kNearFirst orders them nearest first (closest hit);
@@ -1510,9 +1556,10 @@ __device__ __forceinline__ void fma2(float a, float b, uint64_t m, uint64_t c, f
 // every candidate or stop at the first blocker regardless of order).
 //
 // A plane's distance is one FMA, f * (span / d) + (base - o) / d, from
-// per-axis products of the node's span and base.  The boxes' margin covers
-// its rounding; the far bound is widened by a relative 2^-20 for the
-// approximate reciprocal.  A NaN plane (a non-finite box) constrains nothing.
+// per-axis products of the node's span and base.  The boxes' margin and the
+// far bound, widened by a relative 2^-18 (box_admits: 2^-20), cover its
+// rounding, so no box that box_admits would accept is missed.  A NaN plane (a
+// non-finite box) constrains nothing.
 template <bool kNearFirst>
 __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s) {
     uint4 w0, w1, w2, w3;
@@ -1548,7 +1595,7 @@ __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s
     for (int k = 0; k < 4; ++k) {
         const float nr = fmaxf(fmaxf(tnx[k], tny[k]), fmaxf(tnz[k], t.ray.tmin));
         const float fr = fminf(fminf(tfx[k], tfy[k]), fminf(tfz[k], t.tmax));
-        const bool in = nr <= fmaf(fr, 1.00000095367431640625f, 1.0e-30f);
+        const bool in = nr <= fmaf(fr, 1.0000038146972656f, 1.0e-30f);
         near[k] = nr;
         hit[k] = in && int(lk[k]) >= 0;
         // a leaf link is below kInvalidId (-1), an empty slot's
@@ -1568,7 +1615,6 @@ __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s
         t.node = next;
     } else {
         // sort the four (distance, link) pairs, misses last
-        const float kInf = __int_as_float(0x7f800000);
         float key[4];
         uint32_t val[4];
 #pragma unroll
@@ -1576,21 +1622,7 @@ __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s
             key[k] = hit[k] ? near[k] : kInf;
             val[k] = lk[k];
         }
-#define PSY_CSWAP(i, j)                 \
-    if (key[j] < key[i]) {              \
-        const float tk = key[i];        \
-        key[i] = key[j];                \
-        key[j] = tk;                    \
-        const uint32_t tv = val[i];     \
-        val[i] = val[j];                \
-        val[j] = tv;                    \
-    }
-        PSY_CSWAP(0, 1)
-        PSY_CSWAP(2, 3)
-        PSY_CSWAP(0, 2)
-        PSY_CSWAP(1, 3)
-        PSY_CSWAP(1, 2)
-#undef PSY_CSWAP
+        sort_children(key, val);
         if (key[0] == kInf) {
             t.node = t.stack[--t.sp];
         } else {
@@ -1602,12 +1634,30 @@ __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s
     }
 }
 
-// Tests the next noted leaf triangle.
-template <typename OnHit>
+// A ray that starts within the instance's reach meets the instance's box
+// wherever it meets a triangle's in it (instance_reach in psy_host.cpp).
+__device__ __forceinline__ bool within_reach(const Ray &ray, uint32_t visibility_reach) {
+    return fmaxf(fabsf(ray.o.x), fmaxf(fabsf(ray.o.y), fabsf(ray.o.z))) <
+           __uint_as_float(visibility_reach & 0xffff0000u);
+}
+
+__device__ __forceinline__ bool instance_admits(const SceneView &s, uint32_t instance, const SlabRay &world, float tmin,
+                                                float tmax, float &near) {
+    uint4 w0, w1;
+    load_sector_nc(s.instance_boxes + instance, w0, w1);
+    const float4 p = floats4(w0), q = floats4(w1);
+    return box_admits(world, mk3(p.x, p.y, p.z), mk3(p.w, q.x, q.y), tmin, tmax, near);
+}
+
+// Tests the next noted leaf triangle.  A closest hit's boxes are looked at when
+// it is final (closest_ambiguous in psy_kernels.cu), an any-hit ray's here and as
+// it enters an instance.
+template <bool kNearFirst, typename OnHit>
 __device__ __forceinline__ void test_leaf(TraversalState &t, const SceneView &s, OnHit on_hit) {
     const uint32_t k = uint32_t(__ffs(int(t.leaves)) - 1);
     t.leaves &= t.leaves - 1u;
-    const TriGpu *tp = s.tris + (t.leaf_first + k);
+    const uint32_t slot = t.leaf_first + k;
+    const TriGpu *tp = s.tris + slot;
     uint4 ua, ub;
     load_sector_nc(tp, ua, ub);
     const float4 a = floats4(ua), b = floats4(ub), c = __ldg(&tp->v2);
@@ -1616,7 +1666,12 @@ __device__ __forceinline__ void test_leaf(TraversalState &t, const SceneView &s,
     if ((t.src_obj == t.inst && t.src_prim == cp) || (t.light_obj == t.inst && t.light_prim == cp)) return;
     float th, u, v;
     if (!intersect_triangle(t.cur.o, t.cur.d, t.ray.tmin, t.tmax, ld3(a), ld3(b), ld3(c), th, u, v)) return;
-    if (on_hit(t.inst, local, cp, th, u, v)) {
+    if constexpr (!kNearFirst) {
+        const float4 e = __ldg(&tp->lo_z_hi);
+        float near;
+        if (!box_admits(t.cur, mk3(b.w, c.w, e.x), mk3(e.y, e.z, e.w), t.ray.tmin, t.tmax, near)) return;
+    }
+    if (on_hit(t.inst, local, cp, slot, th, u, v)) {
         t.node = kLinkDone;
         t.leaves = 0u;
     }
@@ -1625,6 +1680,7 @@ __device__ __forceinline__ void test_leaf(TraversalState &t, const SceneView &s,
 // Takes the instance or kLinkLeave entry in t.node: leaving an instance
 // continues with the next entry of the instance tree, and only a node of it
 // needs the world ray's slabs back -- the next instance replaces them.
+template <bool kNearFirst>
 __device__ __forceinline__ void cross_instance(TraversalState &t, const SceneView &s) {
     uint32_t e = t.node;
     const bool left = e == kLinkLeave;
@@ -1638,10 +1694,14 @@ __device__ __forceinline__ void cross_instance(TraversalState &t, const SceneVie
         const EntryGpu *ep = s.entries + i;
         load_sector_nc(ep, w0, w1);
         load_sector_nc(ep->w2o + 8, w2, w3);
-        if ((w3.z & t.visibility) != 0u) {
-            const float4 a = floats4(w0), b = floats4(w1), c = floats4(w2);
-            const Xform w2o{mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y), mk3(b.z, b.w, c.x), mk3(c.y, c.z, c.w)};
-            t.cur = make_slab_ray(xform_point(w2o, t.ray.o), xform_direction(w2o, t.ray.d));
+        bool enters = (w3.z & t.visibility) != 0u;
+        if (!kNearFirst && !within_reach(t.ray, w3.z)) {
+            float near;
+            t.cur = make_slab_ray(t.ray.o, t.ray.d);
+            enters = enters && instance_admits(s, i, t.cur, t.ray.tmin, t.tmax, near) && near <= t.tmax;
+        }
+        if (enters) {
+            t.cur = entry_slabs(w0, w1, w2, t.ray);
             t.inst = i;
             t.prim_offset = w3.y;
             stack_push(t.stack, t.sp, kLinkLeave);
@@ -1677,9 +1737,9 @@ __device__ __forceinline__ void traverse_warp(TraversalState &t, const SceneView
         if (nn >= 2 * nl && nn >= 2 * nc) {
             if (node) visit_node<kNearFirst>(t, s);
         } else if (nl >= nc) {
-            if (leaf) test_leaf(t, s, on_hit);
+            if (leaf) test_leaf<kNearFirst>(t, s, on_hit);
         } else {
-            if (cross) cross_instance(t, s);
+            if (cross) cross_instance<kNearFirst>(t, s);
         }
     }
 }

@@ -72,7 +72,7 @@ psy_status PathArena::ensure(uint32_t n, bool with_job) {
     PSY_CUDA_TRY(sh_path.alloc(u1));
     PSY_CUDA_TRY(qa.alloc(u1));
     PSY_CUDA_TRY(qb.alloc(u1));
-    PSY_CUDA_TRY(sq.alloc(u1));
+    PSY_CUDA_TRY(ambiguous.alloc(u1));
     if (with_job) PSY_CUDA_TRY(job.alloc(u1));
     PSY_CUDA_TRY(sort_keys.alloc(u1));
     PSY_CUDA_TRY(queue_sorted.alloc(u1));
@@ -97,7 +97,7 @@ psy_status PathArena::ensure(uint32_t n, bool with_job) {
     b.sh_path = sh_path.as<uint32_t>();
     b.queue_in = qa.as<uint32_t>();
     b.queue_out = qb.as<uint32_t>();
-    b.shadow_queue = sq.as<uint32_t>();
+    b.ambiguous = ambiguous.as<uint32_t>();
     b.counters = counters.as<uint32_t>();
     b.job = job.ptr ? job.as<uint32_t>() : nullptr;
     b.sort_keys = sort_keys.as<uint32_t>();
@@ -327,11 +327,51 @@ void padded(const Box &b, float lo[3], float hi[3]) {
 #define PSY_SAH_AXES 3
 #endif
 
+// How far from the world's origin (largest coordinate) rays may start for which
+// a triangle's own box says all about its instance's: a ray that meets the
+// triangle's padded box in object space then meets the instance's in the
+// world, and no later.  Both tests round: the far bounds' widening comes to
+// 2^-20 of the distance from the ray's origin, products, sums and the
+// approximate reciprocal to a few 2^-23 of the coordinates, those of the object
+// space scaled by its transform.  What the instance's padding exceeds the
+// triangles' by covers twice these; where it does not (an instance flat
+// on an axis at coordinate 0 is not padded there) no distance is small enough.
+float instance_reach(const psy::BoxGpu &world, const Box &mesh, const M34 &o2w, const float *w2o) {
+    if (mesh.empty()) return 0.0f;
+    const float to_world[9] = {o2w.c0.x, o2w.c0.y, o2w.c0.z, o2w.c1.x, o2w.c1.y, o2w.c1.z, o2w.c2.x, o2w.c2.y, o2w.c2.z};
+    double mesh_pad = 0.0, mesh_coordinate = 0.0, scale = 0.0, inverse = 0.0, offset = 0.0;
+    for (int a = 0; a < 3; ++a) {
+        const double c = std::max(std::fabs(mesh.lo[a]), std::fabs(mesh.hi[a]));
+        mesh_pad = std::max(mesh_pad, 1e-5 * (mesh.hi[a] - mesh.lo[a]) + 1e-6 * c);
+        mesh_coordinate = std::max(mesh_coordinate, c);
+        double row = 0.0, inverse_row = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            row += std::fabs(double(to_world[3 * k + a]));
+            inverse_row += std::fabs(double(w2o[3 * k + a]));
+        }
+        scale = std::max(scale, row);
+        inverse = std::max(inverse, inverse_row);
+        offset = std::max(offset, std::fabs(double(w2o[9 + a])));
+    }
+    double pad = 1e300, coordinate = 0.0;
+    for (int a = 0; a < 3; ++a) {
+        // the padding is 1e-4 of the extent and 1e-5 of the coordinate, or little more
+        const double lo = world.lo[a], hi = world.hi[a], c = std::max(std::fabs(lo), std::fabs(hi));
+        pad = std::min(pad, 0.99 * (1e-4 * (hi - lo) / 1.0003 + 1e-5 * std::max(0.0, c - 1.1e-4 * (hi - lo))));
+        coordinate = std::max(coordinate, c);
+    }
+    constexpr double kWiden = 1.0 / (1 << 19), kRound = 1.0 / (1 << 20);
+    const double slack = pad - scale * mesh_pad - kWiden * coordinate - kRound * scale * (mesh_coordinate + offset);
+    const double reach = slack / (kWiden + kRound * (1.0 + scale * inverse));
+    return reach > 0.0 && std::isfinite(reach) ? float(std::min(reach, 1e30)) : 0.0f;
+}
+
 // A 4-wide node as built: child boxes in float, links as the traversal takes
 // them (node indices and leaf triangles relative to the tree).
 struct WideNode {
     float lo[3][4], hi[3][4];
     uint32_t link[4] = {psy::kInvalidId, psy::kInvalidId, psy::kInvalidId, psy::kInvalidId};
+    uint32_t slot[4];  // each child's place before leaves were put first
 };
 
 // The device form of a wide node: its children's boxes on the node's byte
@@ -681,21 +721,22 @@ struct Builder {
         // leaves (of triangles) first, then inner children and instances;
         // empty slots keep kInvalidId
         int k = 0;
-        auto put = [&](const WideChild &c, uint32_t link) {
+        auto put = [&](int slot, uint32_t link) {
             for (int a = 0; a < 3; ++a) {
-                w.lo[a][k] = c.lo[a];
-                w.hi[a][k] = c.hi[a];
+                w.lo[a][k] = kids[slot].lo[a];
+                w.hi[a][k] = kids[slot].hi[a];
             }
+            w.slot[k] = uint32_t(slot);
             w.link[k++] = link;
         };
         for (int c = 0; c < n; ++c) {
             if (leaf_is_id || kids[c].link >= 0 || kids[c].count == 0) continue;
-            put(kids[c], psy::kLinkLeaf | uint32_t(order.size()));
+            put(c, psy::kLinkLeaf | uint32_t(order.size()));
             order.push_back(uint32_t(~kids[c].link));
         }
         for (int c = 0; c < n; ++c) {
-            if (kids[c].link >= 0) put(kids[c], uint32_t(collapse(kids[c].link, wide, order)));
-            else if (leaf_is_id && kids[c].count > 0) put(kids[c], psy::kLinkInstance | uint32_t(~kids[c].link));
+            if (kids[c].link >= 0) put(c, uint32_t(collapse(kids[c].link, wide, order)));
+            else if (leaf_is_id && kids[c].count > 0) put(c, psy::kLinkInstance | uint32_t(~kids[c].link));
         }
         wide[size_t(index)] = w;
         return index;
@@ -1573,6 +1614,8 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
 
     // ---- instances + TLAS
     std::vector<psy::InstanceGpu> instances(d->instance_count);
+    std::vector<psy::EntryGpu> entries(d->instance_count);
+    std::vector<psy::BoxGpu> world_boxes(d->instance_count);
     Builder tl;
     tl.leaf_is_id = true;
     std::vector<M34> o2w(d->instance_count);
@@ -1628,6 +1671,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
                 p.box.hi[a] += pad;
                 p.c[a] = 0.5 * (p.box.lo[a] + p.box.hi[a]);
             }
+            padded(p.box, world_boxes[i].lo, world_boxes[i].hi);
             p.id = i;
             tl.prims.push_back(p);
         }
@@ -1717,6 +1761,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     }
     // the device nodes, in parallel over chunks of each tree
     nodes.resize(node_count);
+    std::vector<psy::BoxGpu> node_boxes(node_count);
     {
         constexpr size_t kNodeChunk = 1024u;
         struct NodeJob {
@@ -1732,8 +1777,19 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         const psy_status quantised = parallel_for(uint32_t(node_jobs.size()), nullptr, [&](uint32_t job) {
             const NodeJob &j = node_jobs[job];
             const size_t end = std::min(j.wide->size(), j.first + kNodeChunk);
-            for (size_t k = j.first; k < end; ++k)
-                nodes[j.node_offset + k] = quantise((*j.wide)[k], j.node_offset, j.tri_offset);
+            for (size_t k = j.first; k < end; ++k) {
+                const WideNode &w = (*j.wide)[k];
+                nodes[j.node_offset + k] = quantise(w, j.node_offset, j.tri_offset);
+                for (int c = 0; c < 4; ++c) {
+                    if (w.link[c] >= psy::kLinkInstance) continue;
+                    psy::BoxGpu &b = node_boxes[j.node_offset + w.link[c]];
+                    for (int a = 0; a < 3; ++a) {
+                        b.lo[a] = w.lo[a][c];
+                        b.hi[a] = w.hi[a][c];
+                    }
+                    b.slot = w.slot[c];
+                }
+            }
         });
         if (quantised != PSY_OK) return quantised;
     }
@@ -1750,14 +1806,17 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         for (uint32_t i = 0; i < d->material_count; ++i) tagged[i] = tagged_material(i);
         for (uint32_t &m : tri_materials) m = tagged[m];
     }
-    std::vector<psy::EntryGpu> entries(d->instance_count);
     for (uint32_t i = 0; i < d->instance_count; ++i) {
         const psy::MeshGpu &mesh = meshes[instances[i].mesh];
         psy::EntryGpu &e = entries[i];
         std::copy(std::begin(instances[i].w2o), std::end(instances[i].w2o), e.w2o);
         e.root = node_offsets[instances[i].mesh];
         e.prim_offset = instances[i].prim_offset = mesh.tri_offset;
-        e.visibility = instances[i].visibility;
+        e.visibility_reach = instances[i].visibility & 0xffffu;
+        const float reach = instance_reach(world_boxes[i], mesh_boxes[instances[i].mesh], o2w[i], instances[i].w2o);
+        uint32_t bits;
+        std::memcpy(&bits, &reach, 4);
+        e.visibility_reach |= bits & 0xffff0000u;
         e.material = instances[i].material =
             mesh.material_offset != psy::kInvalidId ? psy::kInvalidId : tagged_material(d->instances[i].material);
         instances[i].smooth = mesh.smooth;
@@ -1942,11 +2001,13 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     // device pool: a later compile reuses the memory a destroyed scene gave
     // back, and parameter blocks replaced by edits are retired without
     // waiting on the device.
-    for (DeviceBuffer *b : {&sc->nodes, &sc->entries, &sc->tris, &sc->shade_tris, &sc->instances, &sc->material_buf, &sc->baked, &sc->closures, &sc->code, &sc->value_buf, &sc->scalar_buf,
+    for (DeviceBuffer *b : {&sc->nodes, &sc->node_boxes, &sc->instance_boxes, &sc->entries, &sc->tris, &sc->shade_tris, &sc->instances, &sc->material_buf, &sc->baked, &sc->closures, &sc->code, &sc->value_buf, &sc->scalar_buf,
                             &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights, &sc->lamp_consts,
                             &sc->lamp_bounds, &sc->lamp_ids})
         b->ordered = st;
     PSY_CUDA_TRY(sc->nodes.upload(nodes, st));
+    PSY_CUDA_TRY(sc->node_boxes.upload(node_boxes, st));
+    PSY_CUDA_TRY(sc->instance_boxes.upload(world_boxes, st));
     PSY_CUDA_TRY(sc->entries.upload(entries, st));
     PSY_CUDA_TRY(sc->instances.upload(instances, st));
     // the triangle records are packed on the device; the vertex arrays go
@@ -2007,13 +2068,15 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
     PSY_CUDA_TRY(sc->lamp_ids.upload(lamp_ids, st));
     PSY_CUDA_TRY(cudaStreamSynchronize(st));
     sc->stats.upload_bytes = 0u;
-    for (const DeviceBuffer *b : {&sc->nodes, &sc->entries, &mesh_records, &positions_buf, &normals_buf, &indices_buf,
+    for (const DeviceBuffer *b : {&sc->nodes, &sc->node_boxes, &sc->instance_boxes, &sc->entries, &mesh_records, &positions_buf, &normals_buf, &indices_buf,
                                   &tri_materials_buf, &order_buf, &sc->instances, &sc->material_buf, &sc->baked, &sc->closures, &sc->code,
                                   &sc->value_buf, &sc->scalar_buf, &sc->vector_buf, &sc->emitters, &sc->distribution, &sc->ggx_tables, &sc->lights,
                                   &sc->lamp_consts, &sc->lamp_bounds, &sc->lamp_ids})
         sc->stats.upload_bytes += b->bytes;
     psy::SceneView &v = sc->view;
     v.nodes = sc->nodes.as<psy::NodeGpu>();
+    v.node_boxes = sc->node_boxes.as<psy::BoxGpu>();
+    v.instance_boxes = sc->instance_boxes.as<psy::BoxGpu>();
     v.entries = sc->entries.as<psy::EntryGpu>();
     v.tris = sc->tris.as<psy::TriGpu>();
     v.instances = sc->instances.as<psy::InstanceGpu>();
@@ -2238,7 +2301,7 @@ psy_status psy_session_read_trace(psy_session *s, psy_path_trace *out) {
 
 uint64_t psy::host::scene_device_bytes(const psy_scene *s) {
     uint64_t n = 0u;
-    for (const DeviceBuffer *b : {&s->nodes, &s->entries, &s->tris, &s->shade_tris, &s->instances, &s->material_buf, &s->baked, &s->closures, &s->code, &s->value_buf, &s->scalar_buf,
+    for (const DeviceBuffer *b : {&s->nodes, &s->node_boxes, &s->instance_boxes, &s->entries, &s->tris, &s->shade_tris, &s->instances, &s->material_buf, &s->baked, &s->closures, &s->code, &s->value_buf, &s->scalar_buf,
                                   &s->vector_buf, &s->emitters, &s->distribution, &s->ggx_tables, &s->lights, &s->lamp_consts, &s->lamp_bounds,
                                   &s->lamp_ids, &s->lt_nodes, &s->lt_emitters, &s->lt_mapping, &s->lt_lookup})
         n += b->bytes;
@@ -2462,7 +2525,7 @@ psy_status psy_session_render_samples_static(psy_session *s, uint32_t first, uin
     b.sh_path = reinterpret_cast<uint32_t *>(carve(4 * n));
     b.queue_in = reinterpret_cast<uint32_t *>(carve(4 * n));
     b.queue_out = reinterpret_cast<uint32_t *>(carve(4 * n));
-    b.shadow_queue = reinterpret_cast<uint32_t *>(carve(4 * n));
+    b.ambiguous = reinterpret_cast<uint32_t *>(carve(4 * n));
     b.counters = reinterpret_cast<uint32_t *>(carve(64));
     if (cursor > static_cast<unsigned char *>(base) + psy::kStaticPathBytes)
         return fail(PSY_ERROR_STATE, "static path state larger than its array");

@@ -109,7 +109,7 @@ struct DeviceBuffer {
 // for batched wavefronts.
 struct PathArena {
     uint32_t capacity = 0;
-    DeviceBuffer records, rad_final, sample, aov_n, aov_a, mis_n, sh_o, sh_d, sh_c, sh_ids, sh_path, qa, qb, sq, job,
+    DeviceBuffer records, rad_final, sample, aov_n, aov_a, mis_n, sh_o, sh_d, sh_c, sh_ids, sh_path, qa, qb, ambiguous, job,
         sort_keys,
         queue_sorted, sort_hist, counters, stats;
     PathBuffers view{};
@@ -157,7 +157,7 @@ struct psy_scene {
     psy_camera_desc camera{};
     std::vector<psy::MaterialGpu> materials;
     std::vector<float> scalars, vectors;
-    psy::host::DeviceBuffer nodes, entries, tris, shade_tris, instances, material_buf, baked, closures, code,
+    psy::host::DeviceBuffer nodes, node_boxes, instance_boxes, entries, tris, shade_tris, instances, material_buf, baked, closures, code,
         value_buf, scalar_buf, vector_buf, emitters, distribution, ggx_tables, lights, lamp_consts, lamp_bounds, lamp_ids, lt_nodes, lt_emitters,
         lt_mapping, lt_lookup;
     psy::SceneView view{};

@@ -207,16 +207,15 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 // Both traversal kernels were bound by L1 wavefronts (72 % of peak for closest
 // hits: a 128-byte node in eight 16-byte loads, each a wavefront per lane)
 // and by divergence (9 and 7 of 32 lanes).  With 64-byte nodes in two loads
-// and steps taken together (traverse_warp) they are issue-bound; the lower
-// register budgets (64 and 80) give the latency more warps to hide in: 155 and 117 ms at
-// 8 and 5 blocks of 128 an SM, 169 and 134 ms at 6 and 4 (with the refill at 12,
-// closest hits 146 ms at 8, 153 at 7, 155 at 9).  Together 224 -> 144 ms for closest hits and 185 -> 108 ms for
-// shadow rays, and 82 ms (8 blocks; 88 at 6) since they read baked materials.
+// and steps taken together (traverse_warp) they are issue-bound, and the lower
+// register budgets give the latency more warps to hide in.  1080p procedural
+// frame, 64 spp: closest hits 224 -> 151 ms at 7 blocks of 128 an SM (8, where
+// closest_ambiguous spills: 156), shadow rays 185 -> 78 ms at 8.
 #ifndef PSY_REFILL_LANES
 #define PSY_REFILL_LANES 12
 #endif
 #ifndef PSY_INTERSECT_MIN_BLOCKS
-#define PSY_INTERSECT_MIN_BLOCKS 8
+#define PSY_INTERSECT_MIN_BLOCKS 7
 #endif
 #ifndef PSY_SHADE_MIN_BLOCKS
 #define PSY_SHADE_MIN_BLOCKS 4
@@ -258,7 +257,8 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *fetch_counter, uint32_t
 // A path's closest hit so far.
 struct ClosestHit {
     float t, u, v;
-    uint32_t instance, prim;  // kInvalid: none yet
+    uint32_t instance;  // kInvalid: none yet
+    uint32_t slot;      // its triangle's place in SceneView::tris
 };
 
 __device__ __forceinline__ void closest_begin(ClosestHit &best, TraversalState &t, const SceneView &s,
@@ -271,22 +271,159 @@ __device__ __forceinline__ void closest_begin(ClosestHit &best, TraversalState &
     traversal_begin(t, s, ray, contract_visibility(st.y), st2.y, st2.z, kInvalid, kInvalid);
     best.t = ray.tmax;
     best.u = best.v = 0.0f;
-    best.instance = best.prim = kInvalid;
+    best.instance = best.slot = kInvalid;
 }
 
-__device__ __forceinline__ bool closest_hit(ClosestHit &best, TraversalState &t, uint32_t instance, uint32_t prim,
-                                            float th, float u, float v) {
-    // equal distances go to the greatest (object, primitive)
-    const bool later = instance > best.instance || (instance == best.instance && prim > best.prim);
-    if (best.instance != kInvalid && !(th < best.t || (th == best.t && later))) return false;
-    best = {th, u, v, instance, prim};
-    t.tmax = th;
+// Equal distances go to the greatest (object, primitive).  t.stack[kStackVisitor]
+// is the distance of the next hit behind the closest; to see one that lies within
+// rounding, hits a little behind it are looked at too.
+__device__ __forceinline__ bool closest_hit(ClosestHit &best, TraversalState &t, const SceneView &s, uint32_t instance,
+                                            uint32_t prim, uint32_t slot, float th, float u, float v) {
+    if (best.instance != kInvalid && !(th < best.t)) {
+        const bool wins = th == best.t && (instance > best.instance ||
+                                           (instance == best.instance &&
+                                            prim > __float_as_uint(__ldg(&s.tris[best.slot].v0.w))));
+        if (!wins) {
+            t.stack[kStackVisitor] = __float_as_uint(fminf(__uint_as_float(t.stack[kStackVisitor]), th));
+            return false;
+        }
+    }
+    t.stack[kStackVisitor] = __float_as_uint(best.t);
+    best = {th, u, v, instance, slot};
+    t.tmax = fmaf(th, 1.00000095367431640625f, 1.0e-30f);
     return false;
 }
 
-__device__ __forceinline__ void closest_store(const ClosestHit &best, const PathBuffers &b, uint32_t path) {
+// Whether the closest hit of a finished ray depends on the order of visits, or is
+// none.  A subtree is culled if the ray enters its box behind the closest hit so
+// far; where rounding puts a triangle's hit before its box, that can happen to
+// the closest one if another hit lies between the two.  `prim`: its primitive.
+__device__ __forceinline__ bool closest_ambiguous(const ClosestHit &best, const TraversalState &t, const SceneView &s,
+                                                  uint32_t &prim) {
+    prim = kInvalid;
+    if (best.instance == kInvalid) return false;
+    uint4 w0, w1, w2, w3, ua, ub, uc, ud;
+    const EntryGpu *ep = s.entries + best.instance;
+    load_sector_nc(ep, w0, w1);
+    load_sector_nc(ep->w2o + 8, w2, w3);
+    const TriGpu *tp = s.tris + best.slot;
+    load_sector_nc(tp, ua, ub);
+    load_sector_nc(&tp->v2, uc, ud);
+    prim = ua.w;
+    const float4 e = floats4(ud);
+    float near;
+    if (!box_admits(entry_slabs(w0, w1, w2, t.ray), mk3(__uint_as_float(ub.w), __uint_as_float(uc.w), e.x),
+                    mk3(e.y, e.z, e.w), t.ray.tmin, kInf, near))
+        return true;
+    if (!within_reach(t.ray, w3.z)) {
+        float entry;
+        if (!instance_admits(s, best.instance, make_slab_ray(t.ray.o, t.ray.d), t.ray.tmin, kInf, entry)) return true;
+        near = fmaxf(near, entry);
+    }
+    return __uint_as_float(t.stack[kStackVisitor]) < near || t.tmax < near;
+}
+
+// The closest hit of an ambiguous ray, for which the order of visits counts:
+// nodes nearest first by their float boxes, a node's triangles before its
+// other children, these only if the ray enters them before the closest hit so
+// far.  This order, which defines the renderer's results, is the one of
+// traversing float boxes throughout; the byte boxes give the same hit for all
+// other rays.  (Restated on the CPU, 220 M rays aimed at shared edges from up to
+// 1e4 mesh sizes away: at most 1 % ambiguous, one other hit; ordinary
+// rays are ambiguous about once in 1e7.)
+__device__ __noinline__ ClosestHit closest_exact(const NodeGpu *nodes, const BoxGpu *node_boxes, const TriGpu *tris,
+                                                 const EntryGpu *entries, const BoxGpu *instance_boxes, Ray ray,
+                                                 uint32_t visibility, uint32_t src_obj, uint32_t src_prim) {
+    uint32_t stack[kStackSize];
+    uint32_t sp = 0u, node = 0u, instance = kInvalid, prim_offset = 0u;
+    SlabRay cur = make_slab_ray(ray.o, ray.d);
+    float tmax = ray.tmax;
+    stack_push(stack, sp, kLinkDone);
+    ClosestHit best{ray.tmax, 0.0f, 0.0f, kInvalid, kInvalid};
+    uint32_t best_prim = kInvalid;
+    while (node != kLinkDone) {
+        if (node == kLinkLeave) {
+            cur = make_slab_ray(ray.o, ray.d);
+            instance = kInvalid;
+            node = stack[--sp];
+            continue;
+        }
+        if (node >= kLinkInstance) {
+            const EntryGpu &e = entries[node & ~kLinkInstance];
+            if ((e.visibility_reach & visibility) == 0u) {
+                node = stack[--sp];
+                continue;
+            }
+            const Xform w2o = xform12(e.w2o);
+            cur = make_slab_ray(xform_point(w2o, ray.o), xform_direction(w2o, ray.d));
+            instance = node & ~kLinkInstance;
+            prim_offset = e.prim_offset;
+            stack_push(stack, sp, kLinkLeave);
+            node = e.root;
+            continue;
+        }
+        float key[4] = {kInf, kInf, kInf, kInf};
+        uint32_t val[4], leaves = 0u;
+        const uint32_t *link = nodes[node].link;
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const uint32_t v = link[k];
+            float near;
+            if (v == kInvalid) continue;
+            if ((v & kLinkLeaf) != 0u) {
+                const TriGpu &tri = tris[v & ~kLinkLeaf];
+                const float4 e = tri.lo_z_hi;
+                if (box_admits(cur, mk3(tri.v1.w, tri.v2.w, e.x), mk3(e.y, e.z, e.w), ray.tmin, tmax, near))
+                    leaves |= 1u << k;
+                continue;
+            }
+            const bool inner = v < kLinkInstance;
+            const float *box = inner ? node_boxes[v].lo : instance_boxes[v & ~kLinkInstance].lo;
+            const uint32_t slot = inner ? node_boxes[v].slot : k;
+            val[slot] = v;
+            if (box_admits(cur, ld3(box), ld3(box + 3), ray.tmin, tmax, near)) key[slot] = near;
+        }
+        for (uint32_t k = 0; k < 4u; ++k) {
+            if ((leaves >> k & 1u) == 0u) continue;
+            const TriGpu &tri = tris[link[k] & ~kLinkLeaf];
+            const uint32_t prim = __float_as_uint(tri.v0.w);
+            if (src_obj == instance && src_prim == prim_offset + prim) continue;
+            float th, u, v;
+            if (!intersect_triangle(cur.o, cur.d, ray.tmin, tmax, ld3(tri.v0), ld3(tri.v1), ld3(tri.v2), th, u, v))
+                continue;
+            const bool later = instance > best.instance || (instance == best.instance && prim > best_prim);
+            if (best.instance != kInvalid && !(th < best.t || (th == best.t && later))) continue;
+            best = {th, u, v, instance, link[k] & ~kLinkLeaf};
+            best_prim = prim;
+            tmax = th;
+        }
+        for (uint32_t k = 0; k < 4u; ++k)
+            if (!(key[k] <= tmax)) key[k] = kInf;
+        sort_children(key, val);
+        for (uint32_t k = 3u; k >= 1u; --k)
+            if (key[k] != kInf) stack_push(stack, sp, val[k]);
+        node = key[0] != kInf ? val[0] : stack[--sp];
+    }
+    return best;
+}
+
+// The ray of a path as its record holds it, traced so.
+__device__ __forceinline__ ClosestHit closest_exact(const SceneView &s, const PathBuffers &b, uint32_t path) {
+    float4 o, d;
+    uint4 st, st2;
+    load_pair(b.ray_o, path, o, d);
+    load_pair(b.st, path, st, st2);
+    return closest_exact(s.nodes, s.node_boxes, s.tris, s.entries, s.instance_boxes, {mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w},
+                         contract_visibility(st.y), st2.y, st2.z);
+}
+
+__device__ __forceinline__ uint32_t closest_prim(const ClosestHit &best, const SceneView &s) {
+    return best.instance == kInvalid ? kInvalid : __float_as_uint(__ldg(&s.tris[best.slot].v0.w));
+}
+
+__device__ __forceinline__ void closest_store(const ClosestHit &best, uint32_t prim, const PathBuffers &b,
+                                              uint32_t path) {
     store_pair(b.hit, path, make_float4(best.t, best.u, best.v, __uint_as_float(best.instance)),
-               make_uint4(best.prim, 0u, 0u, 0u));
+               make_uint4(prim, 0u, 0u, 0u));
 }
 
 // kMulti: paths of a batched wavefront, each traced in its job's scene.
@@ -317,13 +454,30 @@ __global__ void __launch_bounds__(128, PSY_INTERSECT_MIN_BLOCKS)
         const int busy = __popc(__ballot_sync(kFullMask, active));
         if (busy == 0) break;
         traverse_warp<true>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
-                            [&](uint32_t ii, uint32_t local, uint32_t, float th, float u, float v) {
-            return closest_hit(best, t, ii, local, th, u, v);
+                            [&](uint32_t ii, uint32_t local, uint32_t, uint32_t slot, float th, float u, float v) {
+            return closest_hit(best, t, s, ii, local, slot, th, u, v);
         });
         if (active && t.node == kLinkDone && t.leaves == 0u) {
-            closest_store(best, b, path);
+            uint32_t prim;
+            if (closest_ambiguous(best, t, s, prim)) b.ambiguous[atomicAdd(&b.counters[kCounterAmbiguous], 1u)] = path;
+            closest_store(best, prim, b, path);
             active = false;
         }
+    }
+}
+
+// The closest hits of the paths k_intersect has found ambiguous, mostly none.
+// Called from k_intersect itself, closest_exact cost that kernel registers
+// (1080p procedural frame, 64 spp: 291 -> 308 ms).
+template <bool kMulti>
+__global__ void __launch_bounds__(128)
+    k_closest_exact(const __grid_constant__ SceneView s_arg, const __grid_constant__ PathBuffers b, const JobGpu *jobs) {
+    const uint32_t count = b.counters[kCounterAmbiguous];
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        const uint32_t path = b.ambiguous[q];
+        const SceneView &s = kMulti ? jobs[b.job[path]].s : s_arg;
+        const ClosestHit best = closest_exact(s, b, path);
+        closest_store(best, closest_prim(best, s), b, path);
     }
 }
 
@@ -1179,6 +1333,15 @@ __global__ void __launch_bounds__(128, PSY_SHADE_MIN_BLOCKS)
     }
 }
 
+// A triangle's padded extent on one axis: as the host pads its boxes
+// (padded in psy_host.cpp), in double, rounded outward.
+__device__ __forceinline__ void pad_axis(float a, float b, float c, float &lo, float &hi) {
+    const double l = fminf(a, fminf(b, c)), h = fmaxf(a, fmaxf(b, c));
+    const double pad = 1e-5 * (h - l) + 1e-6 * fmax(fabs(l), fabs(h)) + 1e-30;
+    lo = nextafterf(float(l - pad), -INFINITY);
+    hi = nextafterf(float(h + pad), INFINITY);
+}
+
 // Triangle records of all meshes from their vertex arrays: thread i takes
 // leaf slot i, which holds triangle order[i] of its mesh.
 __global__ void k_pack_triangles(const MeshGpu *meshes, uint32_t mesh_count, const float *positions,
@@ -1203,11 +1366,15 @@ __global__ void k_pack_triangles(const MeshGpu *meshes, uint32_t mesh_count, con
         p[k] = ld3(P + 3u * idx[k]);
         n[k] = m.smooth ? ld3(N + 3u * idx[k]) : mk3(0.0f);
     }
+    float bl[3], bh[3];
+    pad_axis(p[0].x, p[1].x, p[2].x, bl[0], bh[0]);
+    pad_axis(p[0].y, p[1].y, p[2].y, bl[1], bh[1]);
+    pad_axis(p[0].z, p[1].z, p[2].z, bl[2], bh[2]);
     TriGpu t;
     t.v0 = make_float4(p[0].x, p[0].y, p[0].z, __uint_as_float(local));
-    t.v1 = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
-    t.v2 = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
-    t.pad = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    t.v1 = make_float4(p[1].x, p[1].y, p[1].z, bl[0]);
+    t.v2 = make_float4(p[2].x, p[2].y, p[2].z, bl[1]);
+    t.lo_z_hi = make_float4(bl[2], bh[0], bh[1], bh[2]);
     tris[i] = t;
     const f3 ng = safe_normalize(cross(p[1] - p[0], p[2] - p[0]), mk3(0.0f, 0.0f, 1.0f));
     ShadeTriGpu o;
@@ -1420,7 +1587,7 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
         const int busy = __popc(__ballot_sync(kFullMask, active));
         if (busy == 0) break;
         traverse_warp<false>(t, s, exhausted ? 32 : min(32, 32 - busy + kRefillLanes),
-                             [&](uint32_t ii, uint32_t, uint32_t cp, float th, float, float) {
+                             [&](uint32_t ii, uint32_t, uint32_t cp, uint32_t, float th, float, float) {
             return shadow_hit(h, s, p, ii, cp, th);
         });
         if (!active || t.node != kLinkDone || t.leaves != 0u) continue;
@@ -1474,12 +1641,17 @@ __global__ void __launch_bounds__(128, PSY_TAIL_MIN_BLOCKS)
                 closest_begin(best, t, s, b, i);
                 closest_rays += 1u;
             }
-            traverse_warp<true>(t, s, 32, [&](uint32_t ii, uint32_t local, uint32_t, float th, float u, float v) {
-                return closest_hit(best, t, ii, local, th, u, v);
+            traverse_warp<true>(t, s, 32, [&](uint32_t ii, uint32_t local, uint32_t, uint32_t slot, float th, float u, float v) {
+                return closest_hit(best, t, s, ii, local, slot, th, u, v);
             });
             ShadeResult r{};
             if (active) {
-                closest_store(best, b, i);
+                uint32_t prim;
+                if (closest_ambiguous(best, t, s, prim)) {
+                    best = closest_exact(s, b, i);
+                    prim = closest_prim(best, s);
+                }
+                closest_store(best, prim, b, i);
                 r = shade_path<false, kGlossy, false>(s, p, b, i, step, kInvalid, nullptr);
             }
             if (__any_sync(kFullMask, r.shadow)) {
@@ -1494,7 +1666,7 @@ __global__ void __launch_bounds__(128, PSY_TAIL_MIN_BLOCKS)
                     shadow_rays += 1u;
                 }
                 while (__any_sync(kFullMask, pending)) {
-                    traverse_warp<false>(t, s, 32, [&](uint32_t ii, uint32_t, uint32_t cp, float th, float, float) {
+                    traverse_warp<false>(t, s, 32, [&](uint32_t ii, uint32_t, uint32_t cp, uint32_t, float th, float, float) {
                         return shadow_hit(h, s, p, ii, cp, th);
                     });
                     if (pending && shadow_resolve(h, t, s, p)) {
@@ -1605,7 +1777,7 @@ __global__ void k_begin_round(uint32_t *counters, uint32_t *round, BatchItem *it
         counters[kCounterWaveGlossy] = plan_rounds[4u * w + 3u] & 1u;
         counters[kCounterWaveTree] = plan_rounds[4u * w + 3u] >> 1;
         counters[0] = round[0];
-        counters[1] = counters[2] = counters[3] = counters[4] = 0u;
+        counters[1] = counters[2] = counters[3] = counters[4] = counters[kCounterAmbiguous] = 0u;
         counters[kCounterTail] = round[0] < tail_paths ? 1u : 0u;
         *cursor = w + 1u;
     }
@@ -1623,6 +1795,7 @@ __global__ void k_end_step(uint32_t *counters, unsigned long long *stats, uint32
     counters[2] = 0u;
     counters[3] = 0u;
     counters[4] = 0u;
+    counters[kCounterAmbiguous] = 0u;
     if (counters[0] < tail_paths) counters[kCounterTail] = step + 2u;
 }
 
@@ -1632,6 +1805,7 @@ __global__ void k_set_counters(uint32_t *counters, uint32_t n, uint32_t tail_pat
     counters[2] = 0u;
     counters[3] = 0u;
     counters[4] = 0u;
+    counters[kCounterAmbiguous] = 0u;
     counters[kCounterTail] = n < tail_paths ? 1u : 0u;
 }
 
@@ -1774,6 +1948,7 @@ void launch_ray_sort(cudaStream_t st, const LaunchConfig &lc, const SceneView &s
 void launch_intersect(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, uint32_t max_work) {
     if (lc.ray_sort_threshold) launch_ray_sort<false>(st, lc, s, b, nullptr, max_work);
     k_intersect<false><<<persistent_grid(max_work, lc), 128, 0, st>>>(s, b, nullptr, lc.ray_sort_threshold);
+    k_closest_exact<false><<<lc.sms, 128, 0, st>>>(s, b, nullptr);
 }
 void launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                   uint32_t max_work, uint32_t step, uint32_t trace_path, psy_path_trace *trace) {
@@ -1849,6 +2024,7 @@ void launch_raygen_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *
 void launch_intersect_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work) {
     if (lc.ray_sort_threshold) launch_ray_sort<true>(st, lc, SceneView{}, b, jobs, max_work);
     k_intersect<true><<<persistent_grid(max_work, lc), 128, 0, st>>>(SceneView{}, b, jobs, lc.ray_sort_threshold);
+    k_closest_exact<true><<<lc.sms, 128, 0, st>>>(SceneView{}, b, jobs);
 }
 void launch_shade_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work,
                         uint32_t step) {

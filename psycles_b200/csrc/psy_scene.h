@@ -4,8 +4,9 @@
 //   nodes         4-wide BVH nodes with byte-quantised boxes, 64 B each
 //                 (two 32-byte sectors): the instance tree, then every
 //                 mesh's tree
+//   node_boxes / instance_boxes  float boxes, 32 B each
 //   tris          leaf triangles of all meshes in node order, 64 B each:
-//                 object-space vertices, v0.w = local primitive index bits
+//                 object-space vertices, local primitive index, padded box
 //   entries       per instance, the ray's transform and the mesh's root (64 B)
 //   shade_tris    the meshes' triangles as shading reads them, 96 B each
 //   instances     InstanceGpu (object<->world transforms, material)
@@ -60,10 +61,21 @@ struct alignas(32) NodeGpu {
 };
 static_assert(sizeof(NodeGpu) == 64, "a node is two 32-byte sectors");
 
-// A leaf triangle (object space) in two sectors.
+// A padded float box: of a node as its parent's child (what its bytes there
+// enclose; only closest_exact in psy_kernels.cu reads it), or of an instance in
+// the world.
+struct alignas(32) BoxGpu {
+    float lo[3], hi[3];
+    uint32_t slot;  // a node's place among its parent's children as built (leaves come first in NodeGpu)
+    uint32_t pad;
+};
+static_assert(sizeof(BoxGpu) == 32, "a box is one 32-byte sector");
+
+// A leaf triangle (object space) and its padded float box in two sectors.
 struct alignas(32) TriGpu {
-    float4 v0;  // w: local primitive index bits
-    float4 v1, v2, pad;
+    float4 v0;        // w: local primitive index bits
+    float4 v1, v2;    // w: box lo.x, lo.y
+    float4 lo_z_hi;   // box lo.z, hi.x, hi.y, hi.z
 };
 static_assert(sizeof(TriGpu) == 64, "a triangle is two 32-byte sectors");
 
@@ -72,7 +84,9 @@ struct alignas(32) EntryGpu {
     float w2o[12];
     uint32_t root;         // root node of the mesh
     uint32_t prim_offset;  // Cycles primitive id of local primitive 0
-    uint32_t visibility;
+    // low half: visibility; high half: that of a float, how far from the world's
+    // origin rays may start whose hits need no test of the instance's box
+    uint32_t visibility_reach;
     uint32_t material;  // as InstanceGpu::material
 };
 static_assert(sizeof(EntryGpu) == 64, "an instance entry is two 32-byte sectors");
@@ -170,6 +184,8 @@ struct alignas(16) LampConstGpu {
 
 struct SceneView {
     const NodeGpu *nodes;  // the instance tree from node 0, then every mesh's tree
+    const BoxGpu *node_boxes;      // one per node
+    const BoxGpu *instance_boxes;  // one per instance
     const TriGpu *tris;
     const EntryGpu *entries;  // one per instance
     const InstanceGpu *instances;
@@ -273,9 +289,9 @@ struct PathBuffers {
     uint32_t *sh_path;
     uint32_t *queue_in;
     uint32_t *queue_out;
-    uint32_t *shadow_queue;
+    uint32_t *ambiguous;  // paths whose closest hit depends on the order of visits
     uint32_t *counters;  // [0] in count, [1] out count, [2] shadow count, [3..4] fetch cursors, [kCounterMisses],
-                         // [kCounterTail],
+                         // [kCounterTail], [kCounterAmbiguous],
                          // [kCounterWaveGlossy] a batched wavefront's glossy flag
     uint32_t *job;       // batched wavefronts: the job of each path
     // shading-queue sort by material: per-queue-entry bucket, the sorted
@@ -287,6 +303,7 @@ constexpr uint32_t kSortBuckets = 2048u;
 constexpr uint32_t kCounterMisses = 5u;  // misses at the front of a sorted shading queue
 // 1 + the step from which the queue is k_tail's; 0 before that
 constexpr uint32_t kCounterTail = 6u;
+constexpr uint32_t kCounterAmbiguous = 7u;  // paths in PathBuffers::ambiguous
 constexpr uint32_t kCounterWaveGlossy = 8u;
 constexpr uint32_t kCounterWaveTree = 9u;  // a job of the batched wavefront uses its light tree
 // sh_path top bit: the shadow ray's path has ended, its contribution goes to rad_final
