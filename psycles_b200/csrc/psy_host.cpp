@@ -1184,42 +1184,59 @@ psy_status parallel_for(uint32_t n, uint32_t *threads, F &&body) {
     return failed.load() ? fail(PSY_ERROR_OUT_OF_MEMORY, "host memory exhausted while building the scene") : PSY_OK;
 }
 
-// Uploads `v` into a new device buffer that takes the place of `slot`; the
-// buffer it replaces joins the scene's retired list.
-// The new buffer is stream-ordered on the context's stream, and the host
-// copy it is uploaded from stays alive with the retired list, so the caller
-// need not wait for the upload.
-template <typename T>
-cudaError_t replace_buffer(psy_scene *sc, DeviceBuffer &slot, const std::vector<T> &v) {
-    auto source = std::make_shared<const std::vector<T>>(v);
-    auto fresh = std::make_unique<DeviceBuffer>(sc->context->stream);
-    const cudaError_t e = fresh->upload(*source, sc->context->stream);
-    if (e != cudaSuccess) return e;
-    slot.swap(*fresh);
-    if (fresh->ptr) sc->retired.push_back(std::move(fresh));
-    sc->retired_host.push_back(std::move(source));
-    return cudaSuccess;
-}
+// New contents of several device buffers of a scene, put in place together: all
+// are allocated and filled before `commit` swaps any, so that an edit that fails
+// on the way (out of device memory) leaves the scene as it was.  The new buffers
+// are stream-ordered on the context's stream.  The host copies they are uploaded
+// from stay alive with the retired list, so the caller need not wait for the
+// uploads; the buffers they replace join that list.
+struct BufferSwap {
+    explicit BufferSwap(psy_scene *scene) : sc(scene) {}
+    template <typename T>
+    cudaError_t upload(DeviceBuffer &slot, const std::vector<T> &v) {
+        auto source = std::make_shared<const std::vector<T>>(v);
+        sc->retired_host.push_back(source);
+        return add(slot).upload(*source, sc->context->stream);
+    }
+    // A copy, for an edit of part of the buffer.
+    cudaError_t copy(DeviceBuffer &slot) {
+        DeviceBuffer &fresh = add(slot);
+        const cudaError_t e = fresh.alloc(slot.bytes);
+        if (e != cudaSuccess) return e;
+        return cudaMemcpyAsync(fresh.ptr, slot.ptr, slot.bytes, cudaMemcpyDeviceToDevice, sc->context->stream);
+    }
+    // The buffer `slot` will be, itself if it stays.
+    const DeviceBuffer &operator[](const DeviceBuffer &slot) const {
+        for (const auto &i : items)
+            if (i.first == &slot) return *i.second;
+        return slot;
+    }
+    void commit() {
+        sc->retired.reserve(sc->retired.size() + items.size());
+        for (auto &i : items) {
+            i.first->swap(*i.second);
+            if (i.second->ptr) sc->retired.push_back(std::move(i.second));
+        }
+        items.clear();
+    }
 
-// Replaces a device buffer by a stream-ordered copy of itself, for an edit
-// of part of it; the old one is retired.
-cudaError_t copy_buffer(psy_scene *sc, DeviceBuffer &slot) {
-    auto fresh = std::make_unique<DeviceBuffer>(sc->context->stream);
-    cudaError_t e = fresh->alloc(slot.bytes);
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(fresh->ptr, slot.ptr, slot.bytes, cudaMemcpyDeviceToDevice, sc->context->stream);
-    if (e != cudaSuccess) return e;
-    slot.swap(*fresh);
-    if (fresh->ptr) sc->retired.push_back(std::move(fresh));
-    return cudaSuccess;
-}
+private:
+    DeviceBuffer &add(DeviceBuffer &slot) {
+        items.emplace_back(&slot, std::make_unique<DeviceBuffer>(sc->context->stream));
+        return *items.back().second;
+    }
+    psy_scene *sc;
+    std::vector<std::pair<DeviceBuffer *, std::unique_ptr<DeviceBuffer>>> items;
+};
 
 // The many-light tree over the scene's emitter population -- emissive
 // triangles in emitter order, then the analytic lights -- built from the
 // host copies and uploaded (src/luisa/path_tracer_light_sampling_scene.cpp:
 // 160-240).  A tree whose root carries no energy is left empty, and
-// sessions then select lights from the flat distribution.
-psy_status build_light_tree(psy_scene *sc, bool sync = true) {
+// sessions then select lights from the flat distribution.  `stage_light_tree`
+// leaves the buffers to `swap` and the tree's shape to `view`.
+psy_status stage_light_tree(psy_scene *sc, const std::vector<float> &scalars, const std::vector<float> &vectors,
+                            BufferSwap &swap, psy::SceneView &view) {
     const auto t0 = std::chrono::steady_clock::now();
     std::vector<psy::LtNodeGpu> lt_nodes;
     std::vector<psy::LtEmitterGpu> lt_emitters;
@@ -1237,8 +1254,8 @@ psy_status build_light_tree(psy_scene *sc, bool sync = true) {
         m.closures = sc->code_host.data() + g.code_offset;
         m.closure_count = g.code_count;
         m.root = g.root;
-        m.scalars = sc->scalars.data() + g.scalar_offset;
-        m.vectors = sc->vectors.data() + 3ull * g.vector_offset;
+        m.scalars = scalars.data() + g.scalar_offset;
+        m.vectors = vectors.data() + 3ull * g.vector_offset;
         m.values = sc->values_host.data() + g.value_offset;
         m.value_count = g.value_count;
         if (g.has_emission) emission_estimate(m, estimates[i].data());
@@ -1320,26 +1337,34 @@ psy_status build_light_tree(psy_scene *sc, bool sync = true) {
             lt_root = tree.root;
         }
     }
-    cudaStream_t st = sc->context->stream;
     PSY_CUDA_TRY(cudaSetDevice(sc->context->device));
     // new buffers; a tree built before is retired, not freed, as queued
     // work may still read it
-    PSY_CUDA_TRY(replace_buffer(sc, sc->lt_nodes, lt_nodes));
-    PSY_CUDA_TRY(replace_buffer(sc, sc->lt_emitters, lt_emitters));
-    PSY_CUDA_TRY(replace_buffer(sc, sc->lt_mapping, lt_mapping));
-    PSY_CUDA_TRY(replace_buffer(sc, sc->lt_lookup, lt_lookup));
-    if (sync) PSY_CUDA_TRY(cudaStreamSynchronize(st));
-    psy::SceneView &v = sc->view;
-    v.lt_nodes = sc->lt_nodes.as<psy::LtNodeGpu>();
-    v.lt_emitters = sc->lt_emitters.as<psy::LtEmitterGpu>();
-    v.lt_mapping = sc->lt_mapping.as<uint2>();
-    v.lt_lookup = sc->lt_lookup.as<uint4>();
-    v.lt_node_count = uint32_t(lt_nodes.size());
-    v.lt_emitter_count = uint32_t(lt_emitters.size());
-    v.lt_lookup_count = uint32_t(lt_lookup.size());
-    v.lt_root = lt_root;
-    sc->light_tree_built = true;
+    PSY_CUDA_TRY(swap.upload(sc->lt_nodes, lt_nodes));
+    PSY_CUDA_TRY(swap.upload(sc->lt_emitters, lt_emitters));
+    PSY_CUDA_TRY(swap.upload(sc->lt_mapping, lt_mapping));
+    PSY_CUDA_TRY(swap.upload(sc->lt_lookup, lt_lookup));
+    view.lt_nodes = swap[sc->lt_nodes].as<psy::LtNodeGpu>();
+    view.lt_emitters = swap[sc->lt_emitters].as<psy::LtEmitterGpu>();
+    view.lt_mapping = swap[sc->lt_mapping].as<uint2>();
+    view.lt_lookup = swap[sc->lt_lookup].as<uint4>();
+    view.lt_node_count = uint32_t(lt_nodes.size());
+    view.lt_emitter_count = uint32_t(lt_emitters.size());
+    view.lt_lookup_count = uint32_t(lt_lookup.size());
+    view.lt_root = lt_root;
     sc->stats.light_tree_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    return PSY_OK;
+}
+
+psy_status build_light_tree(psy_scene *sc) {
+    BufferSwap swap(sc);
+    psy::SceneView view = sc->view;
+    const psy_status r = stage_light_tree(sc, sc->scalars, sc->vectors, swap, view);
+    if (r != PSY_OK) return r;
+    PSY_CUDA_TRY(cudaStreamSynchronize(sc->context->stream));
+    swap.commit();
+    sc->view = view;
+    sc->light_tree_built = true;
     sc->stats.light_tree_builds++;
     return PSY_OK;
 }
@@ -1352,28 +1377,35 @@ psy_status psy::host::rebind_parameters_versioned(psy_scene *s, uint32_t materia
     if (valid != PSY_OK) return valid;
     const psy::MaterialGpu &m = s->materials[material];
     PSY_CUDA_TRY(cudaSetDevice(s->context->device));
-    if (scalar_count) std::memcpy(s->scalars.data() + m.scalar_offset, scalars, sizeof(float) * scalar_count);
-    if (vector_count) std::memcpy(s->vectors.data() + 3ull * m.vector_offset, vectors, sizeof(float) * 3u * vector_count);
-    PSY_CUDA_TRY(replace_buffer(s, s->scalar_buf, s->scalars));
-    PSY_CUDA_TRY(replace_buffer(s, s->vector_buf, s->vectors));
-    s->view.scalars = s->scalar_buf.as<float>();
-    s->view.vectors = s->vector_buf.as<float>();
-    PSY_CUDA_TRY(copy_buffer(s, s->baked));
-    PSY_CUDA_TRY(copy_buffer(s, s->closures));
-    s->view.baked = s->baked.as<psy::BakedMaterialGpu>();
-    s->view.closures = s->closures.as<psy::BakedClosureGpu>();
-    psy::launch_bake_materials(s->context->stream, s->view, s->baked.as<psy::BakedMaterialGpu>(),
-                               s->closures.as<psy::BakedClosureGpu>(), material, 1u);
-    PSY_CUDA_TRY(cudaGetLastError());
-    if (m.has_emission) {
-        std::lock_guard<std::mutex> lock(s->light_tree_mutex);
-        if (s->light_tree_built) {
-            const psy_status r = build_light_tree(s, false);
-            if (r != PSY_OK) return r;
-        }
-    }
     if (!s->uploads_done) PSY_CUDA_TRY(cudaEventCreateWithFlags(&s->uploads_done, cudaEventDisableTiming));
+    std::vector<float> new_scalars = s->scalars, new_vectors = s->vectors;
+    std::copy(scalars, scalars + scalar_count, new_scalars.begin() + m.scalar_offset);
+    std::copy(vectors, vectors + 3ull * vector_count, new_vectors.begin() + 3ull * m.vector_offset);
+    BufferSwap swap(s);
+    psy::SceneView view = s->view;
+    PSY_CUDA_TRY(swap.upload(s->scalar_buf, new_scalars));
+    PSY_CUDA_TRY(swap.upload(s->vector_buf, new_vectors));
+    PSY_CUDA_TRY(swap.copy(s->baked));
+    PSY_CUDA_TRY(swap.copy(s->closures));
+    view.scalars = swap[s->scalar_buf].as<float>();
+    view.vectors = swap[s->vector_buf].as<float>();
+    view.baked = swap[s->baked].as<psy::BakedMaterialGpu>();
+    view.closures = swap[s->closures].as<psy::BakedClosureGpu>();
+    psy::launch_bake_materials(s->context->stream, view, swap[s->baked].as<psy::BakedMaterialGpu>(),
+                               swap[s->closures].as<psy::BakedClosureGpu>(), material, 1u);
+    PSY_CUDA_TRY(cudaGetLastError());
+    std::lock_guard<std::mutex> lock(s->light_tree_mutex);
+    const bool rebuild = m.has_emission != 0u && s->light_tree_built;
+    if (rebuild) {
+        const psy_status r = stage_light_tree(s, new_scalars, new_vectors, swap, view);
+        if (r != PSY_OK) return r;
+    }
     PSY_CUDA_TRY(cudaEventRecord(s->uploads_done, s->context->stream));
+    swap.commit();
+    s->scalars.swap(new_scalars);
+    s->vectors.swap(new_vectors);
+    s->view = view;
+    if (rebuild) s->stats.light_tree_builds++;
     return PSY_OK;
 }
 
