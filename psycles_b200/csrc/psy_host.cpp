@@ -1515,6 +1515,10 @@ psy_status psy_context_set_tuning(psy_context *c, const psy_tuning *t) {
     c->launch.ray_sort_threshold =
         t->ray_sort_threshold == 0xffffffffu ? defaults.ray_sort_threshold : t->ray_sort_threshold;
     c->launch.stream_block = t->stream_block_size ? t->stream_block_size : defaults.stream_block;
+    // a queue long enough to be sorted is not k_tail's
+    c->launch.tail_paths = defaults.tail_paths;
+    for (const uint32_t sorted : {c->launch.sort_threshold, c->launch.shadow_sort_threshold, c->launch.ray_sort_threshold})
+        if (sorted != 0u) c->launch.tail_paths = std::min(c->launch.tail_paths, sorted);
     return PSY_OK;
 }
 
