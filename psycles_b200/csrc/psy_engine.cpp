@@ -107,17 +107,16 @@ uint32_t WavefrontEngine::issue(uint32_t steps, bool allow_exit, psy_status &sta
     PathBuffers b = arena_.view;
     unsigned long long *stats = arena_.stats.as<unsigned long long>();
     status = PSY_OK;
-    launch_begin_round(st, lc, b.counters, round_.as<uint32_t>(), items_.as<BatchItem>(), plan_rounds_.as<uint32_t>(),
-                       plan_items_.as<BatchItem>(), cursor_.as<uint32_t>(), max_jobs_);
-    launch_raygen_batch(st, lc, jt, it, rd, b, cap);
-    uint32_t launches = 2u;
+    uint32_t launches =
+        launch_begin_round(st, lc, b.counters, round_.as<uint32_t>(), items_.as<BatchItem>(), plan_rounds_.as<uint32_t>(),
+                           plan_items_.as<BatchItem>(), cursor_.as<uint32_t>(), max_jobs_);
+    launches += launch_raygen_batch(st, lc, jt, it, rd, b, cap);
     for (uint32_t step = 0; step < steps; ++step) {
-        launch_intersect_batch(st, lc, jt, b, cap);
-        launch_shade_batch(st, lc, jt, b, cap, step);
-        launch_shadow_batch(st, lc, jt, b, cap, step);
-        launch_end_step(st, lc, b.counters, stats, step);
+        launches += launch_intersect_batch(st, lc, jt, b, cap);
+        launches += launch_shade_batch(st, lc, jt, b, cap, step);
+        launches += launch_shadow_batch(st, lc, jt, b, cap, step);
+        launches += launch_end_step(st, lc, b.counters, stats, step);
         std::swap(b.queue_in, b.queue_out);
-        launches += 4u;
         if (allow_exit && (step + 1u) % check_interval_ == 0u) {
             uint32_t left = 0u;
             if (cudaMemcpyAsync(&left, b.counters, sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -128,9 +127,9 @@ uint32_t WavefrontEngine::issue(uint32_t steps, bool allow_exit, psy_status &sta
             if (left < std::max(lc.tail_paths, 1u)) break;
         }
     }
-    launch_tail_batch(st, lc, jt, arena_.view, cap, stats);
-    launch_film_batch(st, lc, jt, it, rd, b, cap);
-    return launches + 2u;
+    launches += launch_tail_batch(st, lc, jt, arena_.view, cap, stats);
+    launches += launch_film_batch(st, lc, jt, it, rd, b, cap);
+    return launches;
 }
 
 psy_status WavefrontEngine::ensure_graph(uint32_t steps) {
@@ -143,7 +142,7 @@ psy_status WavefrontEngine::ensure_graph(uint32_t steps) {
     cudaStream_t st = context_->stream;
     PSY_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     psy_status s = PSY_OK;
-    issue(steps, false, s);
+    graph_kernels_ = issue(steps, false, s);
     cudaGraph_t g = nullptr;
     const cudaError_t end = cudaStreamEndCapture(st, &g);
     if (s != PSY_OK) {
@@ -192,7 +191,7 @@ psy_status WavefrontEngine::run(const EnginePlan &plan, uint32_t steps, EngineRu
         if (use_graph_) {
             PSY_CUDA_TRY(cudaGraphLaunch(graph_, st));
             out.graph_launches += 1u;
-            out.kernel_launches += 4u + 4u * steps;
+            out.kernel_launches += graph_kernels_;
         } else {
             psy_status s = PSY_OK;
             out.kernel_launches += issue(steps, true, s);

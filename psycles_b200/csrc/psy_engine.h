@@ -86,6 +86,7 @@ class WavefrontEngine {
     bool began_ = false;
     cudaGraphExec_t graph_ = nullptr;
     uint32_t graph_steps_ = 0, graph_capacity_ = 0;
+    uint32_t graph_kernels_ = 0;  // kernel nodes of `graph_`
     uint64_t plan_generation_ = 0, graph_generation_ = 0;
 };
 

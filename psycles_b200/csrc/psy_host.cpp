@@ -2409,11 +2409,11 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
     // synchronisation so the queue sizes the byte model needs are final.
     auto timed = [&](auto &&launch, uint32_t &launches, float &ms) -> psy_status {
         if (!prof) {
-            launch();
+            stats.kernel_launches += launch();
             return PSY_OK;
         }
         PSY_CUDA_TRY(cudaEventRecord(s->ev_k[0], st));
-        launch();
+        stats.kernel_launches += launch();
         PSY_CUDA_TRY(cudaEventRecord(s->ev_k[1], st));
         PSY_CUDA_TRY(cudaEventSynchronize(s->ev_k[1]));
         float t = 0.0f;
@@ -2442,9 +2442,10 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
         }
         psy_path_trace *tr = trace_path != psy::kInvalidId ? trace : nullptr;
         psy::PathBuffers b = ctx->arena.view;
-        psy::launch_set_counters(st, lc, b.counters, paths);
-        if ((ps = timed([&] { psy::launch_raygen(st, lc, p, b, pixels, paths, uint32_t(sample), trace_path, tr); },
-                        pf.raygen_launches, pf.raygen_ms)) != PSY_OK)
+        stats.kernel_launches += psy::launch_set_counters(st, lc, b.counters, paths);
+        if ((ps = timed(
+                 [&] { return psy::launch_raygen(st, lc, p, b, pixels, paths, uint32_t(sample), trace_path, tr); },
+                 pf.raygen_launches, pf.raygen_ms)) != PSY_OK)
             return ps;
         pf.raygen_bytes += 164.0 * paths;
         stats.camera_rays += paths;
@@ -2452,22 +2453,23 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
         for (uint32_t step = 0; step < p.steps && !all_tail; ++step) {
             uint32_t c3[3] = {0u, 0u, 0u};
             if (prof && (ps = read_counters(c3)) != PSY_OK) return ps;
-            if ((ps = timed([&] { psy::launch_intersect(st, lc, s->scene->view, b, paths); }, pf.intersect_launches,
-                            pf.intersect_ms)) != PSY_OK)
+            if ((ps = timed([&] { return psy::launch_intersect(st, lc, s->scene->view, b, paths); },
+                            pf.intersect_launches, pf.intersect_ms)) != PSY_OK)
                 return ps;
             pf.intersect_bytes += 88.0 * c3[0];
-            if ((ps = timed([&] { psy::launch_shade(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
-                            pf.shade_launches, pf.shade_ms)) != PSY_OK)
+            if ((ps = timed(
+                     [&] { return psy::launch_shade(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
+                     pf.shade_launches, pf.shade_ms)) != PSY_OK)
                 return ps;
             if (prof && (ps = read_counters(c3)) != PSY_OK) return ps;
             pf.shade_bytes += 304.0 * c3[0] + 68.0 * c3[2];
-            if ((ps = timed([&] { psy::launch_shadow(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
-                            pf.shadow_launches, pf.shadow_ms)) != PSY_OK)
+            if ((ps = timed(
+                     [&] { return psy::launch_shadow(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
+                     pf.shadow_launches, pf.shadow_ms)) != PSY_OK)
                 return ps;
             pf.shadow_bytes += 100.0 * c3[2];
-            psy::launch_end_step(st, lc, b.counters, ray_stats, step);
+            stats.kernel_launches += psy::launch_end_step(st, lc, b.counters, ray_stats, step);
             std::swap(b.queue_in, b.queue_out);
-            stats.kernel_launches += 4u;
             // every 4 steps, stop early once no more paths are left than
             // the tail kernel takes
             if ((step & 3u) == 3u) {
@@ -2477,15 +2479,14 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
                 if (left < std::max(lc.tail_paths, 1u)) break;
             }
         }
-        psy::launch_tail(st, lc, s->scene->view, p, ctx->arena.view, paths, ray_stats);
-        if (lc.tail_paths != 0u) stats.kernel_launches += 1u;
+        stats.kernel_launches += psy::launch_tail(st, lc, s->scene->view, p, ctx->arena.view, paths, ray_stats);
         if ((ps = timed([&] {
-                 psy::launch_film(st, lc, b, pixels, n_samples, s->combined.as<float4>(), s->normal.as<float4>(),
-                                  s->albedo.as<float4>(), s->sample_count.as<uint32_t>(), trace_path, tr);
+                 return psy::launch_film(st, lc, b, pixels, n_samples, s->combined.as<float4>(),
+                                         s->normal.as<float4>(), s->albedo.as<float4>(),
+                                         s->sample_count.as<uint32_t>(), trace_path, tr);
              }, pf.film_launches, pf.film_ms)) != PSY_OK)
             return ps;
         pf.film_bytes += 48.0 * paths + 104.0 * pixels;
-        stats.kernel_launches += 3u;
         stats.batches += 1u;
         sample += n_samples;
     }
@@ -2588,17 +2589,19 @@ psy_status psy_session_render_samples_static(psy_session *s, uint32_t first, uin
         const uint32_t n_samples = uint32_t(std::min<uint64_t>(per_batch, end - sample));
         const uint32_t paths = pixels * n_samples;
         psy::PathBuffers bb = b;
-        psy::launch_set_counters(st, lc, bb.counters, paths);
-        psy::launch_raygen(st, lc, p, bb, pixels, paths, uint32_t(sample), psy::kInvalidId, nullptr);
+        stats.kernel_launches += psy::launch_set_counters(st, lc, bb.counters, paths);
+        stats.kernel_launches +=
+            psy::launch_raygen(st, lc, p, bb, pixels, paths, uint32_t(sample), psy::kInvalidId, nullptr);
         stats.camera_rays += paths;
         const bool all_tail = paths < lc.tail_paths;
         for (uint32_t step = 0; step < p.steps && !all_tail; ++step) {
-            psy::launch_intersect(st, lc, s->scene->view, bb, paths);
-            psy::launch_shade(st, lc, s->scene->view, p, bb, paths, step, psy::kInvalidId, nullptr);
-            psy::launch_shadow(st, lc, s->scene->view, p, bb, paths, step, psy::kInvalidId, nullptr);
-            psy::launch_end_step(st, lc, bb.counters, ray_stats, step);
+            stats.kernel_launches += psy::launch_intersect(st, lc, s->scene->view, bb, paths);
+            stats.kernel_launches +=
+                psy::launch_shade(st, lc, s->scene->view, p, bb, paths, step, psy::kInvalidId, nullptr);
+            stats.kernel_launches +=
+                psy::launch_shadow(st, lc, s->scene->view, p, bb, paths, step, psy::kInvalidId, nullptr);
+            stats.kernel_launches += psy::launch_end_step(st, lc, bb.counters, ray_stats, step);
             std::swap(bb.queue_in, bb.queue_out);
-            stats.kernel_launches += 4u;
             if ((step & 3u) == 3u) {
                 uint32_t left = 0u;
                 PSY_CUDA_TRY(cudaMemcpyAsync(&left, bb.counters, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -2606,11 +2609,10 @@ psy_status psy_session_render_samples_static(psy_session *s, uint32_t first, uin
                 if (left < std::max(lc.tail_paths, 1u)) break;
             }
         }
-        psy::launch_tail(st, lc, s->scene->view, p, b, paths, ray_stats);
-        if (lc.tail_paths != 0u) stats.kernel_launches += 1u;
-        psy::launch_film(st, lc, bb, pixels, n_samples, s->combined.as<float4>(), s->normal.as<float4>(),
-                         s->albedo.as<float4>(), s->sample_count.as<uint32_t>(), psy::kInvalidId, nullptr);
-        stats.kernel_launches += 3u;
+        stats.kernel_launches += psy::launch_tail(st, lc, s->scene->view, p, b, paths, ray_stats);
+        stats.kernel_launches +=
+            psy::launch_film(st, lc, bb, pixels, n_samples, s->combined.as<float4>(), s->normal.as<float4>(),
+                             s->albedo.as<float4>(), s->sample_count.as<uint32_t>(), psy::kInvalidId, nullptr);
         stats.batches += 1u;
         sample += n_samples;
     }

@@ -1889,13 +1889,15 @@ int launch_grid(uint32_t work, int block, const LaunchConfig &lc) {
     return int(blocks < 1u ? 1u : (blocks > cap ? cap : blocks));
 }
 
-void launch_raygen(cudaStream_t st, const LaunchConfig &lc, const RenderParams &p, const PathBuffers &b, uint32_t pixels,
+uint32_t launch_raygen(cudaStream_t st, const LaunchConfig &lc, const RenderParams &p, const PathBuffers &b, uint32_t pixels,
                    uint32_t paths, uint32_t sample_base, uint32_t trace_path, psy_path_trace *trace) {
     k_raygen<<<launch_grid(paths, int(lc.stream_block), lc), lc.stream_block, 0, st>>>(p, b, pixels, paths, sample_base,
                                                                                     trace_path, trace);
+    return 1u;
 }
-void launch_set_counters(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t n) {
+uint32_t launch_set_counters(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t n) {
     k_set_counters<<<1, 1, 0, st>>>(counters, n, lc.tail_paths);
+    return 1u;
 }
 // Persistent kernels: enough resident warps to fill every SM (bounded by the
 // work so small queues launch few blocks).
@@ -1910,20 +1912,22 @@ bool sorts_queue(const LaunchConfig &lc, uint32_t max_work) {
     return lc.sort_threshold != 0u && max_work >= lc.sort_threshold;
 }
 template <bool kMulti>
-void launch_sort(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+uint32_t launch_sort(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                  const JobGpu *jobs, uint32_t max_work) {
     k_sort_count<kMulti><<<launch_grid(max_work, 256, lc), 256, 0, st>>>(s, p, b, jobs, lc.sort_threshold);
     k_sort_scan<<<1, 1024, 0, st>>>(b, lc.sort_threshold, 0u, true);
     // ranks are packed in 21 bits: keep every block's chunk below 2^20 paths
     const int scatter_blocks = std::max(launch_grid(max_work, 256, lc), int((max_work >> 20) + 1u));
     k_sort_scatter<<<scatter_blocks, 256, 0, st>>>(b, lc.sort_threshold, 0u);
+    return 3u;
 }
-void launch_shadow_sort(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t max_work) {
+uint32_t launch_shadow_sort(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t max_work) {
     const uint32_t thr = lc.shadow_sort_threshold;
     k_sort_count_shadow<<<launch_grid(max_work, 256, lc), 256, 0, st>>>(b, thr);
     k_sort_scan<<<1, 1024, 0, st>>>(b, thr, 2u, false);
     const int scatter_blocks = std::max(launch_grid(max_work, 256, lc), int((max_work >> 20) + 1u));
     k_sort_scatter<<<scatter_blocks, 256, 0, st>>>(b, thr, 2u);
+    return 3u;
 }
 int persistent_grid(uint32_t work, const LaunchConfig &lc) {
     const uint32_t blocks = (work + 127u) / 128u;
@@ -1937,26 +1941,34 @@ uint32_t resident_warps(int grid, int blocks_per_sm, const LaunchConfig &lc) {
 }
 
 template <bool kMulti>
-void launch_ray_sort(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, const JobGpu *jobs,
+uint32_t launch_ray_sort(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, const JobGpu *jobs,
                      uint32_t max_work) {
     const uint32_t thr = lc.ray_sort_threshold;
     k_sort_count_rays<kMulti><<<launch_grid(max_work, 256, lc), 256, 0, st>>>(s, b, jobs, thr);
     k_sort_scan<<<1, 1024, 0, st>>>(b, thr, 0u, false);
     const int scatter_blocks = std::max(launch_grid(max_work, 256, lc), int((max_work >> 20) + 1u));
     k_sort_scatter<<<scatter_blocks, 256, 0, st>>>(b, thr, 0u);
+    return 3u;
 }
-void launch_intersect(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, uint32_t max_work) {
-    if (lc.ray_sort_threshold) launch_ray_sort<false>(st, lc, s, b, nullptr, max_work);
+uint32_t launch_intersect(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const PathBuffers &b, uint32_t max_work) {
+    const uint32_t sort = lc.ray_sort_threshold == 0u ? 0u : launch_ray_sort<false>(st, lc, s, b, nullptr, max_work);
     k_intersect<false><<<persistent_grid(max_work, lc), 128, 0, st>>>(s, b, nullptr, lc.ray_sort_threshold);
     k_closest_exact<false><<<lc.sms, 128, 0, st>>>(s, b, nullptr);
+    return sort + 2u;
 }
-void launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+uint32_t launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                   uint32_t max_work, uint32_t step, uint32_t trace_path, psy_path_trace *trace) {
     const bool sorts = sorts_queue(lc, max_work);
-    if (sorts) launch_sort<false>(st, lc, s, p, b, nullptr, max_work);
+    uint32_t launches = sorts ? launch_sort<false>(st, lc, s, p, b, nullptr, max_work) : 0u;
     const int grid = shade_grid(max_work, lc);
-    if (sorts && !trace) k_shade_miss<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
-    if (p.use_light_tree && !trace) k_light_pick<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
+    if (sorts && !trace) {
+        k_shade_miss<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
+        ++launches;
+    }
+    if (p.use_light_tree && !trace) {
+        k_light_pick<false><<<grid, 128, 0, st>>>(s, p, b, nullptr, lc.sort_threshold);
+        ++launches;
+    }
     if (trace && s.has_glossy)
         k_shade<true, false, true><<<grid, 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr, lc.sort_threshold);
     else if (trace)
@@ -1965,40 +1977,46 @@ void launch_shade(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, c
         k_shade<false, false, true><<<grid, 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr, lc.sort_threshold);
     else
         k_shade<false, false, false><<<grid, 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr, lc.sort_threshold);
+    return launches + 1u;
 }
-void launch_shadow(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+uint32_t launch_shadow(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                    uint32_t max_work, uint32_t step, uint32_t trace_path, psy_path_trace *trace) {
-    if (lc.shadow_sort_threshold) launch_shadow_sort(st, lc, b, max_work);
+    const uint32_t sort = lc.shadow_sort_threshold == 0u ? 0u : launch_shadow_sort(st, lc, b, max_work);
     const int grid = persistent_grid(max_work, lc);
     k_shadow<false><<<grid, 128, 0, st>>>(s, p, b, step, trace_path, trace, nullptr, lc.shadow_sort_threshold,
                                           resident_warps(grid, PSY_SHADOW_MIN_BLOCKS, lc));
+    return sort + 1u;
 }
-void launch_begin_round(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t *round, BatchItem *items,
+uint32_t launch_begin_round(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, uint32_t *round, BatchItem *items,
                         const uint32_t *plan_rounds, const BatchItem *plan_items, uint32_t *cursor, uint32_t max_items) {
     k_begin_round<<<1, 256, 0, st>>>(counters, round, items, plan_rounds, plan_items, cursor, max_items, lc.tail_paths);
+    return 1u;
 }
-void launch_end_step(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, unsigned long long *stats,
+uint32_t launch_end_step(cudaStream_t st, const LaunchConfig &lc, uint32_t *counters, unsigned long long *stats,
                      uint32_t step) {
     k_end_step<<<1, 1, 0, st>>>(counters, stats, step, lc.tail_paths);
+    return 1u;
 }
 // Blocks of the tail kernel: all that are resident, but no more than give
 // each warp a path.
 int tail_grid(const LaunchConfig &lc, uint32_t max_work) {
     return int(std::min(uint32_t(lc.sms) * PSY_TAIL_MIN_BLOCKS, (std::min(max_work, lc.tail_paths) + 3u) / 4u));
 }
-void launch_tail(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
+uint32_t launch_tail(cudaStream_t st, const LaunchConfig &lc, const SceneView &s, const RenderParams &p, const PathBuffers &b,
                  uint32_t max_work, unsigned long long *stats) {
-    if (lc.tail_paths == 0u) return;
+    if (lc.tail_paths == 0u) return 0u;
     const int grid = tail_grid(lc, max_work);
     if (s.has_glossy) k_tail<false, true><<<grid, 128, 0, st>>>(s, p, b, b.queue_out, nullptr, stats);
     else k_tail<false, false><<<grid, 128, 0, st>>>(s, p, b, b.queue_out, nullptr, stats);
+    return 1u;
 }
-void launch_tail_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b,
+uint32_t launch_tail_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b,
                        uint32_t max_work, unsigned long long *stats) {
-    if (lc.tail_paths == 0u) return;
+    if (lc.tail_paths == 0u) return 0u;
     const int grid = tail_grid(lc, max_work);
     k_tail<true, false><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, b.queue_out, jobs, stats);
     k_tail<true, true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, b.queue_out, jobs, stats);
+    return 2u;
 }
 void launch_check_counts(cudaStream_t st, const uint32_t *counts, uint32_t n, uint32_t expected, uint32_t *mismatch) {
     cudaMemsetAsync(mismatch, 0, sizeof(uint32_t), st);
@@ -2010,44 +2028,53 @@ void launch_resolve_pass(cudaStream_t st, const float4 *film, const uint32_t *co
     const uint32_t blocks = n == 0u ? 1u : (n + 255u) / 256u;
     k_resolve_pass<<<blocks < 2368u ? blocks : 2368u, 256, 0, st>>>(film, counts, n, kind, exposure, out);
 }
-void launch_film(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t pixels, uint32_t samples, float4 *combined,
+uint32_t launch_film(cudaStream_t st, const LaunchConfig &lc, const PathBuffers &b, uint32_t pixels, uint32_t samples, float4 *combined,
                  float4 *normal, float4 *albedo, uint32_t *sample_count, uint32_t trace_path, psy_path_trace *trace) {
     k_film<<<launch_grid(pixels, int(lc.stream_block), lc), lc.stream_block, 0, st>>>(b, pixels, samples, combined, normal,
                                                                                       albedo, sample_count, trace_path,
                                                                                       trace);
+    return 1u;
 }
 // Batched wavefront: every kernel reads each path's job record.
-void launch_raygen_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const BatchItem *items, const uint32_t *round,
+uint32_t launch_raygen_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const BatchItem *items, const uint32_t *round,
                          const PathBuffers &b, uint32_t max_paths) {
     k_raygen_batch<<<launch_grid(max_paths, int(lc.stream_block), lc), lc.stream_block, 0, st>>>(jobs, items, round, b);
+    return 1u;
 }
-void launch_intersect_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work) {
-    if (lc.ray_sort_threshold) launch_ray_sort<true>(st, lc, SceneView{}, b, jobs, max_work);
+uint32_t launch_intersect_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work) {
+    const uint32_t sort = lc.ray_sort_threshold == 0u ? 0u : launch_ray_sort<true>(st, lc, SceneView{}, b, jobs, max_work);
     k_intersect<true><<<persistent_grid(max_work, lc), 128, 0, st>>>(SceneView{}, b, jobs, lc.ray_sort_threshold);
     k_closest_exact<true><<<lc.sms, 128, 0, st>>>(SceneView{}, b, jobs);
+    return sort + 2u;
 }
-void launch_shade_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work,
+uint32_t launch_shade_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work,
                         uint32_t step) {
     const bool sorts = sorts_queue(lc, max_work);
-    if (sorts) launch_sort<true>(st, lc, SceneView{}, RenderParams{}, b, jobs, max_work);
+    uint32_t launches = sorts ? launch_sort<true>(st, lc, SceneView{}, RenderParams{}, b, jobs, max_work) : 0u;
     const int grid = shade_grid(max_work, lc);
-    if (sorts) k_shade_miss<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, jobs, lc.sort_threshold);
+    if (sorts) {
+        k_shade_miss<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, jobs, lc.sort_threshold);
+        ++launches;
+    }
     k_light_pick<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, jobs, lc.sort_threshold);
     k_shade<false, true, false><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, step, kInvalid, nullptr, jobs,
                                                       lc.sort_threshold);
     k_shade<false, true, true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, step, kInvalid, nullptr, jobs,
                                                      lc.sort_threshold);
+    return launches + 3u;
 }
-void launch_shadow_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work,
+uint32_t launch_shadow_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const PathBuffers &b, uint32_t max_work,
                          uint32_t step) {
-    if (lc.shadow_sort_threshold) launch_shadow_sort(st, lc, b, max_work);
+    const uint32_t sort = lc.shadow_sort_threshold == 0u ? 0u : launch_shadow_sort(st, lc, b, max_work);
     const int grid = persistent_grid(max_work, lc);
     k_shadow<true><<<grid, 128, 0, st>>>(SceneView{}, RenderParams{}, b, step, kInvalid, nullptr, jobs,
                                          lc.shadow_sort_threshold, resident_warps(grid, PSY_SHADOW_MIN_BLOCKS, lc));
+    return sort + 1u;
 }
-void launch_film_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const BatchItem *items, const uint32_t *round,
+uint32_t launch_film_batch(cudaStream_t st, const LaunchConfig &lc, const JobGpu *jobs, const BatchItem *items, const uint32_t *round,
                        const PathBuffers &b, uint32_t max_pixels) {
     k_film_batch<<<launch_grid(max_pixels, int(lc.stream_block), lc), lc.stream_block, 0, st>>>(jobs, items, round, b);
+    return 1u;
 }
 
 void launch_debug_light_tree(cudaStream_t st, const SceneView &s, const float4 *queries, const uint32_t *pdf_emitters,

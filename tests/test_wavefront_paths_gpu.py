@@ -7,6 +7,7 @@ server against sessions alone."""
 
 import numpy as np
 import pytest
+import torch
 
 import test_batch
 import test_camera
@@ -21,7 +22,7 @@ import test_tail_gpu
 import test_traversal_gpu
 import test_value_stream_gpu
 from psycles_b200 import autotune, scenes
-from psycles_b200.backend import SampleRange
+from psycles_b200.backend import BatchRenderer, SampleRange
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +89,33 @@ def test_thresholds_below_the_tail_limit_take_effect(backend, knob):
     assert launches[4801] == launches[default[knob]] < launches[4800] <= launches[1]
     for image in images.values():
         assert np.array_equal(image, images[1])
+
+
+def count_kernels(work):
+    """Kernels of this library that `work` ran, as the CUDA activity records show them."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        work()
+        torch.cuda.synchronize()
+    return sum("psy::k_" in e.name for e in prof.events())
+
+
+@pytest.mark.parametrize("tree", [0, 1])
+@pytest.mark.parametrize("tuning", [{}, SORTED], ids=["default", "sorted"])
+def test_kernel_launch_counts(backend, tuning, tree):
+    torch.zeros(1, device="cuda")
+    default = autotune.get_tuning(backend)
+    compiled = backend.compile_scene(scenes.small_test_scene(seed=6)).scene
+    settings = scenes.render_settings(80, 60, max_bounces=5, use_light_tree=tree)
+    try:
+        autotune.set_tuning(backend, dict(default, **tuning))
+        session = backend.create_session(compiled, settings)
+        ran = count_kernels(lambda: session.render_samples(SampleRange(0, 1, 0, 4)))
+        assert session.stats().kernel_launches == ran
+        for graph in (False, True):
+            batch = BatchRenderer(backend.context, path_capacity=9000, use_graph=graph)
+            ran = count_kernels(lambda: batch.render([(session, SampleRange(1, 3, 0, 4))]))
+            assert batch.stats().kernel_launches == ran
+            batch.close()
+            session = backend.create_session(compiled, settings)
+    finally:
+        autotune.set_tuning(backend, default)
