@@ -607,7 +607,7 @@ psy_status psy_sobol_generate_table(uint32_t sequence_size, float *out);
 psy_status psy_pixel_filter_table(uint32_t filter, float width, float *out);
 
 /* Launch and capacity tuning of a context (what psycles_b200.autotune
- * searches).  Queues of fewer than 65536 paths, or than the least sort
+ * searches).  Queues of fewer than 20480 paths, or than the least sort
  * threshold below that, take their remaining steps in one kernel.  No counterpart in the reference, whose dispatch size is
  * max_samples_per_dispatch.  Zero fields take the defaults. */
 typedef struct psy_tuning {

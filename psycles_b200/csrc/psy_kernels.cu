@@ -1608,11 +1608,15 @@ __global__ void __launch_bounds__(128, PSY_SHADOW_MIN_BLOCKS)
 // while the GPU idles, so a path that still bounces pays that wait for
 // every step; here it pays only for the paths of its own warp, and a warp
 // takes few of them (as many as spread the queue over all resident warps).
-// 128x128 procedural viewport at 1 spp: 3.12 -> 1.15 ms; value materials at
-// 512x512, 4 spp: 2.68 -> 2.00 ms; 1080p frame, 64 spp: 340.5 -> 338.8 ms.  The
-// limit of 64 Ki paths lies where these turn: 16 Ki 1.32 / 2.11 / 340.2 ms, 32 Ki
-// 1.21 / 2.16 / 339.5, 64 Ki 1.21 / 2.06 / 339.1 (4 blocks an SM; 3 as above), 128 Ki
-// 1.22 / 2.76 / 341.3.
+// 128x128 procedural viewport at 1 spp: 2.44 -> 1.11 ms; value materials at
+// 512x512, 4 spp: 2.68 -> 2.19 ms.  A path's steps take longer here than spread
+// over wavefronts (fewer warps an SM, all kinds of steps in one), so a queue has
+// to leave most lanes idle: the limit of 20 Ki paths is about a third of the
+// resident lanes.  Device ms of renders of 8 scenes, 96x96 to 1280x720 at 1 spp,
+// with limits of 0 / 16 Ki / 20 Ki / 32 Ki / 64 Ki paths: closed box, 255x257 0.50 / 0.44 /
+// 0.44 / 0.48 / 0.84; glass, 1024x512 2.22 / 2.31 / 2.30 / 2.58 / 2.82; glossy with the light
+// tree, 181x181 1.16 / 0.66 / 0.75 / 0.62 / 0.62; procedural, 512x512 3.86 / 3.06 / 3.08 /
+// 3.00 / 3.62.
 template <bool kMulti, bool kGlossy>
 __global__ void __launch_bounds__(128, PSY_TAIL_MIN_BLOCKS)
     k_tail(const __grid_constant__ SceneView s_arg, const __grid_constant__ RenderParams p_arg,

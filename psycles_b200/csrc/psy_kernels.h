@@ -18,7 +18,7 @@ struct LaunchConfig {
     uint32_t shadow_sort_threshold = 0;     // shadow queue by direction (off: it measured slower); 0: never
     uint32_t ray_sort_threshold = 0;        // closest-hit queue by origin cell and octant (off: it measured slower)
     uint32_t stream_block = 256;            // threads per block of raygen and film
-    uint32_t tail_paths = 1u << 16;         // queues shorter than this finish in k_tail; 0: none (at most the
+    uint32_t tail_paths = 20u << 10;        // queues shorter than this finish in k_tail; 0: none (at most the
                                             // least sort threshold: a queue that is sorted does not)
 };
 

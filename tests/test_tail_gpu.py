@@ -22,7 +22,8 @@ def passes(session):
 
 @pytest.mark.parametrize("name,width,height,spp,tree", [
     ("small", 1, 1, 1, 0), ("small", 33, 3, 1, 0), ("glass", 255, 257, 1, 0), ("small", 256, 256, 1, 1),
-    ("lamps", 65537, 1, 1, 0), ("values", 331, 199, 3, 0), ("glass", 160, 120, 9, 1)])
+    ("lamps", 65537, 1, 1, 0), ("values", 331, 199, 3, 0), ("glass", 160, 120, 9, 1),
+    ("small", 160, 128, 1, 0), ("lamps", 20479, 1, 1, 1), ("glass", 20480, 1, 1, 0), ("values", 143, 143, 1, 0)])
 def test_tail_equals_wavefronts(backend, name, width, height, spp, tree):
     compiled = backend.compile_scene(SCENES[name](seed=5)).scene
     st = scenes.render_settings(width, height, max_bounces=7, use_light_tree=tree, seed=3)

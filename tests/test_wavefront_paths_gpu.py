@@ -1,5 +1,5 @@
 """Short renders step by step in wavefronts (gpu-marked).  A render of fewer than
-64 Ki paths otherwise ends in one kernel, which most GPU tests' renders would
+20 Ki paths otherwise ends in one kernel, which most GPU tests' renders would
 do as a whole; with sort thresholds of one path every queue is traced, sorted,
 shaded and shadowed by the wavefront kernels.  Other files' tests run here
 again in that way: single sessions against the oracle, batches and the render
