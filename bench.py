@@ -675,18 +675,21 @@ def run_viewports(backend, compiled, count: int = 64, sweep: str = "descent") ->
             "batched_vs_plain": plain_wall / batch_result["wall_s"], "identical": bool(same)}
 
 
-# DRAM bytes per second of device time of the traversal and shading kernels,
-# from one ncu capture of each (the third launch of the 4-spp
-# procedural render: DRAM read + write of the launch over its duration).
-# The traffic of a bench launch is this rate times the launch's mean
-# event-timed duration (the procedural workload only).
-NCU_DRAM_GBS = {"intersect": (323.5 + 66.3) / 1.283, "shadow": (111.7 + 13.4) / 0.758,
-                "shade": (424.0 + 231.5) / 0.537}
+# DRAM bytes per second of device time of the traversal and shading classes, from
+# one ncu capture of every kernel of the third step of the 4-spp procedural
+# render: DRAM read + write over duration in MB / ms, summed over the kernels
+# the class times together (intersect: k_intersect, k_closest_exact; shade: the
+# three sort kernels, k_shade_miss, k_shade).  The traffic of a class's step in
+# the bench is this rate times its mean event-timed duration (the procedural
+# workload only).
+NCU_DRAM_GBS = {"intersect": (320.1 + 64.1) / (1.363 + 0.004), "shadow": (119.7 + 53.5) / 0.772,
+                "shade": (331.5 + 10.0 + 17.6 + 196.2 + 36.5 + 423.3 + 229.1) / (0.076 + 0.006 + 0.032 + 0.080 + 0.538)}
 
 
 def kernel_profile(args, backend, compiled, settings) -> dict:
-    """Per-kernel device time of one render with CUDA events around each
-    launch class (psy_session profile mode)."""
+    """Device time of each launch class of one render with CUDA events around
+    its launches (psy_session profile mode).  Such a render takes every step
+    in wavefronts; a plain one ends in the tail kernel."""
     from psycles_b200 import _abi
     from psycles_b200.backend import SampleRange
     lib = backend.context.lib
@@ -719,11 +722,11 @@ def kernel_profile(args, backend, compiled, settings) -> dict:
         if args.config == "procedural" and name in NCU_DRAM_GBS and rec["launches"]:
             # DRAM bytes per launch (read + write), from the ncu rate above
             rec["traffic_per_launch"] = NCU_DRAM_GBS[name] * 1e9 * (rec["ms"] / 1e3) / rec["launches"]
-    return {"kernels": kernels,
+    return {"kernels": kernels, "kernels_of": "a render with the tail kernel off; shade with its sorts and misses",
             "roofline": {"kernel": f"k_{top}", "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "traffic": traffic,
                          "algorithmic_bytes_per_launch": k["algorithmic_bytes"] / k["launches"] if k["launches"] else 0.0,
-                         "traffic_source": "ncu DRAM bytes per device-second of this kernel x mean launch duration"
+                         "traffic_source": "ncu DRAM bytes per device-second of this class x its mean duration"
                          if traffic is not None else None,
                          "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if not peaks.get("fallback")
                          else "fallback 6.65 TB/s"}}

@@ -2422,8 +2422,8 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
         launches += 1u;
         return PSY_OK;
     };
-    auto read_counters = [&](uint32_t *c3) -> psy_status {
-        PSY_CUDA_TRY(cudaMemcpyAsync(c3, ctx->arena.view.counters, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    auto read_counters = [&](uint32_t (&c)[psy::kCounterMisses + 1u]) -> psy_status {
+        PSY_CUDA_TRY(cudaMemcpyAsync(c, ctx->arena.view.counters, sizeof(c), cudaMemcpyDeviceToHost, st));
         PSY_CUDA_TRY(cudaStreamSynchronize(st));
         return PSY_OK;
     };
@@ -2451,23 +2451,28 @@ psy_status psy_session_render_samples(psy_session *s, uint32_t first, uint32_t c
         stats.camera_rays += paths;
         const bool all_tail = paths < lc.tail_paths;  // the step launches would find nothing to do
         for (uint32_t step = 0; step < p.steps && !all_tail; ++step) {
-            uint32_t c3[3] = {0u, 0u, 0u};
-            if (prof && (ps = read_counters(c3)) != PSY_OK) return ps;
+            uint32_t c[psy::kCounterMisses + 1u] = {};
+            if (prof && (ps = read_counters(c)) != PSY_OK) return ps;
             if ((ps = timed([&] { return psy::launch_intersect(st, lc, s->scene->view, b, paths); },
                             pf.intersect_launches, pf.intersect_ms)) != PSY_OK)
                 return ps;
-            pf.intersect_bytes += 88.0 * c3[0];
+            pf.intersect_bytes += 88.0 * c[0];
             if ((ps = timed(
                      [&] { return psy::launch_shade(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
                      pf.shade_launches, pf.shade_ms)) != PSY_OK)
                 return ps;
-            if (prof && (ps = read_counters(c3)) != PSY_OK) return ps;
-            pf.shade_bytes += 304.0 * c3[0] + 68.0 * c3[2];
+            if (prof && (ps = read_counters(c)) != PSY_OK) return ps;
+            // a sorted queue's misses only read their ray, state and
+            // radiance and write the ended path's
+            const uint32_t misses = !trace && lc.sort_threshold != 0u && c[0] >= lc.sort_threshold
+                                        ? c[psy::kCounterMisses]
+                                        : 0u;
+            pf.shade_bytes += 304.0 * (c[0] - misses) + 112.0 * misses + 68.0 * c[2];
             if ((ps = timed(
                      [&] { return psy::launch_shadow(st, lc, s->scene->view, p, b, paths, step, trace_path, tr); },
                      pf.shadow_launches, pf.shadow_ms)) != PSY_OK)
                 return ps;
-            pf.shadow_bytes += 100.0 * c3[2];
+            pf.shadow_bytes += 100.0 * c[2];
             stats.kernel_launches += psy::launch_end_step(st, lc, b.counters, ray_stats, step);
             std::swap(b.queue_in, b.queue_out);
             // every 4 steps, stop early once no more paths are left than
