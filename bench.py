@@ -371,6 +371,7 @@ def run_cuda(args) -> None:
     if kernel:
         line["roofline"] = kernel["roofline"]
         line["kernels"] = kernel["kernels"]
+        line["kernels_of"] = kernel["kernels_of"]
     if args.serving and args.config == "procedural":
         line["viewports"] = run_viewports(backend, comp.scene)
         line["serving"] = run_serving(backend, jobs=args.serving_jobs, rate=args.serving_rate,

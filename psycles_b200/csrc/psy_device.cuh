@@ -527,20 +527,15 @@ __device__ __forceinline__ float input_scalar(const SceneView &s, const Material
     return eval_value(s, m, ref & ~PSY_INPUT_VALUE).x;
 }
 
-// Leaf kinds a closure walk reports (kLeaves of walk_closures).
-constexpr uint32_t kLeafDiffuse = 1u, kLeafTransparent = 2u, kLeafEmission = 4u, kLeafGlossy = 8u, kLeafAll = 15u;
-
 // Visits closure leaves depth-first, `a` before `b`, with the add / mix
 // weight rule; `visit(op, weight, color, roughness, ior)` receives the
-// diffuse / microfacet / transparent / emission leaves selected by kLeaves
-// with their authored colour (x strength for emission), the roughness input
+// diffuse / microfacet / transparent / emission leaves with their authored
+// colour (x strength for emission), the roughness input
 // of diffuse and microfacet leaves, and the IOR of glass and refraction (a
 // Beckmann leaf's op carries kGlossyBeckmann).  Glass is allocated with the
 // mix weight and takes its colour as a tint; refraction's weight is colour x
 // mix weight (graph_surface_closures.cpp:290-320).
-// Unselected leaves read no inputs (a shadow ray's extinction needs only
-// the transparent ones).
-template <uint32_t kLeaves = kLeafAll, typename Visit>
+template <typename Visit>
 __device__ __forceinline__ void walk_closures(const SceneView &s, const MaterialGpu &m, Visit visit) {
     uint32_t stack_id[kMaxClosureStack];
     float stack_w[kMaxClosureStack];
@@ -564,31 +559,23 @@ __device__ __forceinline__ void walk_closures(const SceneView &s, const Material
             stack_id[sp] = c.b; stack_w[sp] = w * f; ++sp;
             stack_id[sp] = c.a; stack_w[sp] = w * (1.0f - f); ++sp;
         } else if (c.op == PSY_CLOSURE_DIFFUSE) {
-            if constexpr ((kLeaves & kLeafDiffuse) != 0u) {
-                const f3 color = input_vector(s, m, c.color);
-                visit(c.op, color * w, color, input_scalar(s, m, c.roughness), 1.0f);
-            }
+            const f3 color = input_vector(s, m, c.color);
+            visit(c.op, color * w, color, input_scalar(s, m, c.roughness), 1.0f);
         } else if (c.op == PSY_CLOSURE_TRANSPARENT) {
-            if constexpr ((kLeaves & kLeafTransparent) != 0u) {
-                const f3 color = input_vector(s, m, c.color);
-                visit(c.op, color * w, color, 0.0f, 1.0f);
-            }
+            const f3 color = input_vector(s, m, c.color);
+            visit(c.op, color * w, color, 0.0f, 1.0f);
         } else if (c.op == PSY_CLOSURE_GLOSSY) {
-            if constexpr ((kLeaves & kLeafGlossy) != 0u) {
-                const f3 color = input_vector(s, m, c.color);
-                const uint32_t op = c.a == PSY_GLOSSY_BECKMANN    ? (uint32_t(PSY_CLOSURE_GLOSSY) | kGlossyBeckmann)
-                                    : c.a == PSY_GLOSSY_MULTI_GGX ? (uint32_t(PSY_CLOSURE_GLOSSY) | kGlossyMultiscatter)
-                                                                  : uint32_t(PSY_CLOSURE_GLOSSY);
-                visit(op, color * w, color, input_scalar(s, m, c.roughness), 1.0f);
-            }
+            const f3 color = input_vector(s, m, c.color);
+            const uint32_t op = c.a == PSY_GLOSSY_BECKMANN    ? (uint32_t(PSY_CLOSURE_GLOSSY) | kGlossyBeckmann)
+                                : c.a == PSY_GLOSSY_MULTI_GGX ? (uint32_t(PSY_CLOSURE_GLOSSY) | kGlossyMultiscatter)
+                                                              : uint32_t(PSY_CLOSURE_GLOSSY);
+            visit(op, color * w, color, input_scalar(s, m, c.roughness), 1.0f);
         } else if (c.op == PSY_CLOSURE_GLASS || c.op == PSY_CLOSURE_REFRACTION) {
-            if constexpr ((kLeaves & kLeafGlossy) != 0u) {
-                const f3 color = max3(input_vector(s, m, c.color), mk3(0.0f));
-                const uint32_t op = uint32_t(c.op) | (c.a == PSY_GLOSSY_BECKMANN ? kGlossyBeckmann : 0u);
-                visit(op, c.op == PSY_CLOSURE_GLASS ? mk3(w) : color * w, color, input_scalar(s, m, c.roughness),
-                      maxf_(input_scalar(s, m, c.scalar), 1.0e-5f));
-            }
-        } else if (c.op == PSY_CLOSURE_EMISSION && (kLeaves & kLeafEmission) != 0u) {
+            const f3 color = max3(input_vector(s, m, c.color), mk3(0.0f));
+            const uint32_t op = uint32_t(c.op) | (c.a == PSY_GLOSSY_BECKMANN ? kGlossyBeckmann : 0u);
+            visit(op, c.op == PSY_CLOSURE_GLASS ? mk3(w) : color * w, color, input_scalar(s, m, c.roughness),
+                  maxf_(input_scalar(s, m, c.scalar), 1.0e-5f));
+        } else if (c.op == PSY_CLOSURE_EMISSION) {
             const f3 color = input_vector(s, m, c.color) * input_scalar(s, m, c.scalar);
             visit(c.op, color * w, color, 0.0f, 1.0f);
         }
@@ -774,7 +761,7 @@ __device__ __forceinline__ BakedMaterialGpu bake_material(const SceneView &s, co
     // cycles_runtime_flags (src/luisa/graph_surface_scattering.cpp:292-365)
     uint32_t count = 0u, runtime = 0u;
     int transparent_slot = -1;
-    walk_closures<kLeafAll>(s, m, [&](uint32_t op, f3 w, f3 color, float roughness, float ior) {
+    walk_closures(s, m, [&](uint32_t op, f3 w, f3 color, float roughness, float ior) {
         if (op == PSY_CLOSURE_EMISSION) {
             emission = emission + w;
             return;

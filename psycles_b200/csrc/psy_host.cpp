@@ -1275,8 +1275,7 @@ psy_status stage_light_tree(psy_scene *sc, const std::vector<float> &scalars, co
                             tree.nodes[tree.root].measure.energy > 0.0f;
         if (usable) {
             auto flags = [](const psy::LtMeasure &m, bool distant) {
-                return (!m.bounds.empty ? psy::kLtFlagBounds : 0u) | (!m.orientation.empty ? psy::kLtFlagOrientation : 0u) |
-                       (distant ? psy::kLtFlagDistant : 0u);
+                return (!m.orientation.empty ? psy::kLtFlagOrientation : 0u) | (distant ? psy::kLtFlagDistant : 0u);
             };
             // returns the bits of half the half extent's length
             auto pack = [](const psy::LtMeasure &m, float4 &a, float4 &b, float4 &c) {
@@ -1778,7 +1777,6 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         psy::MeshGpu &g = meshes[i];
         g.vertex_offset = uint32_t(positions.size() / 3u);
         g.index_offset = uint32_t(indices.size());
-        g.triangle_count = m.triangle_count;
         g.smooth = m.smooth ? 1u : 0u;
         positions.insert(positions.end(), m.positions, m.positions + 3ull * m.vertex_count);
         if (m.smooth) normals.insert(normals.end(), m.normals, m.normals + 3ull * m.vertex_count);

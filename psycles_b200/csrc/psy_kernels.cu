@@ -200,9 +200,7 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 // Persistent closest-hit kernel: each lane owns one ray at a time and, when
 // some have finished, the warp refills its idle lanes from a global fetch
 // counter (one atomic per warp), so lanes do not wait for the warp's longest
-// ray.  Refilling at 12 idle lanes measured best (4: 182 ms of closest hits
-// per 1080p procedural frame of 64 spp, 8: 169, 12: 165, 16: 164 with shadow
-// rays slower again).
+// ray.  Refilling at 12 idle lanes measured best of 4, 8, 12 and 16.
 //
 // Both traversal kernels were bound by L1 wavefronts (72 % of peak for closest
 // hits: a 128-byte node in eight 16-byte loads, each a wavefront per lane)

@@ -75,7 +75,7 @@ LtEmitter lt_analytic_emitter(uint32_t id, const void *light_desc);
 // the kernels' float expressions: the bounds as centre and half extent, the
 // normalised cone axis, half the half extent's length (`emitters.w` /
 // `identity.w`, float bits).
-constexpr uint32_t kLtFlagOrientation = 1u, kLtFlagBounds = 2u, kLtFlagDistant = 4u;
+constexpr uint32_t kLtFlagOrientation = 1u, kLtFlagDistant = 4u;
 
 // `cone` holds the orientation cone's cosines and sine the importance
 // bounds use, computed on the host in double and rounded once:

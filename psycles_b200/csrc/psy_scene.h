@@ -120,11 +120,10 @@ static_assert(sizeof(ShadeTriGpu) == 96, "a shading triangle is three 32-byte se
 // A mesh while its triangle records are packed (k_pack_triangles).
 struct alignas(16) MeshGpu {
     uint32_t tri_offset;  // first leaf triangle in `tris`, also the Cycles primitive id of local primitive 0
-    uint32_t triangle_count;
     uint32_t vertex_offset;    // into positions / normals (vertices)
     uint32_t index_offset;     // into indices (uint32 elements)
     uint32_t material_offset;  // into the triangle materials, kInvalid = instance material
-    uint32_t smooth, pad0, pad1;
+    uint32_t smooth, pad[3];
 };
 
 struct alignas(16) MaterialGpu {
