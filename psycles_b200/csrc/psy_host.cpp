@@ -380,10 +380,10 @@ struct WideNode {
 // (base - o) / d in float; in units of position its rounding stays within a
 // few 2^-24 of the extent, the coordinates and the ray's own origin and
 // reach.  The margin takes 4e-6 (64 such units) of the first two on either
-// side; the last two are covered as they were for float planes, by the boxes' own
-// padding and the widened far bound.  span is chosen so that the planes of
-// bytes 0 and 255 enclose the padded extent.  Boxes that are not finite in
-// float (or whose span would not be) give NaN planes, which the test ignores.
+// side; the last two are covered by the widened far bound (visit_node).  span
+// is chosen so that the planes of bytes 0 and 255 enclose the padded extent.
+// Boxes that are not finite in float (or whose span would not be) give NaN
+// planes, which the test ignores.
 psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offset) {
     psy::NodeGpu g{};
     uint32_t *words[6] = {&g.lox, &g.hix, &g.loy, &g.hiy, &g.loz, &g.hiz};
@@ -407,8 +407,9 @@ psy::NodeGpu quantise(const WideNode &w, uint32_t node_offset, uint32_t tri_offs
         float base = 0.0f;
         for (int tries = 0; tries < 64; ++tries) {
             base = std::nextafter(float(lo - 0.5 * double(span)), -INFINITY);
-            if (double(base) + double(span) * (255.0 / 128.0) >= hi) break;
-            span = std::nextafter(span * 1.000001f, INFINITY);
+            const double missing = hi - (double(base) + double(span) * (255.0 / 128.0));
+            if (!(missing > 0.0)) break;
+            span = std::nextafter(float(double(span) + missing), INFINITY);
         }
         if (!std::isfinite(base) || !std::isfinite(span)) base = span = NAN;
         g.base[a] = base;

@@ -22,3 +22,8 @@ def run(name, tmp_path, *sources):
 def test_edits_rejected_for_memory_leave_the_scene_as_it_was(tmp_path):
     r = run("versioned_edit", tmp_path, "psy_host.cpp", "psy_light_tree.cpp")
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_byte_boxes_against_float_boxes(tmp_path):
+    r = run("node_boxes", tmp_path, "psy_light_tree.cpp")
+    assert r.returncode == 0, r.stdout + r.stderr
