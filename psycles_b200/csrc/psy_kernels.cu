@@ -3,6 +3,7 @@
 // One render batch holds P window pixels x S samples = N paths whose state
 // lives in HBM as structure-of-arrays (PathBuffers).  Per path step:
 //   k_intersect  closest hit of every queued path (two-level BVH)
+//   k_closest_exact  the few closest hits that depend on the order of visits
 //   k_sort_*     long queues grouped by material and lamp kind, misses first
 //   k_shade_miss the sorted queue's misses: lamps, background
 //   k_light_pick light tree: the paths' picks and forward pdfs
