@@ -564,8 +564,9 @@ psy_status psy_session_stats(const psy_session *session,
                              psy_render_stats *out);
 
 /* Per-kernel-class device time of the last render_samples call in profiling
- * mode (CUDA events around every launch; one host synchronisation per path
- * step) and the algorithmic HBM bytes each class moved: the path-state,
+ * mode (CUDA events around every class's launches; one host synchronisation
+ * per path step, and every step in wavefronts: no queue ends in the tail
+ * kernel) and the algorithmic HBM bytes each class moved: the path-state,
  * ray, hit, queue, shadow and film records it must read and write, counted
  * from the live queue sizes.  No reference counterpart: measurement
  * support for the roofline report. */

@@ -1621,13 +1621,6 @@ __device__ __forceinline__ void visit_node(TraversalState &t, const SceneView &s
     }
 }
 
-// A ray that starts within the instance's reach meets the instance's box
-// wherever it meets a triangle's in it (instance_reach in psy_host.cpp).
-__device__ __forceinline__ bool within_reach(const Ray &ray, uint32_t visibility_reach) {
-    return fmaxf(fabsf(ray.o.x), fmaxf(fabsf(ray.o.y), fabsf(ray.o.z))) <
-           __uint_as_float(visibility_reach & 0xffff0000u);
-}
-
 __device__ __forceinline__ bool instance_admits(const SceneView &s, uint32_t instance, const SlabRay &world, float tmin,
                                                 float tmax, float &near) {
     uint4 w0, w1;
@@ -1682,9 +1675,9 @@ __device__ __forceinline__ void cross_instance(TraversalState &t, const SceneVie
         load_sector_nc(ep, w0, w1);
         load_sector_nc(ep->w2o + 8, w2, w3);
         bool enters = (w3.z & t.visibility) != 0u;
-        if (!kNearFirst && !within_reach(t.ray, w3.z)) {
+        if (!kNearFirst) {
             float near;
-            t.cur = make_slab_ray(t.ray.o, t.ray.d);
+            if (left) t.cur = make_slab_ray(t.ray.o, t.ray.d);
             enters = enters && instance_admits(s, i, t.cur, t.ray.tmin, t.tmax, near) && near <= t.tmax;
         }
         if (enters) {

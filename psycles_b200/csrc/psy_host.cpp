@@ -327,45 +327,6 @@ void padded(const Box &b, float lo[3], float hi[3]) {
 #define PSY_SAH_AXES 3
 #endif
 
-// How far from the world's origin (largest coordinate) rays may start for which
-// a triangle's own box says all about its instance's: a ray that meets the
-// triangle's padded box in object space then meets the instance's in the
-// world, and no later.  Both tests round: the far bounds' widening comes to
-// 2^-20 of the distance from the ray's origin, products, sums and the
-// approximate reciprocal to a few 2^-23 of the coordinates, those of the object
-// space scaled by its transform.  What the instance's padding exceeds the
-// triangles' by covers twice these; where it does not (an instance flat
-// on an axis at coordinate 0 is not padded there) no distance is small enough.
-float instance_reach(const psy::BoxGpu &world, const Box &mesh, const M34 &o2w, const float *w2o) {
-    if (mesh.empty()) return 0.0f;
-    const float to_world[9] = {o2w.c0.x, o2w.c0.y, o2w.c0.z, o2w.c1.x, o2w.c1.y, o2w.c1.z, o2w.c2.x, o2w.c2.y, o2w.c2.z};
-    double mesh_pad = 0.0, mesh_coordinate = 0.0, scale = 0.0, inverse = 0.0, offset = 0.0;
-    for (int a = 0; a < 3; ++a) {
-        const double c = std::max(std::fabs(mesh.lo[a]), std::fabs(mesh.hi[a]));
-        mesh_pad = std::max(mesh_pad, 1e-5 * (mesh.hi[a] - mesh.lo[a]) + 1e-6 * c);
-        mesh_coordinate = std::max(mesh_coordinate, c);
-        double row = 0.0, inverse_row = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            row += std::fabs(double(to_world[3 * k + a]));
-            inverse_row += std::fabs(double(w2o[3 * k + a]));
-        }
-        scale = std::max(scale, row);
-        inverse = std::max(inverse, inverse_row);
-        offset = std::max(offset, std::fabs(double(w2o[9 + a])));
-    }
-    double pad = 1e300, coordinate = 0.0;
-    for (int a = 0; a < 3; ++a) {
-        // the padding is 1e-4 of the extent and 1e-5 of the coordinate, or little more
-        const double lo = world.lo[a], hi = world.hi[a], c = std::max(std::fabs(lo), std::fabs(hi));
-        pad = std::min(pad, 0.99 * (1e-4 * (hi - lo) / 1.0003 + 1e-5 * std::max(0.0, c - 1.1e-4 * (hi - lo))));
-        coordinate = std::max(coordinate, c);
-    }
-    constexpr double kWiden = 1.0 / (1 << 19), kRound = 1.0 / (1 << 20);
-    const double slack = pad - scale * mesh_pad - kWiden * coordinate - kRound * scale * (mesh_coordinate + offset);
-    const double reach = slack / (kWiden + kRound * (1.0 + scale * inverse));
-    return reach > 0.0 && std::isfinite(reach) ? float(std::min(reach, 1e30)) : 0.0f;
-}
-
 // A 4-wide node as built: child boxes in float, links as the traversal takes
 // them (node indices and leaf triangles relative to the tree).
 struct WideNode {
@@ -1847,11 +1808,7 @@ psy_status psy_scene_compile(psy_context *ctx, const psy_scene_desc *d, psy_scen
         std::copy(std::begin(instances[i].w2o), std::end(instances[i].w2o), e.w2o);
         e.root = node_offsets[instances[i].mesh];
         e.prim_offset = instances[i].prim_offset = mesh.tri_offset;
-        e.visibility_reach = instances[i].visibility & 0xffffu;
-        const float reach = instance_reach(world_boxes[i], mesh_boxes[instances[i].mesh], o2w[i], instances[i].w2o);
-        uint32_t bits;
-        std::memcpy(&bits, &reach, 4);
-        e.visibility_reach |= bits & 0xffff0000u;
+        e.visibility = instances[i].visibility;
         e.material = instances[i].material =
             mesh.material_offset != psy::kInvalidId ? psy::kInvalidId : tagged_material(d->instances[i].material);
         instances[i].smooth = mesh.smooth;

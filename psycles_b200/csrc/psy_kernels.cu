@@ -208,8 +208,8 @@ __device__ __forceinline__ uint32_t contract_visibility(uint32_t v) {
 // and by divergence (9 and 7 of 32 lanes).  With 64-byte nodes in two loads
 // and steps taken together (traverse_warp) they are issue-bound, and the lower
 // register budgets give the latency more warps to hide in.  1080p procedural
-// frame, 64 spp: closest hits 224 -> 151 ms at 7 blocks of 128 an SM (8, where
-// closest_ambiguous spills: 156), shadow rays 185 -> 78 ms at 8.
+// frame, 64 spp: closest hits 224 -> 152 ms at 7 blocks of 128 an SM (8, where
+// closest_ambiguous spills: 157), shadow rays 185 -> 81 ms at 8.
 #ifndef PSY_REFILL_LANES
 #define PSY_REFILL_LANES 12
 #endif
@@ -301,10 +301,10 @@ __device__ __forceinline__ bool closest_ambiguous(const ClosestHit &best, const 
                                                   uint32_t &prim) {
     prim = kInvalid;
     if (best.instance == kInvalid) return false;
-    uint4 w0, w1, w2, w3, ua, ub, uc, ud;
+    uint4 w0, w1, ua, ub, uc, ud;
     const EntryGpu *ep = s.entries + best.instance;
     load_sector_nc(ep, w0, w1);
-    load_sector_nc(ep->w2o + 8, w2, w3);
+    const uint4 w2 = __ldg(reinterpret_cast<const uint4 *>(ep->w2o + 8));
     const TriGpu *tp = s.tris + best.slot;
     load_sector_nc(tp, ua, ub);
     load_sector_nc(&tp->v2, uc, ud);
@@ -314,11 +314,9 @@ __device__ __forceinline__ bool closest_ambiguous(const ClosestHit &best, const 
     if (!box_admits(entry_slabs(w0, w1, w2, t.ray), mk3(__uint_as_float(ub.w), __uint_as_float(uc.w), e.x),
                     mk3(e.y, e.z, e.w), t.ray.tmin, kInf, near))
         return true;
-    if (!within_reach(t.ray, w3.z)) {
-        float entry;
-        if (!instance_admits(s, best.instance, make_slab_ray(t.ray.o, t.ray.d), t.ray.tmin, kInf, entry)) return true;
-        near = fmaxf(near, entry);
-    }
+    float entry;
+    if (!instance_admits(s, best.instance, make_slab_ray(t.ray.o, t.ray.d), t.ray.tmin, kInf, entry)) return true;
+    near = fmaxf(near, entry);
     return __uint_as_float(t.stack[kStackVisitor]) < near || t.tmax < near;
 }
 
@@ -349,7 +347,7 @@ __device__ __noinline__ ClosestHit closest_exact(const NodeGpu *nodes, const Box
         }
         if (node >= kLinkInstance) {
             const EntryGpu &e = entries[node & ~kLinkInstance];
-            if ((e.visibility_reach & visibility) == 0u) {
+            if ((e.visibility & visibility) == 0u) {
                 node = stack[--sp];
                 continue;
             }

@@ -84,9 +84,7 @@ struct alignas(32) EntryGpu {
     float w2o[12];
     uint32_t root;         // root node of the mesh
     uint32_t prim_offset;  // Cycles primitive id of local primitive 0
-    // low half: visibility; high half: that of a float, how far from the world's
-    // origin rays may start whose hits need no test of the instance's box
-    uint32_t visibility_reach;
+    uint32_t visibility;
     uint32_t material;  // as InstanceGpu::material
 };
 static_assert(sizeof(EntryGpu) == 64, "an instance entry is two 32-byte sectors");
