@@ -2,8 +2,8 @@
 // the CPU in the kernels' float expressions:
 //   planes    a node's bytes enclose its children's float boxes and the margin
 //   slabs     a ray that a child's float box admits is admitted by its bytes
-//   traversal the closest hit through byte boxes, unless found ambiguous, is that
-//             through float boxes
+//   traversal the closest hit through byte boxes, of instances under transforms
+//             too, is that through float boxes unless found ambiguous
 #include "fake_cuda.h"
 
 #include "../../psycles_b200/csrc/psy_host.cpp"
@@ -231,80 +231,161 @@ struct Mesh {
         for (const WideNode &w : wide) nodes.push_back(quantise(w, 0u, 0u));
     }
 };
+// Instances of meshes under the instance tree, as scene compile lays them out.
+struct Scene {
+    std::vector<const Mesh *> mesh;  // of each instance
+    std::vector<M34> o2w, w2o;
+    std::vector<std::array<float, 6>> box;
+    std::vector<WideNode> wide;
+    std::vector<psy::NodeGpu> nodes;
+    void add(const Mesh &m, const M34 &t) {
+        mesh.push_back(&m);
+        o2w.push_back(t);
+        w2o.push_back(inverse34(t));
+    }
+    void build() {
+        Builder b;
+        b.leaf_is_id = true;
+        box.resize(mesh.size());
+        for (uint32_t i = 0; i < mesh.size(); ++i) {
+            Prim q;
+            const M34 &t = o2w[i];
+            for (const V3 &v : mesh[i]->p) {
+                const double x = v.x, y = v.y, z = v.z;
+                q.box.grow(x * t.c0.x + y * t.c1.x + z * t.c2.x + t.c3.x, x * t.c0.y + y * t.c1.y + z * t.c2.y + t.c3.y,
+                           x * t.c0.z + y * t.c1.z + z * t.c2.z + t.c3.z);
+            }
+            for (int a = 0; a < 3; ++a) {
+                const double pad = 1e-4 * (q.box.hi[a] - q.box.lo[a]) +
+                                   1e-5 * std::max(std::fabs(q.box.lo[a]), std::fabs(q.box.hi[a]));
+                q.box.lo[a] -= pad;
+                q.box.hi[a] += pad;
+                q.c[a] = 0.5 * (q.box.lo[a] + q.box.hi[a]);
+            }
+            padded(q.box, &box[i][0], &box[i][3]);
+            q.id = i;
+            b.prims.push_back(q);
+        }
+        b.build_root();
+        std::vector<uint32_t> order;
+        wide = b.widen(order);
+        for (const WideNode &w : wide) nodes.push_back(quantise(w, 0u, 0u));
+    }
+};
+// A ray in the world and in every instance's object space.
+struct SceneRay {
+    Slabs world;
+    std::vector<Slabs> object;
+    SceneRay(const Scene &s, V3 o, V3 d) : world(slabs(o, d)) {
+        for (const M34 &t : s.w2o) {
+            V3 od = xaff(t, d, false);
+            for (int a = 0; a < 3; ++a)
+                if (std::fabs((&od.x)[a]) <= 8.271806e-25f) (&od.x)[a] = std::copysign(8.271806e-25f, (&od.x)[a]);
+            object.push_back(slabs(xaff(t, o, true), od));
+        }
+    }
+};
 struct Found {
     float t;
-    uint32_t prim;
-    bool operator==(const Found &o) const { return t == o.t && prim == o.prim; }
+    uint32_t instance, prim;
+    bool operator==(const Found &o) const { return t == o.t && instance == o.instance && prim == o.prim; }
 };
-bool better(const Found &best, float t, uint32_t prim) {
-    return best.prim == psy::kInvalidId || t < best.t || (t == best.t && prim > best.prim);
+bool better(const Found &best, float t, uint32_t instance, uint32_t prim) {
+    return best.instance == psy::kInvalidId || t < best.t ||
+           (t == best.t && (instance > best.instance || (instance == best.instance && prim > best.prim)));
+}
+using Children = std::vector<std::pair<float, uint32_t>>;
+void push(std::vector<uint32_t> &stack, Children &c) {
+    std::stable_sort(c.begin(), c.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+    for (const auto &i : c) stack.push_back(i.second);
 }
 
-// closest_exact
-Found through_floats(const Mesh &m, const Slabs &r, float tmin) {
-    Found best{1e30f, psy::kInvalidId};
+// closest_exact: one tree, the instance tree's entries handed to `enter`
+template <typename Enter, typename Leaf>
+void walk_floats(const std::vector<WideNode> &wide, const Slabs &r, float tmin, const Found &best, Enter enter, Leaf leaf) {
     std::vector<uint32_t> stack{0u};
     while (!stack.empty()) {
-        const WideNode &w = m.wide[stack.back()];
+        const uint32_t e = stack.back();
         stack.pop_back();
+        if (e >= psy::kLinkInstance) {
+            enter(e - psy::kLinkInstance);
+            continue;
+        }
+        const WideNode &w = wide[e];
         float near[4];
         bool hit[4];
         for (int k = 0; k < 4; ++k) {
             const float lo[3] = {w.lo[0][k], w.lo[1][k], w.lo[2][k]}, hi[3] = {w.hi[0][k], w.hi[1][k], w.hi[2][k]};
             hit[k] = w.link[k] != psy::kInvalidId && admits(r, lo, hi, tmin, best.t, near[k]);
         }
-        for (int k = 0; k < 4; ++k) {
-            float t;
-            if (!hit[k] || (w.link[k] & psy::kLinkLeaf) == 0u) continue;
-            const uint32_t prim = m.leaf[w.link[k] & ~psy::kLinkLeaf];
-            if (m.hit(prim, r, tmin, best.t, t) && better(best, t, prim)) best = {t, prim};
-        }
-        std::vector<std::pair<float, uint32_t>> inner;
+        Children inner;
+        for (int k = 0; k < 4; ++k)
+            if (hit[k] && (w.link[k] & psy::kLinkLeaf) != 0u) leaf(w.link[k] & ~psy::kLinkLeaf);
         for (int k = 0; k < 4; ++k)
             if (hit[k] && (w.link[k] & psy::kLinkLeaf) == 0u && near[k] <= best.t) inner.push_back({near[k], w.link[k]});
-        std::stable_sort(inner.begin(), inner.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-        for (const auto &i : inner) stack.push_back(i.second);
+        push(stack, inner);
     }
+}
+Found through_floats(const Scene &s, const SceneRay &ray, float tmin) {
+    Found best{1e30f, psy::kInvalidId, psy::kInvalidId};
+    walk_floats(s.wide, ray.world, tmin, best, [&](uint32_t i) {
+        const Mesh &m = *s.mesh[i];
+        walk_floats(m.wide, ray.object[i], tmin, best, [](uint32_t) {}, [&](uint32_t slot) {
+            float t;
+            if (m.hit(m.leaf[slot], ray.object[i], tmin, best.t, t) && better(best, t, i, m.leaf[slot]))
+                best = {t, i, m.leaf[slot]};
+        });
+    }, [](uint32_t) {});
     return best;
 }
 
 // k_intersect's traversal, closest_hit and closest_ambiguous
-Found through_bytes(const Mesh &m, const Slabs &r, float tmin, bool &ambiguous) {
-    Found best{1e30f, psy::kInvalidId};
-    float tmax = 1e30f, second = 1e30f;
+template <typename Enter, typename Leaf>
+void walk_bytes(const std::vector<psy::NodeGpu> &nodes, const Slabs &r, float tmin, const float &tmax, Enter enter, Leaf leaf) {
     std::vector<uint32_t> stack{0u};
     while (!stack.empty()) {
-        const psy::NodeGpu &g = m.nodes[stack.back()];
+        const uint32_t e = stack.back();
         stack.pop_back();
+        if (e >= psy::kLinkInstance) {
+            enter(e - psy::kLinkInstance);
+            continue;
+        }
         float near[4];
         bool hit[4];
-        node_hits(g, r, tmin, tmax, near, hit);
-        std::vector<std::pair<float, uint32_t>> inner;
+        node_hits(nodes[e], r, tmin, tmax, near, hit);
+        Children inner;
         for (int k = 0; k < 4; ++k) {
+            const uint32_t link = nodes[e].link[k];
+            if (hit[k] && (link & psy::kLinkLeaf) != 0u) leaf(link & ~psy::kLinkLeaf);
+            else if (hit[k]) inner.push_back({near[k], link});
+        }
+        push(stack, inner);
+    }
+}
+Found through_bytes(const Scene &s, const SceneRay &ray, float tmin, bool &ambiguous) {
+    Found best{1e30f, psy::kInvalidId, psy::kInvalidId};
+    float tmax = 1e30f, second = 1e30f;
+    walk_bytes(s.nodes, ray.world, tmin, tmax, [&](uint32_t i) {
+        const Mesh &m = *s.mesh[i];
+        walk_bytes(m.nodes, ray.object[i], tmin, tmax, [](uint32_t) {}, [&](uint32_t slot) {
             float t;
-            if (!hit[k]) continue;
-            if ((g.link[k] & psy::kLinkLeaf) == 0u) {
-                inner.push_back({near[k], g.link[k]});
-                continue;
-            }
-            const uint32_t prim = m.leaf[g.link[k] & ~psy::kLinkLeaf];
-            if (!m.hit(prim, r, tmin, tmax, t)) continue;
-            if (!better(best, t, prim)) {
+            if (!m.hit(m.leaf[slot], ray.object[i], tmin, tmax, t)) return;
+            if (!better(best, t, i, m.leaf[slot])) {
                 second = std::fmin(second, t);
-                continue;
+                return;
             }
             second = best.t;
-            best = {t, prim};
+            best = {t, i, m.leaf[slot]};
             tmax = std::fma(t, 1.00000095367431640625f, 1.0e-30f);
-        }
-        std::stable_sort(inner.begin(), inner.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-        for (const auto &i : inner) stack.push_back(i.second);
-    }
+        });
+    }, [](uint32_t) {});
     ambiguous = false;
-    if (best.prim != psy::kInvalidId) {
-        float near;
-        const float *b = m.box[best.prim].data();
-        ambiguous = !admits(r, b, b + 3, tmin, INFINITY, near) || second < near || tmax < near;
+    if (best.instance != psy::kInvalidId) {
+        float near, entry;
+        const float *b = s.mesh[best.instance]->box[best.prim].data(), *w = s.box[best.instance].data();
+        ambiguous = !admits(ray.object[best.instance], b, b + 3, tmin, INFINITY, near) ||
+                    !admits(ray.world, w, w + 3, tmin, INFINITY, entry) || second < std::fmax(near, entry) ||
+                    tmax < std::fmax(near, entry);
     }
     return best;
 }
@@ -333,32 +414,63 @@ Mesh room(float x, float y0, float y1) {
     return m;
 }
 
+// A mirrored or even scale, a rotation and a translation; `plain`: none.
+M34 placed(bool plain, double spread) {
+    M34 t{{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {0, 0, 0}};
+    if (plain) return t;
+    const V3 u = direction();
+    V3 v = crs(u, direction());
+    const float length = std::sqrt(dt(v, v));
+    if (length > 1e-2f) {
+        v = {v.x / length, v.y / length, v.z / length};
+        t = {u, v, crs(u, v), {}};
+    }
+    const float k = float(std::pow(10.0, uniform(-0.5, 0.5)) * (rng() % 4u ? 1.0 : -1.0));
+    for (V3 *c : {&t.c0, &t.c1, &t.c2}) *c = {c->x * k, c->y * k, c->z * k};
+    t.c3 = {float(uniform(-spread, spread)), float(uniform(-spread, spread)), float(uniform(-spread, spread))};
+    return t;
+}
+
 void traversal() {
     Mesh meshes[] = {sphere(24, 1.0f, {0, 0, 0}), sphere(6, 0.3f, {0, 0, 0}), sphere(40, 2.3f, {4, 1, -7}),
                      room(1.0f, 0.0f, 2.0f), room(0.5f, -0.5f, 0.5f)};
-    long rays = 0, ambiguous_rays = 0, changed = 0;
+    std::vector<Scene> scenes;
     for (Mesh &m : meshes) {
         m.build();
-        for (const double reach : {3.0, 30.0, 3000.0})
-            for (int n = 0; n < 20000; ++n) {
+        scenes.emplace_back();
+        scenes.back().add(m, placed(true, 0.0));
+    }
+    for (const double spread : {0.5, 3.0})
+        for (int copies : {1, 6}) {
+            scenes.emplace_back();
+            for (int k = 0; k < copies; ++k)
+                for (const int m : {0, 1, 3, 4}) scenes.back().add(meshes[m], placed(k == 0 && m == 3, spread));
+        }
+    long rays = 0, ambiguous_rays = 0, changed = 0;
+    for (Scene &s : scenes) {
+        s.build();
+        for (const double distance : {3.0, 30.0, 3000.0})
+            for (int n = 0; n < 12000; ++n) {
                 // towards an edge or a corner, then on behind each hit
+                const uint32_t i = uint32_t(rng() % s.mesh.size());
+                const Mesh &m = *s.mesh[i];
                 const uint32_t tri = uint32_t(rng() % (m.idx.size() / 3u)), e = uint32_t(rng() % 3u);
                 const V3 a = m.p[m.idx[3 * tri + e]], b = m.p[m.idx[3 * tri + (e + 1u) % 3u]];
                 const float u = rng() % 8u ? float(uniform(0, 1)) : 0.0f;
                 V3 o, d;
-                if (!aim({a.x + u * (b.x - a.x), a.y + u * (b.y - a.y), a.z + u * (b.z - a.z)},
-                         reach * uniform(0.01, 1.0), o, d))
+                if (!aim(xaff(s.o2w[i], {a.x + u * (b.x - a.x), a.y + u * (b.y - a.y), a.z + u * (b.z - a.z)}, true),
+                         distance * uniform(0.01, 1.0), o, d))
                     continue;
-                const Slabs r = slabs(o, d);
+                const SceneRay ray(s, o, d);
                 float tmin = 0.0f;
                 for (int k = 0; k < 3; ++k) {
                     bool ambiguous;
-                    const Found bytes = through_bytes(m, r, tmin, ambiguous), floats = through_floats(m, r, tmin);
+                    const Found bytes = through_bytes(s, ray, tmin, ambiguous), floats = through_floats(s, ray, tmin);
                     ++rays;
                     ambiguous_rays += ambiguous;
                     changed += !(bytes == floats);
                     CHECK(ambiguous || bytes == floats);
-                    if (floats.prim == psy::kInvalidId) break;
+                    if (floats.instance == psy::kInvalidId) break;
                     tmin = std::nextafter(floats.t, INFINITY);
                 }
             }
